@@ -799,17 +799,18 @@ __device__ __forceinline__ void relax_polar_item(const ScParams &P, const RelaxA
 // of its rule and chain bonds do not depend on the running sums, so they are
 // evaluated first, from its bond matches (k_build_pp records them in the
 // order the reference meets them), with every lane of a warp on its own
-// first bond, then its second ...; the list is then walked once more to add
-// every term in the reference's order (the slerps of dAV and the float sums
-// are order-dependent).  A test bond rotates the particle itself, which
-// later terms read: such particles (SC_MATCH_INORDER) take the in-order
-// scan of k_relax_overflow.
-struct BondTerm {
-    sc_f3 dv;   // velocity term
-    sc_f4 q;    // dAV slerp target
-    float t;    // dAV slerp weight
-    sc_f3 dbg;  // chain bonds: rrp - ppos for the debug vector
-};
+// first bond, then its second ...  Only bond terms turn dAV and move the
+// debug vector, so those two chains are carried along in the same pass (the
+// matches come in list order); what remains per bond is its velocity term,
+// and the list is then walked once to add every velocity term in the
+// reference's order.  A test bond rotates the particle itself, which later
+// terms read: such particles (SC_MATCH_INORDER) take the in-order scan of
+// k_relax_overflow.
+//
+// Bound: the latency of one item's instruction chain (a few warps per
+// scheduler at most).  With the slerp of dAV inside the list walk, where a
+// warp's lanes meet their partners at different entries, nearly every round
+// of the walk ran it.
 
 __device__ __forceinline__ void relax_bonded_item(const ScParams &P, const RelaxArgs &A, int i, int4 in, float4 v4,
                                                   float4 r4, float4 a4) {
@@ -829,10 +830,13 @@ __device__ __forceinline__ void relax_bonded_item(const ScParams &P, const Relax
     // 1. the terms of its bond matches (list order, then bond-slot order)
     const uint32_t *__restrict__ myMatch = A.match + (size_t)i * SC_MAX_ACTIVE_INTERACTIONS;
     const int nm = min(A.matchN[i] & SC_MATCH_COUNT, SC_MAX_ACTIVE_INTERACTIONS);
-    // the first term stays in registers (most bonded items have one); the
-    // rest go to a per-thread array
-    BondTerm T0, T[SC_MAX_ACTIVE_INTERACTIONS - 1];
+    // the first velocity term stays in registers (most bonded items have
+    // one); the rest go to a per-thread array
+    sc_f3 T0 = sc_zero3(), T[SC_MAX_ACTIVE_INTERACTIONS - 1];
     int nt = 0;
+    sc_f4 pdbg = sc_make_f4(0, 0, 0, 0);
+    bool dbgTouched = false;
+    sc_f4 dAV = sc_qid();
     for (int m = 0; m < nm; m++) {
         const uint32_t me = myMatch[m];
         const int j = (int)(me & SC_PP_INDEX), k = (int)(me >> 29);
@@ -845,7 +849,8 @@ __device__ __forceinline__ void relax_bonded_item(const ScParams &P, const Relax
         const float trad = t4.w, idist = prad + trad;
         const sc_f4 trot = ld4(A.rotIn, j), tav = ld4(A.avIn, j);
         const sc_f3 tvel = ld3(A.velIn, j);
-        BondTerm b;
+        sc_f3 dv;
+        sc_f4 q;
         if (it >= 10) {
             // dynamics.cuh:591-655
             const sc_rule &pii = rule_at(P, it);
@@ -856,22 +861,20 @@ __device__ __forceinline__ void relax_bonded_item(const ScParams &P, const Relax
             sc_f4 tro_t = o2 ? sc_qmul(prot, sc_qinv(ro)) : sc_qmul(prot, ro);
             sc_f4 rro = sc_qmul(sc_qinv(sc_qmul(pav, prot)), sc_qmul(tav, tro_p));
             sc_f4 orro = sc_qmul(sc_qinv(sc_qmul(tav, trot)), sc_qmul(pav, tro_t));
-            b.q = sc_qmul(sc_slerp(rro, orro, 0.5f), rro);
-            b.t = 0.9f * trad / (prad + trad);
+            q = sc_qmul(sc_slerp(rro, orro, 0.5f), rro);
             sc_f3 rrp = o1 ? sc_rotate(-rp, sc_qmul(sc_qinv(ro), sc_qmul(tav, trot))) : sc_rotate(rp, sc_qmul(tav, trot));
             rrp += tpos;
             sc_f3 orrp = o2 ? sc_rotate(-rp, sc_qmul(sc_qinv(ro), sc_qmul(pav, prot))) : sc_rotate(rp, sc_qmul(pav, prot));
             orrp += ppos;
             sc_f3 pDV = (rrp + tvel - (ppos + pvel)) * 0.9f * trad / (prad + trad) * 1.0f;
             sc_f3 tpDV = (orrp + pvel - (tpos + tvel)) * 0.9f * prad / (prad + trad) * 1.0f;
-            b.dv = (pDV - (pDV + tpDV) / 2.0f) * 0.9f * prad / (prad + trad) * 1.0f;
+            dv = (pDV - (pDV + tpDV) / 2.0f) * 0.9f * prad / (prad + trad) * 1.0f;
         } else {
             // dynamics.cuh:692-769
             sc_f3 nextTup = sc_rotate(sc_rotate(sc_up(), trot), pav);
             sc_f3 nnd = normalize(tpos + tvel - (ppos + pvel));
             bool fwd = myBonds[3 * k + 1] == SC_INTERACTION_GROUP_FORWARD;
-            b.q = sc_quat_from_to(nextUp, (fwd ? -1.0f : 1.0f) * nnd);
-            b.t = 0.9f * trad / (prad + trad);
+            q = sc_quat_from_to(nextUp, (fwd ? -1.0f : 1.0f) * nnd);
             sc_f3 relUp = (fwd ? 1.0f : -1.0f) * nextTup;
             sc_f3 axis = sc_safe_cross(relUp, -nnd);
             float ang = sc_angle3(relUp, -nnd);
@@ -886,20 +889,25 @@ __device__ __forceinline__ void relax_bonded_item(const ScParams &P, const Relax
             orrp += ppos;
             sc_f3 pDV = (rrp + tvel - (ppos + pvel)) * 0.9f * trad / (prad + trad) * 1.0f;
             sc_f3 tpDV = (orrp + pvel - (tpos + tvel)) * 0.9f * prad / (prad + trad) * 1.0f;
-            b.dv = (pDV - (pDV + tpDV) / 2.0f) * 0.9f * prad / (prad + trad) * 1.0f;
-            b.dbg = rrp - ppos;
+            dv = (pDV - (pDV + tpDV) / 2.0f) * 0.9f * prad / (prad + trad) * 1.0f;
+            const sc_f3 dd = rrp - ppos;
+            if (!dbgTouched) {
+                pdbg = ld4(A.dbg, i);
+                dbgTouched = true;
+            }
+            pdbg.x = (float)((double)pdbg.x + (double)dd.x * (1.0 - (double)0.9f));
+            pdbg.y = (float)((double)pdbg.y + (double)dd.y * (1.0 - (double)0.9f));
+            pdbg.z = (float)((double)pdbg.z + (double)dd.z * (1.0 - (double)0.9f));
         }
+        dAV = sc_slerp(dAV, q, 0.9f * trad / (prad + trad));
         if (nt == 0)
-            T0 = b;
+            T0 = dv;
         else
-            T[nt - 1] = b;
+            T[nt - 1] = dv;
         nt++;
     }
-    // 3. every term in the reference's order
-    sc_f4 pdbg = sc_make_f4(0, 0, 0, 0);
-    bool dbgTouched = false;
+    // 2. every velocity term in the reference's order
     sc_f3 dV = sc_zero3();
-    sc_f4 dAV = sc_qid();
     sc_f3 phobPos = sc_zero3();
     float phobSum = 0.0f;
     float w = 0.0f;
@@ -926,23 +934,11 @@ __device__ __forceinline__ void relax_bonded_item(const ScParams &P, const Relax
         if (fl & SC_PP_PARTNER) {
             // this neighbour's bond matches are the next ones in order
             for (; mi < nm && (int)(myMatch[mi] & SC_PP_INDEX) == j; mi++) {
-                const int k = (int)(myMatch[mi] >> 29);
-                const int it = myBonds[3 * k];
+                const int it = myBonds[3 * (int)(myMatch[mi] >> 29)];
                 if ((it >= 10 || it == SC_INTERACTION_TYPE_CHAIN) && ut < nt) {
-                    const BondTerm b = ut == 0 ? T0 : T[ut - 1];
-                    ut++;
-                    if (it == SC_INTERACTION_TYPE_CHAIN && !dbgTouched) {
-                        pdbg = ld4(A.dbg, i);
-                        dbgTouched = true;
-                    }
-                    dAV = sc_slerp(dAV, b.q, b.t);
                     w += 1.0f;
-                    dV += b.dv;
-                    if (it == SC_INTERACTION_TYPE_CHAIN) {
-                        pdbg.x = (float)((double)pdbg.x + (double)b.dbg.x * (1.0 - (double)0.9f));
-                        pdbg.y = (float)((double)pdbg.y + (double)b.dbg.y * (1.0 - (double)0.9f));
-                        pdbg.z = (float)((double)pdbg.z + (double)b.dbg.z * (1.0 - (double)0.9f));
-                    }
+                    dV += ut == 0 ? T0 : T[ut - 1];
+                    ut++;
                 }
             }
         }
