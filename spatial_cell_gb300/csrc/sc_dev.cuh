@@ -86,7 +86,7 @@ struct ScCounters {
     int polyConflict; // 1: two listed items touch the same particle (k_poly_plan)
     int step;         // the step loop counter (main.cu:347)
     int tileCounter[4];
-    int ppClassCount[4];  // items per relax work class (k_build_pp)
+    int ppClassCount[4];  // items per relax work class (k_build_pp); [3]: RelaxArgs::unsettled
     int ovfPP, ovfM;      // items whose particle / metabolic list overflowed (k_build_pp, k_build_m)
     int _pad;
     unsigned long long poolM;   // entries the metabolic list blocks asked of their pool (k_build_m)
@@ -98,9 +98,12 @@ struct ScCounters {
 };
 
 // Relax work classes: 0 bonded items, 1 items with polar (lipid) pairs and no
-// bonds, 2 the rest.  Each class has its own kernel, so a warp's items take
-// the same branches.
+// bonds, 2 the rest (inactive items with the top bit of their index set).
+// Each class has its own blocks, so a warp's items take the same branches.
 #define SC_RELAX_CLASSES 3
+#define SC_CLASS_INACTIVE 0x80000000u
+// Particle list entries per item whose collision geometry is kept (k_build_pp).
+#define SC_GEO_PP 8
 // Bond match count of a bonded item (low bits) and its in-order flag (a
 // test bond: relaxed by the in-order scan).
 #define SC_MATCH_COUNT 0xff

@@ -53,6 +53,9 @@ struct ScBuffers {
     // list order then bond-slot order, and their count (k_build_pp).
     uint32_t *matchPP;
     int *matchN;
+    float4 *geoPP;                // collision geometry of the particle list's first SC_GEO_PP entries
+    uint4 *bondRec;               // bonded class: a record per item, in the blocks' ranked order (k_bond_plan)
+    int relaxAge;                 // relax launches since rot / angvel were last out of step (RelaxArgs::age)
     int *permM, *permLM, *permD;  // count-ordered list position -> item
     uint32_t *scratchLM;          // build scratch of the LM list (aliases listD when it fits)
     int *ovfPP, *ovfM;            // overflowed items
@@ -79,7 +82,7 @@ struct ScBuffers {
     long long *warpOffLM;         // lipid-metabolic pair pool: the same
     uint8_t *lipidP;              // per sorted particle slot: active lipid (after each particle sort)
     bool validPP, validM, validLM, validD;
-    void invalidateLists() { validPP = validM = validLM = validD = false; }
+    void invalidateLists() { validPP = validM = validLM = validD = false; relaxAge = 0; }
     // polymerisation list
     // polymerize: the scheduled items in index order, per slot the rank of
     // its new monomer and its previous monomer, per item a claim count, per

@@ -421,6 +421,8 @@ void sort_metabolic(sc_sim *s) {
 // Which pair lists a phase invalidates (it changes positions, flags, types,
 // radii or interactions their tests read, or re-sorts slots they index).
 void invalidate_after(ScBuffers &B, int phase) {
+    // only the relaxation loop's phases leave rot and angvel to relax alone
+    if (phase != SC_PHASE_RELAX && phase != SC_PHASE_RELAX_METAB && phase != SC_PHASE_RELAX_PARTNERS) B.relaxAge = 0;
     switch (phase) {
         case SC_PHASE_SORT_PARTICLES: B.validPP = B.validM = B.validLM = false; break;
         case SC_PHASE_SORT_METABOLIC: B.validM = B.validLM = B.validD = false; break;
@@ -451,7 +453,7 @@ std::vector<int> host_state(const sc_sim *s) {
     std::vector<int> v(B.cp, B.cp + FP_COUNT);
     v.insert(v.end(), B.cm, B.cm + FM_COUNT);
     v.insert(v.end(), {B.sortCurP, B.sortCurM, (int)B.validPP, (int)B.validM, (int)B.validLM, (int)B.validD,
-                       s->P.binned, s->P.mAllActive, s->P.lipidValid, B.mParity});
+                       s->P.binned, s->P.mAllActive, s->P.lipidValid, B.mParity, B.relaxAge});
     return v;
 }
 void set_host_state(sc_sim *s, const std::vector<int> &v) {
@@ -469,6 +471,7 @@ void set_host_state(sc_sim *s, const std::vector<int> &v) {
     s->P.mAllActive = v[k++];
     s->P.lipidValid = v[k++];
     B.setMParity(v[k++]);
+    B.relaxAge = v[k++];
 }
 
 int run_phase(sc_sim *s, int phase, int arg) {
@@ -734,9 +737,10 @@ static int create_sim(const sc_config *cfg_in, const sc_replica *replicas, int32
     P.SP = P.S <= 4 ? 4 : P.S <= 8 ? 8 : 12;
     P.N = cfg->num_particles;
     P.Nm = cfg->num_metabolic_particles;
-    // Concurrent work classes pay off for a sim whose particles fill the
-    // device; smaller sims keep one stream, so many of them run side by side
-    // without the cross-stream joins (class_streams 1 / 3 overrides).
+    // A kernel per relax work class, on three streams, pays off for a sim
+    // whose particles fill the device; smaller sims relax all classes in one
+    // launch on one stream, so many of them run side by side without the
+    // cross-stream joins (class_streams 1 / 3 overrides).
     s->forkClasses = cfg->class_streams == 0 ? (int64_t)P.N >= (int64_t)s->gridCap * SC_THREADS
                                              : cfg->class_streams > 1;
     P.coordSteps = cfg->noise_coordination_steps;
@@ -908,6 +912,7 @@ static int create_sim(const sc_config *cfg_in, const sc_replica *replicas, int32
         (rc = dalloc(s, &B.cntPP, N)) ||
         (rc = dalloc(s, &B.classPP, (size_t)SC_RELAX_CLASSES * N)) ||
         (rc = dalloc(s, &B.matchPP, (size_t)SC_MAX_ACTIVE_INTERACTIONS * N)) || (rc = dalloc(s, &B.matchN, N)) ||
+        (rc = dalloc(s, &B.geoPP, sc_list_words(SC_GEO_PP, (int)N))) || (rc = dalloc(s, &B.bondRec, N)) ||
         (rc = dalloc(s, &B.listM, poolWords)) ||
         (rc = dalloc(s, &B.cntM, Nm)) || (rc = dalloc(s, &B.listLM, sc_list_words(SC_LIST_LM, (int)N))) ||
         (rc = dalloc(s, &B.cntLM, N)) || (rc = dalloc(s, &B.listD, sc_list_words(SC_LIST_DBUF, (int)Nm))) ||

@@ -248,13 +248,16 @@ __global__ void __launch_bounds__(SC_THREADS) k_build_pp(ScParams P, const uint3
                                                          uint32_t *__restrict__ list, int *__restrict__ cnt, int cap,
                                                          int *__restrict__ classIdx, int *__restrict__ classCount,
                                                          int *__restrict__ ovf, int *__restrict__ ovfCount,
-                                                         uint32_t *__restrict__ match, int *__restrict__ matchN) {
+                                                         uint32_t *__restrict__ match, int *__restrict__ matchN,
+                                                         float4 *__restrict__ geo) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= *nActivePtr) return;
     int4 in = info[i];
     int cls = 2;
+    uint32_t inactive = 0;
     if (!(in.z & SC_ACTIVE)) {
         cnt[i] = 0;
+        inactive = SC_CLASS_INACTIVE;
     } else {
         rep_apply<BATCH>(P, in.w);
         BondRegs B;
@@ -267,8 +270,18 @@ __global__ void __launch_bounds__(SC_THREADS) k_build_pp(ScParams P, const uint3
         uint32_t any = 0;
         uint32_t *__restrict__ myMatch = match + (size_t)i * SC_MAX_ACTIVE_INTERACTIONS;
         const int K = min(SC_LIST_PP, P.listLimit);
-        auto add = [&](int j, uint32_t f) {
+        auto add = [&](int j, uint32_t f, sc_f3 delta, float trad) {
             if (c < K) list[sc_list_at(SC_LIST_PP, i, c)] = (uint32_t)j | f;
+            // a colliding pair's position-only part of dynamics.cuh:775-786,
+            // tpos - normalize(tpos - pos) * collisionDistance: the first
+            // float3 its velocity term evaluates, the same in every
+            // relaxation sub-iteration
+            if ((f & SC_PP_COLLIDE) && c < SC_GEO_PP) {
+                const float4 t4 = pos[j];
+                const sc_f3 tpos = IM(sc_make_f3(t4.x, t4.y, t4.z));
+                const sc_f3 a = tpos - normalize(delta) * (p4.w + trad);
+                geo[sc_list_at(SC_GEO_PP, i, c)] = make_float4(a.x, a.y, a.z, trad);
+            }
             c++;
             any |= f;
             if (f & SC_PP_PARTNER) {  // the bond slots naming this neighbour, in slot order
@@ -296,13 +309,16 @@ __global__ void __launch_bounds__(SC_THREADS) k_build_pp(ScParams P, const uint3
                 const float4 t4 = pos[j];
                 const sc_f3 delta = IM(sc_make_f3(t4.x, t4.y, t4.z)) - ppos;
                 const uint32_t f = pp_flags_in_cube(delta, t4.w, j, p4.w, phydro, B, info);
-                if (f) add(j, f);
+                if (f) add(j, f, delta, t4.w);
             }
         } else {
             // more in-cube candidates than the list holds: every test in one scan
             scan27(P, cellStart, ppos, reach(P, ppos, P.maxInt, SC_BINNED_P), [&](int j) {
                 const uint32_t f = pp_flags(P, IM, i, j, ppos, p4.w, phydro, B, pos, info);
-                if (f) add(j, f);
+                if (f) {
+                    const float4 t4 = pos[j];
+                    add(j, f, IM(sc_make_f3(t4.x, t4.y, t4.z)) - ppos, t4.w);
+                }
             });
         }
         cnt[i] = c;
@@ -323,7 +339,7 @@ __global__ void __launch_bounds__(SC_THREADS) k_build_pp(ScParams P, const uint3
     int base = 0;
     if (lane == leader) base = atomicAdd(&classCount[cls], __popc(same));
     base = __shfl_sync(same, base, leader);
-    classIdx[(size_t)cls * cap + base + __popc(same & ((1u << lane) - 1u))] = i;
+    classIdx[(size_t)cls * cap + base + __popc(same & ((1u << lane) - 1u))] = i | (int)inactive;
 }
 
 // Visits the contributing pairs of particle i in the reference's order: from
@@ -463,17 +479,22 @@ struct RelaxArgs {
     const int *__restrict__ classCount;
     const uint32_t *__restrict__ match;  // bond matches of the list (k_build_pp)
     const int *__restrict__ matchN;
+    const float4 *__restrict__ geo;      // colliding pairs' geometry (k_build_pp)
+    const uint4 *__restrict__ bondRec;   // bonded class, a record per item (k_bond_plan)
+    const int *__restrict__ ovf, *__restrict__ ovfCount;   // items left to the in-order scan
+    int *__restrict__ unsettled;  // set when an unturned angular velocity is not a fixed point (relax_still)
+    // sub-iterations since the input and output buffers of rot / angvel were
+    // last out of step (0, 1, 2 and more): what does not change in a
+    // sub-iteration is written until both buffers hold it
+    int age;
 };
 
-// One particle's relaxation.  SCAN = false reads the particle's pair list;
-// SCAN = true (list overflow) visits its 27 cells and applies the list's
-// tests to each candidate.  MODE is the particle's work class: 0 all pair
-// kinds, 1 no bond partners, 2 collisions only (the class guarantees the
-// list holds no other kinds).  The bond loop reads the particle's bonds from
-// memory one at a time, so its body is emitted once.
-#define SC_PLAIN_GROUP 4
-template <bool SCAN, int MODE>
-__device__ __forceinline__ void relax_item(const ScParams &P, const RelaxArgs &A, int i, int4 in, float4 v4, float4 r4,
+// The relaxation of a particle whose list overflowed or that holds a test
+// bond: its 27 cells are visited and the list's tests applied to each
+// candidate.  The bond loop reads the particle's bonds from memory one at a
+// time, so its body is emitted once; out of line, so that the lists' code
+// does not carry its registers.
+__device__ __noinline__ void relax_scan_item(const ScParams &P, const RelaxArgs &A, int i, int4 in, float4 v4, float4 r4,
                                            float4 a4) {
     float4 p4 = A.pos[i];
     const sc_f3 ppos = sc_make_f3(p4.x, p4.y, p4.z);
@@ -500,7 +521,7 @@ __device__ __forceinline__ void relax_item(const ScParams &P, const RelaxArgs &A
         const sc_f3 tpos = IM(sc_make_f3(t4.x, t4.y, t4.z));
         const float trad = t4.w;
         const float idist = prad + trad;
-        if (MODE <= 1 && (fl & SC_PP_POLAR)) {
+        if (fl & SC_PP_POLAR) {
             // dynamics.cuh:478-582: polar (lipid) head / tail attraction
             sc_f3 tvel = ld3(A.velIn, j);
             sc_f3 nextTup = sc_rotate(sc_rotate(sc_up(), ld4(A.rotIn, j)), pav);
@@ -514,7 +535,7 @@ __device__ __forceinline__ void relax_item(const ScParams &P, const RelaxArgs &A
             phobSum += pap;
             phobPos += tpPV * pap;
         }
-        if (MODE == 0 && (fl & SC_PP_PARTNER)) {
+        if (fl & SC_PP_PARTNER) {
             // dynamics.cuh:584-771: interaction partners, in bond-slot order
             int4 tin = A.info[j];
             const int tid_ = tin.x, ttype = tin.y;
@@ -598,55 +619,12 @@ __device__ __forceinline__ void relax_item(const ScParams &P, const RelaxArgs &A
             dV += (tpos - nd * cd + tvel - (ppos + pvel)) * 0.9f * trad / (prad + trad) * 1.0f;
         }
     };
-    if (SCAN) {
-        BondRegs B;
-        B.load(A.nb, A.bonds, i);
-        scan27(P, A.cellStart, ppos, reach(P, ppos, P.maxInt, SC_BINNED_P), [&](int j) {
-            uint32_t fl = pp_flags(P, IM, i, j, ppos, prad, phydro, B, A.pos, A.info);
-            if (fl) body(j, fl);
-        });
-    } else if (MODE == 2) {
-        // plain items list collisions only: the entries, then the
-        // neighbours' positions and velocities, of SC_PLAIN_GROUP pairs are
-        // loaded together, and the terms added in list order
-        const int c = A.L.cnt[i];
-        for (int k0 = 0; k0 < c; k0 += SC_PLAIN_GROUP) {
-            uint32_t e[SC_PLAIN_GROUP];
-            float4 t4[SC_PLAIN_GROUP], tv[SC_PLAIN_GROUP];
-#pragma unroll
-            for (int q = 0; q < SC_PLAIN_GROUP; q++)
-                e[q] = k0 + q < c ? A.L.list[sc_list_at(SC_LIST_PP, i, k0 + q)] : 0u;
-#pragma unroll
-            for (int q = 0; q < SC_PLAIN_GROUP; q++) {
-                t4[q] = make_float4(0, 0, 0, 0);
-                tv[q] = t4[q];
-                if (k0 + q < c) {
-                    const int j = (int)(e[q] & SC_PP_INDEX);
-                    t4[q] = A.pos[j];
-                    tv[q] = A.velIn[j];
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < SC_PLAIN_GROUP; q++) {
-                if (k0 + q < c && (e[q] & SC_PP_COLLIDE)) {
-                    // dynamics.cuh:775-786
-                    const sc_f3 tpos = IM(sc_make_f3(t4[q].x, t4[q].y, t4[q].z));
-                    const float trad = t4[q].w;
-                    sc_f3 nd = normalize(tpos - ppos);
-                    float cd = prad + trad;
-                    sc_f3 tvel = sc_make_f3(tv[q].x, tv[q].y, tv[q].z);
-                    w += 1.0f;
-                    dV += (tpos - nd * cd + tvel - (ppos + pvel)) * 0.9f * trad / (prad + trad) * 1.0f;
-                }
-            }
-        }
-    } else {
-        const int c = A.L.cnt[i];
-        for (int k = 0; k < c; k++) {
-            uint32_t e = A.L.list[sc_list_at(SC_LIST_PP, i, k)];
-            body((int)(e & SC_PP_INDEX), e);
-        }
-    }
+    BondRegs B;
+    B.load(A.nb, A.bonds, i);
+    scan27(P, A.cellStart, ppos, reach(P, ppos, P.maxInt, SC_BINNED_P), [&](int j) {
+        uint32_t fl = pp_flags(P, IM, i, j, ppos, prad, phydro, B, A.pos, A.info);
+        if (fl) body(j, fl);
+    });
     sc_f3 nv = pvel + dV / fmaxf(w, 1.0f);
     pav = sc_qmul(sc_slerp(sc_qid(), dAV, 1.0f / fmaxf(w, 1.0f)), pav);
     if (phobSum > 0.0f) {
@@ -659,78 +637,119 @@ __device__ __forceinline__ void relax_item(const ScParams &P, const RelaxArgs &A
     if (dbgTouched) st4(A.dbg, i, pdbg);
 }
 
-// A plain particle's relaxation (work class 2: collisions only, list path),
-// with every load that depends on the item alone already issued by the
-// caller (its records, its list count and its first SC_PLAIN_GROUP entries,
-// which lie in its list row whatever the count), so the item waits one
-// memory latency for them and one more for its neighbours.  The terms are
-// relax_item's for this class, in list order.
-__device__ __forceinline__ void relax_plain_item(const ScParams &P, const RelaxArgs &A, int i, float4 v4, float4 r4,
-                                                 float4 a4, float4 p4, int c, const uint32_t (&e0)[SC_PLAIN_GROUP]) {
+// The geometry of colliding entry k of item i with neighbour j, as k_build_pp
+// stores it for the first SC_GEO_PP entries ({A.x, A.y, A.z, radius}).
+__device__ __forceinline__ float4 collide_geo(const Imager &IM, sc_f3 ppos, float prad, float4 t4) {
+    const sc_f3 tpos = IM(sc_make_f3(t4.x, t4.y, t4.z));
+    const sc_f3 a = tpos - normalize(tpos - ppos) * (prad + t4.w);
+    return make_float4(a.x, a.y, a.z, t4.w);
+}
+// dynamics.cuh:775-786, the velocity term of a colliding pair (ppv the item's
+// position plus its velocity).
+__device__ __forceinline__ sc_f3 collide_term(float4 g, float4 tv, sc_f3 ppv, float prad) {
+    return (sc_make_f3(g.x, g.y, g.z) + sc_make_f3(tv.x, tv.y, tv.z) - ppv) * 0.9f * g.w / (prad + g.w) * 1.0f;
+}
+
+// The angular velocity of an item no bond or polar pair turns.  The
+// reference multiplies it by slerp(1, 1, t), t = 1 / max(w, 1) with w a count:
+// fl(1 - t) + t rounds to 1 for every such t, so the factor is exactly the
+// identity quaternion (0, 0, 0, 1), and the product changes nothing but the
+// sign of a zero component or non-finite values.  The product is formed until
+// both buffers hold it; when the second sub-iteration still changes a bit of
+// some item (A.unsettled), every later one forms it too.
+__device__ __forceinline__ void relax_still(const RelaxArgs &A, int i) {
+    if (A.age >= 2 && *A.unsettled == 0) return;
+    const float4 a4 = A.avIn[i];
+    const sc_f4 o = sc_qmul(sc_qid(), sc_make_f4(a4.x, a4.y, a4.z, a4.w));
+    A.avOut[i] = make_float4(o.x, o.y, o.z, o.w);
+    if (A.age == 1 && (sc_f2u(o.x) != sc_f2u(a4.x) || sc_f2u(o.y) != sc_f2u(a4.y) || sc_f2u(o.z) != sc_f2u(a4.z) ||
+                       sc_f2u(o.w) != sc_f2u(a4.w)))
+        *A.unsettled = 1;
+}
+
+// A plain particle's relaxation (work class 2: collisions only): its records,
+// its list count and its first SC_PLAIN_GROUP entries with their geometry lie
+// at places known from its index, so the item waits one memory latency for
+// them and one more for its neighbours' velocities.  Neither rot nor angvel
+// turns (relax_still), so from the third sub-iteration on only velocities
+// move: 56 bytes an item instead of 156, beside its pairs.
+#define SC_PLAIN_GROUP 4
+template <bool BATCH>
+__device__ __forceinline__ void relax_plain(const ScParams &P0, const RelaxArgs &A, int e) {
+    const int i = (int)((uint32_t)e & ~SC_CLASS_INACTIVE);
+    if ((uint32_t)e & SC_CLASS_INACTIVE) {
+        if (A.age == 0) {   // both buffers hold its records from then on
+            A.velOut[i] = A.velIn[i];
+            A.rotOut[i] = A.rotIn[i];
+            A.avOut[i] = A.avIn[i];
+        }
+        return;
+    }
+    const int c = A.L.cnt[i];
+    const float4 v4 = A.velIn[i], p4 = A.pos[i];
+    uint32_t en[SC_PLAIN_GROUP];
+    float4 g[SC_PLAIN_GROUP];
+#pragma unroll
+    for (int q = 0; q < SC_PLAIN_GROUP; q++) en[q] = A.L.list[sc_list_at(SC_LIST_PP, i, q)];
+    if (c > min(SC_LIST_PP, P0.listLimit)) return;   // left to the scan
     const sc_f3 ppos = sc_make_f3(p4.x, p4.y, p4.z);
-    const Imager IM(P, ppos, SC_BINNED_P);
     const float prad = p4.w;
     const sc_f3 pvel = sc_make_f3(v4.x, v4.y, v4.z);
-    sc_f4 pav = sc_make_f4(a4.x, a4.y, a4.z, a4.w);
+    const sc_f3 ppv = ppos + pvel;
     sc_f3 dV = sc_zero3();
-    const sc_f4 dAV = sc_qid();
-    float w = 0.0f;
-    uint32_t e[SC_PLAIN_GROUP];
-#pragma unroll
-    for (int q = 0; q < SC_PLAIN_GROUP; q++) e[q] = e0[q];
     for (int k0 = 0; k0 < c; k0 += SC_PLAIN_GROUP) {
         if (k0 > 0) {
 #pragma unroll
             for (int q = 0; q < SC_PLAIN_GROUP; q++)
-                e[q] = k0 + q < c ? A.L.list[sc_list_at(SC_LIST_PP, i, k0 + q)] : 0u;
+                en[q] = k0 + q < c ? A.L.list[sc_list_at(SC_LIST_PP, i, k0 + q)] : 0u;
         }
-        float4 t4[SC_PLAIN_GROUP], tv[SC_PLAIN_GROUP];
+        float4 tv[SC_PLAIN_GROUP];
+        const bool kept = k0 < SC_GEO_PP;
 #pragma unroll
         for (int q = 0; q < SC_PLAIN_GROUP; q++) {
-            t4[q] = make_float4(0, 0, 0, 0);
-            tv[q] = t4[q];
+            g[q] = make_float4(0, 0, 0, 0);
+            tv[q] = g[q];
             if (k0 + q < c) {
-                const int j = (int)(e[q] & SC_PP_INDEX);
-                t4[q] = A.pos[j];
+                const int j = (int)(en[q] & SC_PP_INDEX);
+                g[q] = kept ? A.geo[sc_list_at(SC_GEO_PP, i, k0 + q)] : A.pos[j];
                 tv[q] = A.velIn[j];
             }
         }
+        if (!kept) {
+            ScParams P = P0;
+            if (BATCH) rep_apply<BATCH>(P, A.info[i].w);
+            const Imager IM(P, ppos, SC_BINNED_P);
 #pragma unroll
-        for (int q = 0; q < SC_PLAIN_GROUP; q++) {
-            if (k0 + q < c && (e[q] & SC_PP_COLLIDE)) {
-                // dynamics.cuh:775-786
-                const sc_f3 tpos = IM(sc_make_f3(t4[q].x, t4[q].y, t4[q].z));
-                const float trad = t4[q].w;
-                sc_f3 nd = normalize(tpos - ppos);
-                float cd = prad + trad;
-                sc_f3 tvel = sc_make_f3(tv[q].x, tv[q].y, tv[q].z);
-                w += 1.0f;
-                dV += (tpos - nd * cd + tvel - (ppos + pvel)) * 0.9f * trad / (prad + trad) * 1.0f;
-            }
+            for (int q = 0; q < SC_PLAIN_GROUP; q++)
+                if (k0 + q < c) g[q] = collide_geo(IM, ppos, prad, g[q]);
         }
+#pragma unroll
+        for (int q = 0; q < SC_PLAIN_GROUP; q++)
+            if (k0 + q < c) dV += collide_term(g[q], tv[q], ppv, prad);
     }
-    sc_f3 nv = pvel + dV / fmaxf(w, 1.0f);
-    pav = sc_qmul(sc_slerp(sc_qid(), dAV, 1.0f / fmaxf(w, 1.0f)), pav);
-    st3(A.velOut, i, nv, v4.w);
-    A.rotOut[i] = r4;
-    st4(A.avOut, i, pav);
+    st3(A.velOut, i, pvel + dV / fmaxf((float)c, 1.0f), v4.w);
+    if (A.age == 0) A.rotOut[i] = A.rotIn[i];
+    relax_still(A, i);
 }
 
-// A polar particle's relaxation (work class 1: polar and collision pairs,
-// list path): relax_item's terms for this class in list order, with the
-// entries of SC_POLAR_GROUP pairs, then their neighbours' positions,
-// velocities and (polar pairs) rotations, loaded together.
+// A polar particle's relaxation (work class 1: polar and collision pairs):
+// the terms in list order, with the entries of SC_POLAR_GROUP pairs, then
+// their neighbours' records, loaded together.
 #define SC_POLAR_GROUP 2
-__device__ __forceinline__ void relax_polar_item(const ScParams &P, const RelaxArgs &A, int i, int4 in, float4 v4,
-                                                 float4 r4, float4 a4, float4 p4, int c) {
+template <bool BATCH>
+__device__ __forceinline__ void relax_polar(const ScParams &P0, const RelaxArgs &A, int i) {
+    const int c = A.L.cnt[i];
+    const float4 v4 = A.velIn[i], r4 = A.rotIn[i], a4 = A.avIn[i], p4 = A.pos[i];
+    if (c > min(SC_LIST_PP, P0.listLimit)) return;   // left to the scan
+    ScParams P = P0;
+    if (BATCH) rep_apply<BATCH>(P, A.info[i].w);
     const sc_f3 ppos = sc_make_f3(p4.x, p4.y, p4.z);
     const Imager IM(P, ppos, SC_BINNED_P);
     const float prad = p4.w;
     const sc_f3 pvel = sc_make_f3(v4.x, v4.y, v4.z);
+    const sc_f3 ppv = ppos + pvel;
     const sc_f4 prot = sc_make_f4(r4.x, r4.y, r4.z, r4.w);
     sc_f4 pav = sc_make_f4(a4.x, a4.y, a4.z, a4.w);
-    const int phydro = (int)(int8_t)(in.w & 0xff);
-    (void)phydro;
     sc_f3 dV = sc_zero3();
     const sc_f4 dAV = sc_qid();
     sc_f3 phobPos = sc_zero3();
@@ -759,11 +778,11 @@ __device__ __forceinline__ void relax_polar_item(const ScParams &P, const RelaxA
         for (int q = 0; q < SC_POLAR_GROUP; q++) {
             if (k0 + q >= c) break;
             const uint32_t fl = e[q];
-            const sc_f3 tpos = IM(sc_make_f3(t4[q].x, t4[q].y, t4[q].z));
             const float trad = t4[q].w;
-            const sc_f3 tvel = sc_make_f3(tv[q].x, tv[q].y, tv[q].z);
             if (fl & SC_PP_POLAR) {
                 // dynamics.cuh:478-582: polar (lipid) head / tail attraction
+                const sc_f3 tpos = IM(sc_make_f3(t4[q].x, t4[q].y, t4[q].z));
+                const sc_f3 tvel = sc_make_f3(tv[q].x, tv[q].y, tv[q].z);
                 sc_f3 nextTup = sc_rotate(sc_rotate(sc_up(), sc_make_f4(tr[q].x, tr[q].y, tr[q].z, tr[q].w)), pav);
                 sc_f3 pPV = -nextUp * prad + ppos + pvel;
                 sc_f3 tpPV = -nextTup * trad + tpos + tvel;
@@ -776,11 +795,8 @@ __device__ __forceinline__ void relax_polar_item(const ScParams &P, const RelaxA
                 phobPos += tpPV * pap;
             }
             if (fl & SC_PP_COLLIDE) {
-                // dynamics.cuh:775-786: soft collision with a non-partner
-                sc_f3 nd = normalize(tpos - ppos);
-                float cd = prad + trad;
                 w += 1.0f;
-                dV += (tpos - nd * cd + tvel - (ppos + pvel)) * 0.9f * trad / (prad + trad) * 1.0f;
+                dV += collide_term(collide_geo(IM, ppos, prad, t4[q]), tv[q], ppv, prad);
             }
         }
     }
@@ -791,260 +807,353 @@ __device__ __forceinline__ void relax_polar_item(const ScParams &P, const RelaxA
         pav = sc_slerp(pav, sc_quat_from_to(-up, dir), 0.2f);
     }
     st3(A.velOut, i, nv, v4.w);
-    A.rotOut[i] = r4;
+    if (A.age == 0) A.rotOut[i] = r4;
     st4(A.avOut, i, pav);
 }
 
-// A bonded particle's relaxation (work class 0, list path).  The pose terms
-// of its rule and chain bonds do not depend on the running sums, so they are
-// evaluated first, from its bond matches (k_build_pp records them in the
-// order the reference meets them), with every lane of a warp on its own
-// first bond, then its second ...  Only bond terms turn dAV and move the
-// debug vector, so those two chains are carried along in the same pass (the
-// matches come in list order); what remains per bond is its velocity term,
-// and the list is then walked once to add every velocity term in the
-// reference's order.  A test bond rotates the particle itself, which later
-// terms read: such particles (SC_MATCH_INORDER) take the in-order scan of
-// k_relax_overflow.
-//
-// Bound: the latency of one item's instruction chain (a few warps per
-// scheduler at most).  With the slerp of dAV inside the list walk, where a
-// warp's lanes meet their partners at different entries, nearly every round
-// of the walk ran it.
-
-__device__ __forceinline__ void relax_bonded_item(const ScParams &P, const RelaxArgs &A, int i, int4 in, float4 v4,
-                                                  float4 r4, float4 a4) {
-    const int *__restrict__ myBonds = A.bonds + (size_t)i * 24;
-    float4 p4 = A.pos[i];
-    const sc_f3 ppos = sc_make_f3(p4.x, p4.y, p4.z);
-    const Imager IM(P, ppos, SC_BINNED_P);
-    const float prad = p4.w;
-    const sc_f3 pvel = sc_make_f3(v4.x, v4.y, v4.z);
-    const sc_f4 prot = sc_make_f4(r4.x, r4.y, r4.z, r4.w);
-    sc_f4 pav = sc_make_f4(a4.x, a4.y, a4.z, a4.w);
-    const int pid = in.x, ptype = in.y;
-    const sc_f3 up = sc_rotate(sc_up(), prot);
-    const sc_f3 nextUp = sc_rotate(up, pav);
-    const float flex = SC_PI_REF / 8;
-    const int c = A.L.cnt[i];
-    // 1. the terms of its bond matches (list order, then bond-slot order)
-    const uint32_t *__restrict__ myMatch = A.match + (size_t)i * SC_MAX_ACTIVE_INTERACTIONS;
-    const int nm = min(A.matchN[i] & SC_MATCH_COUNT, SC_MAX_ACTIVE_INTERACTIONS);
-    // the first velocity term stays in registers (most bonded items have
-    // one); the rest go to a per-thread array
-    sc_f3 T0 = sc_zero3(), T[SC_MAX_ACTIVE_INTERACTIONS - 1];
-    int nt = 0;
-    sc_f4 pdbg = sc_make_f4(0, 0, 0, 0);
-    bool dbgTouched = false;
-    sc_f4 dAV = sc_qid();
-    for (int m = 0; m < nm; m++) {
-        const uint32_t me = myMatch[m];
-        const int j = (int)(me & SC_PP_INDEX), k = (int)(me >> 29);
-        const int it = myBonds[3 * k];
-        if (!(it >= 10 || it == SC_INTERACTION_TYPE_CHAIN) || nt >= SC_MAX_ACTIVE_INTERACTIONS) continue;
-        const int4 tin = A.info[j];
-        const int tid_ = tin.x, ttype = tin.y;
-        const float4 t4 = A.pos[j];
-        const sc_f3 tpos = IM(sc_make_f3(t4.x, t4.y, t4.z));
-        const float trad = t4.w, idist = prad + trad;
-        const sc_f4 trot = ld4(A.rotIn, j), tav = ld4(A.avIn, j);
-        const sc_f3 tvel = ld3(A.velIn, j);
-        sc_f3 dv;
-        sc_f4 q;
-        if (it >= 10) {
-            // dynamics.cuh:591-655
-            const sc_rule &pii = rule_at(P, it);
-            sc_f4 ro = rule_ori(pii);
-            sc_f3 rp = rule_pos(pii);
-            bool o1 = p_order(ptype, pid, ttype, tid_), o2 = p_order(ttype, tid_, ptype, pid);
-            sc_f4 tro_p = o1 ? sc_qmul(trot, sc_qinv(ro)) : sc_qmul(trot, ro);
-            sc_f4 tro_t = o2 ? sc_qmul(prot, sc_qinv(ro)) : sc_qmul(prot, ro);
-            sc_f4 rro = sc_qmul(sc_qinv(sc_qmul(pav, prot)), sc_qmul(tav, tro_p));
-            sc_f4 orro = sc_qmul(sc_qinv(sc_qmul(tav, trot)), sc_qmul(pav, tro_t));
-            q = sc_qmul(sc_slerp(rro, orro, 0.5f), rro);
-            sc_f3 rrp = o1 ? sc_rotate(-rp, sc_qmul(sc_qinv(ro), sc_qmul(tav, trot))) : sc_rotate(rp, sc_qmul(tav, trot));
-            rrp += tpos;
-            sc_f3 orrp = o2 ? sc_rotate(-rp, sc_qmul(sc_qinv(ro), sc_qmul(pav, prot))) : sc_rotate(rp, sc_qmul(pav, prot));
-            orrp += ppos;
-            sc_f3 pDV = (rrp + tvel - (ppos + pvel)) * 0.9f * trad / (prad + trad) * 1.0f;
-            sc_f3 tpDV = (orrp + pvel - (tpos + tvel)) * 0.9f * prad / (prad + trad) * 1.0f;
-            dv = (pDV - (pDV + tpDV) / 2.0f) * 0.9f * prad / (prad + trad) * 1.0f;
-        } else {
-            // dynamics.cuh:692-769
-            sc_f3 nextTup = sc_rotate(sc_rotate(sc_up(), trot), pav);
-            sc_f3 nnd = normalize(tpos + tvel - (ppos + pvel));
-            bool fwd = myBonds[3 * k + 1] == SC_INTERACTION_GROUP_FORWARD;
-            q = sc_quat_from_to(nextUp, (fwd ? -1.0f : 1.0f) * nnd);
-            sc_f3 relUp = (fwd ? 1.0f : -1.0f) * nextTup;
-            sc_f3 axis = sc_safe_cross(relUp, -nnd);
-            float ang = sc_angle3(relUp, -nnd);
-            sc_f3 rrp = sc_rotate(relUp, sc_quat(axis, fminf(fmaxf(ang, -flex), flex)));
-            rrp *= idist;
-            rrp += tpos;
-            sc_f3 oUp = (fwd ? -1.0f : 1.0f) * nextUp;
-            sc_f3 oaxis = sc_safe_cross(oUp, nnd);
-            float oang = sc_angle3(oUp, nnd);
-            sc_f3 orrp = sc_rotate(oUp, sc_quat(oaxis, fminf(fmaxf(oang, -flex), flex)));
-            orrp *= idist;
-            orrp += ppos;
-            sc_f3 pDV = (rrp + tvel - (ppos + pvel)) * 0.9f * trad / (prad + trad) * 1.0f;
-            sc_f3 tpDV = (orrp + pvel - (tpos + tvel)) * 0.9f * prad / (prad + trad) * 1.0f;
-            dv = (pDV - (pDV + tpDV) / 2.0f) * 0.9f * prad / (prad + trad) * 1.0f;
-            const sc_f3 dd = rrp - ppos;
-            if (!dbgTouched) {
-                pdbg = ld4(A.dbg, i);
-                dbgTouched = true;
-            }
-            pdbg.x = (float)((double)pdbg.x + (double)dd.x * (1.0 - (double)0.9f));
-            pdbg.y = (float)((double)pdbg.y + (double)dd.y * (1.0 - (double)0.9f));
-            pdbg.z = (float)((double)pdbg.z + (double)dd.z * (1.0 - (double)0.9f));
-        }
-        dAV = sc_slerp(dAV, q, 0.9f * trad / (prad + trad));
-        if (nt == 0)
-            T0 = dv;
-        else
-            T[nt - 1] = dv;
-        nt++;
-    }
-    // 2. every velocity term in the reference's order
-    sc_f3 dV = sc_zero3();
-    sc_f3 phobPos = sc_zero3();
-    float phobSum = 0.0f;
-    float w = 0.0f;
-    int ut = 0, mi = 0;
-    for (int kk = 0; kk < c; kk++) {
-        const uint32_t fl = A.L.list[sc_list_at(SC_LIST_PP, i, kk)];
-        const int j = (int)(fl & SC_PP_INDEX);
-        float4 t4 = A.pos[j];
-        const sc_f3 tpos = IM(sc_make_f3(t4.x, t4.y, t4.z));
-        const float trad = t4.w;
-        if (fl & SC_PP_POLAR) {
-            sc_f3 tvel = ld3(A.velIn, j);
-            sc_f3 nextTup = sc_rotate(sc_rotate(sc_up(), ld4(A.rotIn, j)), pav);
-            sc_f3 pPV = -nextUp * prad + ppos + pvel;
-            sc_f3 tpPV = -nextTup * trad + tpos + tvel;
-            float Lr = length(tpPV - pPV) / (prad + trad);
-            float attr = sc_polar_attr(Lr);
-            w += 1.0f;
-            dV += (tpPV - pPV) * 0.05f * attr * 1.0f;
-            float pap = sc_powf(fminf(1.0f / fmaxf(Lr, 1e-6f), 10.0f) / 10.0f, 0.2f);
-            phobSum += pap;
-            phobPos += tpPV * pap;
-        }
-        if (fl & SC_PP_PARTNER) {
-            // this neighbour's bond matches are the next ones in order
-            for (; mi < nm && (int)(myMatch[mi] & SC_PP_INDEX) == j; mi++) {
-                const int it = myBonds[3 * (int)(myMatch[mi] >> 29)];
-                if ((it >= 10 || it == SC_INTERACTION_TYPE_CHAIN) && ut < nt) {
-                    w += 1.0f;
-                    dV += ut == 0 ? T0 : T[ut - 1];
-                    ut++;
+// The bonded class's items in the order its blocks relax them: each block of
+// SC_BOND_ITEMS ranked by bond-match count, chain-bonded items apart from
+// rule-bonded ones (their pose terms are different code), so that a warp's
+// lanes walk about as many bond terms of the same kind, with what an item's
+// first loads depend on beside its index:
+//   x  the item (-1: left to the scan)
+//   y  its first bond match (k_build_pp; ~0: none)
+//   z  that bond's interaction type
+//   w  match count (bits 0-3) | first bond forward (4) | has polar pairs (5) |
+//      list count (8-15) | terms in all (16-31)
+#define SC_BOND_ITEMS (SC_THREADS / 2)
+__global__ void __launch_bounds__(SC_THREADS) k_bond_plan(ScParams P, PairList<SC_LIST_PP> L,
+                                                          const int *__restrict__ classIdx,
+                                                          const int *__restrict__ classCount,
+                                                          const int *__restrict__ bonds,
+                                                          const uint32_t *__restrict__ match,
+                                                          const int *__restrict__ matchN, uint4 *__restrict__ rec) {
+    __shared__ uint4 s_rec[SC_THREADS];
+    const int n = classCount[0];
+    for (int base = blockIdx.x * SC_THREADS; base < n; base += gridDim.x * SC_THREADS) {
+        const int t = base + threadIdx.x;
+        int key = 0;
+        if (t < n) {
+            const int i = classIdx[t];
+            const int c = L.cnt[i];
+            uint4 r = make_uint4(0xffffffffu, 0xffffffffu, 0u, 0u);
+            if (c <= min(SC_LIST_PP, P.listLimit) && !(matchN[i] & SC_MATCH_INORDER)) {
+                const int nm = min(matchN[i] & SC_MATCH_COUNT, SC_MAX_ACTIVE_INTERACTIONS);
+                const int *__restrict__ b = bonds + (size_t)i * 24;
+                int terms = 0;
+                uint32_t any = 0;
+                for (int k = 0; k < c; k++) {
+                    const uint32_t e = L.list[sc_list_at(SC_LIST_PP, i, k)];
+                    any |= e;
+                    terms += ((e & SC_PP_POLAR) != 0) + ((e & SC_PP_COLLIDE) != 0);
                 }
+                const uint32_t *__restrict__ m = match + (size_t)i * SC_MAX_ACTIVE_INTERACTIONS;
+                for (int k = 0; k < nm; k++) {
+                    const int it = b[3 * (int)(m[k] >> 29)];
+                    terms += it >= 10 || it == SC_INTERACTION_TYPE_CHAIN;
+                }
+                r.x = (uint32_t)i;
+                uint32_t fwd = 0;
+                if (nm > 0) {
+                    const int k = (int)(m[0] >> 29);
+                    r.y = m[0];
+                    r.z = (uint32_t)b[3 * k];
+                    fwd = b[3 * k + 1] == SC_INTERACTION_GROUP_FORWARD;
+                }
+                r.w = (uint32_t)nm | (fwd << 4) | ((any & SC_PP_POLAR) ? 1u << 5 : 0u) | ((uint32_t)c << 8) |
+                      ((uint32_t)terms << 16);
             }
+            key = (matchN[i] & SC_MATCH_COUNT) +
+                  (bonds[(size_t)i * 24] == SC_INTERACTION_TYPE_CHAIN ? SC_MAX_ACTIVE_INTERACTIONS + 1 : 0);
+            s_rec[threadIdx.x] = r;
         }
-        if (fl & SC_PP_COLLIDE) {
-            sc_f3 nd = normalize(tpos - ppos);
-            float cd = prad + trad;
-            sc_f3 tvel = ld3(A.velIn, j);
-            w += 1.0f;
-            dV += (tpos - nd * cd + tvel - (ppos + pvel)) * 0.9f * trad / (prad + trad) * 1.0f;
-        }
+        int src, cs;
+        count_rank<2 * SC_MAX_ACTIVE_INTERACTIONS + 1>(t < n, key, &src, &cs);
+        if (cs >= 0) rec[t] = s_rec[src];
+        __syncthreads();  // the shared arrays are reused by the next round
     }
-    sc_f3 nv = pvel + dV / fmaxf(w, 1.0f);
-    pav = sc_qmul(sc_slerp(sc_qid(), dAV, 1.0f / fmaxf(w, 1.0f)), pav);
-    if (phobSum > 0.0f) {
-        sc_f3 dir = normalize(phobPos / phobSum - (ppos + nv));
-        pav = sc_slerp(pav, sc_quat_from_to(-up, dir), 0.2f);
-    }
-    st3(A.velOut, i, nv, v4.w);
-    st4(A.rotOut, i, prot);
-    st4(A.avOut, i, pav);
-    if (dbgTouched) st4(A.dbg, i, pdbg);
 }
 
-// One item of a work class (the items whose list overflowed, and bonded
-// items with a test bond, are left to k_relax_overflow).
-template <int MODE, bool BATCH>
-__device__ __forceinline__ void relax_class_item(const ScParams &P0, const RelaxArgs &A, int i) {
-    if (MODE == 2) {
+// One bond of a bonded particle: what its pose terms read of the neighbour.
+struct BondPair {
+    int it;          // interaction type
+    bool fwd;        // chain bonds: this particle's side
+    bool o1, o2;     // rule bonds: p_order both ways
+    sc_f3 tpos, tvel;
+    float trad;
+    sc_f4 trot, tav;
+};
+struct BondSelf {
+    sc_f3 ppos, pvel, nextUp;
+    float prad;
+    sc_f4 prot, pav;
+};
+__device__ __forceinline__ bool bond_turns(int it) { return it >= 10 || it == SC_INTERACTION_TYPE_CHAIN; }
+
+// The slerp target of dAV (dynamics.cuh:591-622, 700-712).
+__device__ __forceinline__ sc_f4 bond_target(const ScParams &P, const BondSelf &S, const BondPair &b) {
+    if (b.it >= 10) {
+        const sc_f4 ro = rule_ori(rule_at(P, b.it));
+        sc_f4 tro_p = b.o1 ? sc_qmul(b.trot, sc_qinv(ro)) : sc_qmul(b.trot, ro);
+        sc_f4 tro_t = b.o2 ? sc_qmul(S.prot, sc_qinv(ro)) : sc_qmul(S.prot, ro);
+        sc_f4 rro = sc_qmul(sc_qinv(sc_qmul(S.pav, S.prot)), sc_qmul(b.tav, tro_p));
+        sc_f4 orro = sc_qmul(sc_qinv(sc_qmul(b.tav, b.trot)), sc_qmul(S.pav, tro_t));
+        return sc_qmul(sc_slerp(rro, orro, 0.5f), rro);
+    }
+    sc_f3 nnd = normalize(b.tpos + b.tvel - (S.ppos + S.pvel));
+    return sc_quat_from_to(S.nextUp, (b.fwd ? -1.0f : 1.0f) * nnd);
+}
+
+// The velocity term (dynamics.cuh:623-655, 713-769); chain bonds also give
+// rrp - ppos for the debug vector.
+__device__ __forceinline__ sc_f3 bond_velocity(const ScParams &P, const BondSelf &S, const BondPair &b, sc_f3 *dd) {
+    const float prad = S.prad, trad = b.trad, idist = prad + trad;
+    const sc_f3 ppos = S.ppos, pvel = S.pvel;
+    sc_f3 rrp, orrp;
+    if (b.it >= 10) {
+        const sc_rule &pii = rule_at(P, b.it);
+        const sc_f4 ro = rule_ori(pii);
+        const sc_f3 rp = rule_pos(pii);
+        rrp = b.o1 ? sc_rotate(-rp, sc_qmul(sc_qinv(ro), sc_qmul(b.tav, b.trot))) : sc_rotate(rp, sc_qmul(b.tav, b.trot));
+        rrp += b.tpos;
+        orrp = b.o2 ? sc_rotate(-rp, sc_qmul(sc_qinv(ro), sc_qmul(S.pav, S.prot))) : sc_rotate(rp, sc_qmul(S.pav, S.prot));
+        orrp += ppos;
+    } else {
+        const float flex = SC_PI_REF / 8;
+        sc_f3 nextTup = sc_rotate(sc_rotate(sc_up(), b.trot), S.pav);
+        sc_f3 nnd = normalize(b.tpos + b.tvel - (ppos + pvel));
+        sc_f3 relUp = (b.fwd ? 1.0f : -1.0f) * nextTup;
+        sc_f3 axis = sc_safe_cross(relUp, -nnd);
+        float ang = sc_angle3(relUp, -nnd);
+        rrp = sc_rotate(relUp, sc_quat(axis, fminf(fmaxf(ang, -flex), flex)));
+        rrp *= idist;
+        rrp += b.tpos;
+        sc_f3 oUp = (b.fwd ? -1.0f : 1.0f) * S.nextUp;
+        sc_f3 oaxis = sc_safe_cross(oUp, nnd);
+        float oang = sc_angle3(oUp, nnd);
+        orrp = sc_rotate(oUp, sc_quat(oaxis, fminf(fmaxf(oang, -flex), flex)));
+        orrp *= idist;
+        orrp += ppos;
+        *dd = rrp - ppos;
+    }
+    sc_f3 pDV = (rrp + b.tvel - (ppos + pvel)) * 0.9f * trad / (prad + trad) * 1.0f;
+    sc_f3 tpDV = (orrp + pvel - (b.tpos + b.tvel)) * 0.9f * prad / (prad + trad) * 1.0f;
+    return (pDV - (pDV + tpDV) / 2.0f) * 0.9f * prad / (prad + trad) * 1.0f;
+}
+
+// A block of bonded particles (work class 0): SC_BOND_ITEMS items, each
+// relaxed by two threads in different warps.  Only bond terms turn dAV, and
+// the velocity needs none of it, so the block's first half of threads carries
+// the orientation -- the slerp targets of the item's bond matches and dAV's
+// chain over them -- and the second half the velocity: the matches' velocity
+// terms, then the list walked once to add every term in the reference's order
+// (a test bond rotates the particle itself, which later terms read: such
+// particles take the in-order scan).  The divisor of dAV's last slerp is a
+// count the plan knows.  An item with polar pairs turns once more, towards
+// its neighbours, when its velocity is known: its second thread finishes it
+// with the first one's quaternion.
+//
+// Bound: the latency of one item's instruction chain, at a few warps per
+// scheduler; two threads per item cut the chain in two, and the record takes
+// two dependent loads out of it.  The class alone, 524,288 + 2,097,152 items
+// (a quarter of the large workload): 37 -> 22 us a launch.
+template <bool BATCH>
+__device__ __forceinline__ void relax_bonded_block(const ScParams &P0, const RelaxArgs &A, int base, int n,
+                                                   float4 *s_av) {
+    const bool turner = threadIdx.x < SC_BOND_ITEMS;
+    const int slot = turner ? threadIdx.x : threadIdx.x - SC_BOND_ITEMS;
+    const int t = base + slot;
+    const uint4 r = t < n ? A.bondRec[t] : make_uint4(0xffffffffu, 0, 0, 0);
+    const int i = (int)r.x;
+    const bool polar = (r.w >> 5) & 1u;
+    sc_f3 up = sc_zero3(), towards = sc_zero3(), newPos = sc_zero3();
+    float phobSum = 0.0f;
+    if (i >= 0) {
+        const int nm = (int)(r.w & 15u), c = (int)((r.w >> 8) & 0xffu);
+        const float4 p4 = A.pos[i], v4 = A.velIn[i], r4 = A.rotIn[i], a4 = A.avIn[i];
         const int4 in = A.info[i];
-        const float4 v4 = A.velIn[i], r4 = A.rotIn[i], a4 = A.avIn[i], p4 = A.pos[i];
-        const int c = A.L.cnt[i];
-        uint32_t e0[SC_PLAIN_GROUP];
-#pragma unroll
-        for (int q = 0; q < SC_PLAIN_GROUP; q++) e0[q] = A.L.list[sc_list_at(SC_LIST_PP, i, q)];
-        if (!(in.z & SC_ACTIVE)) {
-            A.velOut[i] = v4;
-            A.rotOut[i] = r4;
-            A.avOut[i] = a4;
-            return;
-        }
         ScParams P = P0;
         rep_apply<BATCH>(P, in.w);
-        if (c > min(SC_LIST_PP, P.listLimit)) return;
-        relax_plain_item(P, A, i, v4, r4, a4, p4, c, e0);
-        return;
-    }
-    int4 in = A.info[i];
-    float4 v4 = A.velIn[i], r4 = A.rotIn[i], a4 = A.avIn[i];
-    if (!(in.z & SC_ACTIVE)) {
-        A.velOut[i] = v4;
-        A.rotOut[i] = r4;
-        A.avOut[i] = a4;
-        return;
-    }
-    ScParams P = P0;
-    rep_apply<BATCH>(P, in.w);
-    if (A.L.cnt[i] > min(SC_LIST_PP, P.listLimit)) return;
-    if (MODE == 0) {
-        if (!(A.matchN[i] & SC_MATCH_INORDER)) relax_bonded_item(P, A, i, in, v4, r4, a4);
-    } else {
-        relax_polar_item(P, A, i, in, v4, r4, a4, A.pos[i], A.L.cnt[i]);
-    }
-}
-
-// The items of one work class, grid-stride over the class's index segment.
-// The bonded class goes block by block, its items ranked by bond-match
-// count (chain-bonded apart from rule-bonded) inside the block, so a warp's
-// lanes walk about as many bond terms of the same kind (items with more
-// bonds would otherwise hold back the rest of their warp).
-template <int MODE, bool BATCH>
-__global__ void __launch_bounds__(SC_THREADS, MODE == 0 ? 2 : 4) k_relax(ScParams P, RelaxArgs A) {
-    const int n = A.classCount[MODE];
-    const int *__restrict__ idx = A.classIdx + (size_t)MODE * A.L.cap;
-    if (MODE == 0) {
-        __shared__ int s_item[SC_THREADS];
-        for (int base = blockIdx.x * SC_THREADS; base < n; base += gridDim.x * SC_THREADS) {
-            const int t = base + threadIdx.x;
-            const int i = t < n ? idx[t] : -1;
-            s_item[threadIdx.x] = i;
-            // rank key: bond-match count, chain-bonded items apart from rule-bonded ones (their
-            // pose terms are different code)
-            int key = 0;
-            if (i >= 0)
-                key = (A.matchN[i] & SC_MATCH_COUNT) +
-                      (A.bonds[(size_t)i * 24] == SC_INTERACTION_TYPE_CHAIN ? SC_MAX_ACTIVE_INTERACTIONS + 1 : 0);
-            int src, cs;
-            count_rank<2 * SC_MAX_ACTIVE_INTERACTIONS + 1>(i >= 0, key, &src, &cs);
-            if (cs >= 0) relax_class_item<MODE, BATCH>(P, A, s_item[src]);
-            __syncthreads();  // the ranking's shared arrays are reused by the next round
+        BondSelf S;
+        S.ppos = sc_make_f3(p4.x, p4.y, p4.z);
+        S.prad = p4.w;
+        S.pvel = sc_make_f3(v4.x, v4.y, v4.z);
+        S.prot = sc_make_f4(r4.x, r4.y, r4.z, r4.w);
+        S.pav = sc_make_f4(a4.x, a4.y, a4.z, a4.w);
+        const Imager IM(P, S.ppos, SC_BINNED_P);
+        const uint32_t *__restrict__ myMatch = A.match + (size_t)i * SC_MAX_ACTIVE_INTERACTIONS;
+        const int *__restrict__ myBonds = A.bonds + (size_t)i * 24;
+        auto pair_of = [&](int m, BondPair &b) {
+            const uint32_t me = m == 0 ? r.y : myMatch[m];
+            const int j = (int)(me & SC_PP_INDEX), k = (int)(me >> 29);
+            b.it = m == 0 ? (int)r.z : myBonds[3 * k];
+            if (!bond_turns(b.it)) return false;
+            b.fwd = m == 0 ? (r.w >> 4) & 1u : myBonds[3 * k + 1] == SC_INTERACTION_GROUP_FORWARD;
+            const int4 tin = A.info[j];
+            const float4 t4 = A.pos[j];
+            b.tpos = IM(sc_make_f3(t4.x, t4.y, t4.z));
+            b.trad = t4.w;
+            b.trot = ld4(A.rotIn, j);
+            b.tav = ld4(A.avIn, j);
+            b.tvel = ld3(A.velIn, j);
+            b.o1 = p_order(in.y, in.x, tin.y, tin.x);
+            b.o2 = p_order(tin.y, tin.x, in.y, in.x);
+            return true;
+        };
+        up = sc_rotate(sc_up(), S.prot);
+        S.nextUp = sc_rotate(up, S.pav);
+        if (turner) {
+            sc_f4 dAV = sc_qid();
+            for (int m = 0; m < nm; m++) {
+                BondPair b;
+                if (!pair_of(m, b)) continue;
+                dAV = sc_slerp(dAV, bond_target(P, S, b), 0.9f * b.trad / (S.prad + b.trad));
+            }
+            const sc_f4 pav = sc_qmul(sc_slerp(sc_qid(), dAV, 1.0f / fmaxf((float)(r.w >> 16), 1.0f)), S.pav);
+            if (polar) s_av[slot] = make_float4(pav.x, pav.y, pav.z, pav.w);
+            else st4(A.avOut, i, pav);
+        } else {
+            const sc_f3 ppv = S.ppos + S.pvel;
+            // 1. the bonds' velocity terms: the first stays in registers (most
+            // bonded items have one), the rest go to a per-thread array
+            sc_f3 T0 = sc_zero3(), T[SC_MAX_ACTIVE_INTERACTIONS - 1];
+            sc_f4 pdbg = sc_make_f4(0, 0, 0, 0);
+            bool dbgTouched = false;
+            int nt = 0;
+            for (int m = 0; m < nm; m++) {
+                BondPair b;
+                if (!pair_of(m, b)) continue;
+                sc_f3 dd = sc_zero3();
+                const sc_f3 dv = bond_velocity(P, S, b, &dd);
+                if (b.it == SC_INTERACTION_TYPE_CHAIN) {
+                    if (!dbgTouched) {
+                        pdbg = ld4(A.dbg, i);
+                        dbgTouched = true;
+                    }
+                    pdbg.x = (float)((double)pdbg.x + (double)dd.x * (1.0 - (double)0.9f));
+                    pdbg.y = (float)((double)pdbg.y + (double)dd.y * (1.0 - (double)0.9f));
+                    pdbg.z = (float)((double)pdbg.z + (double)dd.z * (1.0 - (double)0.9f));
+                }
+                if (nt == 0) T0 = dv;
+                else T[nt - 1] = dv;
+                nt++;
+            }
+            if (dbgTouched) st4(A.dbg, i, pdbg);
+            // 2. every velocity term in the reference's order
+            sc_f3 dV = sc_zero3(), phobPos = sc_zero3();
+            int ut = 0, mi = 0;
+            for (int k0 = 0; k0 < c; k0 += SC_POLAR_GROUP) {
+                uint32_t e[SC_POLAR_GROUP];
+                float4 g[SC_POLAR_GROUP], tv[SC_POLAR_GROUP];
+                const bool kept = k0 < SC_GEO_PP;
+#pragma unroll
+                for (int q = 0; q < SC_POLAR_GROUP; q++)
+                    e[q] = k0 + q < c ? A.L.list[sc_list_at(SC_LIST_PP, i, k0 + q)] : 0u;
+#pragma unroll
+                for (int q = 0; q < SC_POLAR_GROUP; q++) {
+                    g[q] = make_float4(0, 0, 0, 0);
+                    tv[q] = g[q];
+                    if (e[q] & SC_PP_COLLIDE)
+                        g[q] = kept ? A.geo[sc_list_at(SC_GEO_PP, i, k0 + q)] : A.pos[(int)(e[q] & SC_PP_INDEX)];
+                    if (e[q] & (SC_PP_COLLIDE | SC_PP_POLAR)) tv[q] = A.velIn[(int)(e[q] & SC_PP_INDEX)];
+                }
+#pragma unroll
+                for (int q = 0; q < SC_POLAR_GROUP; q++) {
+                    const uint32_t fl = e[q];
+                    const int j = (int)(fl & SC_PP_INDEX);
+                    if (fl & SC_PP_POLAR) {
+                        // dynamics.cuh:478-582
+                        const float4 t4 = A.pos[j];
+                        const sc_f3 tpos = IM(sc_make_f3(t4.x, t4.y, t4.z));
+                        const float trad = t4.w;
+                        const sc_f3 tvel = sc_make_f3(tv[q].x, tv[q].y, tv[q].z);
+                        sc_f3 nextTup = sc_rotate(sc_rotate(sc_up(), ld4(A.rotIn, j)), S.pav);
+                        sc_f3 pPV = -S.nextUp * S.prad + S.ppos + S.pvel;
+                        sc_f3 tpPV = -nextTup * trad + tpos + tvel;
+                        float Lr = length(tpPV - pPV) / (S.prad + trad);
+                        float attr = sc_polar_attr(Lr);
+                        dV += (tpPV - pPV) * 0.05f * attr * 1.0f;
+                        float pap = sc_powf(fminf(1.0f / fmaxf(Lr, 1e-6f), 10.0f) / 10.0f, 0.2f);
+                        phobSum += pap;
+                        phobPos += tpPV * pap;
+                    }
+                    if (fl & SC_PP_PARTNER) {
+                        // this neighbour's bond matches are the next ones in order
+                        for (; mi < nm; mi++) {
+                            const uint32_t me = mi == 0 ? r.y : myMatch[mi];
+                            if ((int)(me & SC_PP_INDEX) != j) break;
+                            const int it = mi == 0 ? (int)r.z : myBonds[3 * (int)(me >> 29)];
+                            if (bond_turns(it)) {
+                                dV += ut == 0 ? T0 : T[ut - 1];
+                                ut++;
+                            }
+                        }
+                    }
+                    if (fl & SC_PP_COLLIDE)
+                        dV += collide_term(kept ? g[q] : collide_geo(IM, S.ppos, S.prad, g[q]), tv[q], ppv, S.prad);
+                }
+            }
+            const sc_f3 nv = S.pvel + dV / fmaxf((float)(r.w >> 16), 1.0f);
+            st3(A.velOut, i, nv, v4.w);
+            if (A.age == 0) A.rotOut[i] = r4;
+            if (phobSum > 0.0f) {
+                newPos = S.ppos + nv;
+                towards = normalize(phobPos / phobSum - newPos);
+            }
         }
-    } else {
-        for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
-            relax_class_item<MODE, BATCH>(P, A, idx[t]);
     }
+    __syncthreads();
+    if (!turner && i >= 0 && polar) {
+        const float4 q = s_av[slot];
+        sc_f4 pav = sc_make_f4(q.x, q.y, q.z, q.w);
+        if (phobSum > 0.0f) pav = sc_slerp(pav, sc_quat_from_to(-up, towards), 0.2f);
+        st4(A.avOut, i, pav);
+    }
+    __syncthreads();  // s_av is reused by the block's next items
 }
 
-// Active items whose list overflowed: their neighbourhood is scanned.  A
-// separate kernel keeps the scan code out of k_relax's instruction stream.
-template <bool BATCH>
-__global__ void __launch_bounds__(SC_THREADS) k_relax_overflow(ScParams P, RelaxArgs A, const int *__restrict__ ovf,
-                                                               const int *__restrict__ ovfCount) {
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < *ovfCount; t += gridDim.x * blockDim.x) {
-        const int i = ovf[t];
-        int4 in = A.info[i];
-        rep_apply<BATCH>(P, in.w);
-        if (in.z & SC_ACTIVE) relax_item<true, 0>(P, A, i, in, A.velIn[i], A.rotIn[i], A.avIn[i]);
+// ---- dynamics.cuh:405-822 relax ------------------------------------------------
+// The classes write disjoint items and read only the input buffers, so they
+// run side by side.  CLS = SC_RELAX_ALL: one grid over all of them, its blocks
+// taking the bonded class first (the longest chains), then the polar and plain
+// classes and the items left to the scan, so the short classes run while the
+// long one does.  CLS = 0, 1, 2: one class (0 with the scan's items), at the
+// occupancy its registers allow.
+//
+// The line between them is whether the particles fill the device
+// (forkClasses in sc_sim.cu): 4,096 + 8,192 items take 1.95 ms a step with a
+// launch per class in turn and 1.2 ms with one launch; 2,097,152 + 8,388,608
+// take 27.5 ms with a kernel per class and 30.7 ms with one launch, whose two
+// blocks per SM starve the plain and polar items.
+#define SC_RELAX_ALL 3
+template <int CLS, bool BATCH>
+__global__ void __launch_bounds__(SC_THREADS, CLS == 1 ? 4 : CLS == 2 ? 5 : 2) k_relax(ScParams P, RelaxArgs A) {
+    __shared__ float4 s_av[CLS == 0 || CLS == SC_RELAX_ALL ? SC_BOND_ITEMS : 1];
+    constexpr bool B0 = CLS == 0 || CLS == SC_RELAX_ALL, B1 = CLS == 1 || CLS == SC_RELAX_ALL,
+                   B2 = CLS == 2 || CLS == SC_RELAX_ALL;
+    const int n0 = B0 ? A.classCount[0] : 0, n1 = B1 ? A.classCount[1] : 0, n2 = B2 ? A.classCount[2] : 0,
+              nv = B0 ? *A.ovfCount : 0;
+    const int b0 = (n0 + SC_BOND_ITEMS - 1) / SC_BOND_ITEMS, b1 = b0 + (n1 + SC_THREADS - 1) / SC_THREADS,
+              b2 = b1 + (n2 + SC_THREADS - 1) / SC_THREADS, b3 = b2 + (nv + SC_THREADS - 1) / SC_THREADS;
+    for (int b = blockIdx.x; b < b3; b += gridDim.x) {
+        if (B0 && b < b0) {
+            relax_bonded_block<BATCH>(P, A, b * SC_BOND_ITEMS, n0, s_av);
+        } else if (B1 && b < b1) {
+            const int t = (b - b0) * SC_THREADS + threadIdx.x;
+            if (t < n1) relax_polar<BATCH>(P, A, A.classIdx[(size_t)A.L.cap + t]);
+        } else if (B2 && b < b2) {
+            const int t = (b - b1) * SC_THREADS + threadIdx.x;
+            if (t < n2) relax_plain<BATCH>(P, A, A.classIdx[2 * (size_t)A.L.cap + t]);
+        } else if (B0) {
+            const int t = (b - b2) * SC_THREADS + threadIdx.x;
+            if (t < nv) {
+                const int i = A.ovf[t];
+                const int4 in = A.info[i];
+                ScParams Q = P;
+                rep_apply<BATCH>(Q, in.w);
+                if (in.z & SC_ACTIVE) relax_scan_item(Q, A, i, in, A.velIn[i], A.rotIn[i], A.avIn[i]);
+            }
+        }
     }
 }
 
@@ -3096,6 +3205,15 @@ void sc_phase_move_brownian(ScLaunchCtx &c, bool metabolic) {
     (*c.launches)++;
 }
 
+static PairList<SC_LIST_PP> pp_list(const ScLaunchCtx &c) {
+    PairList<SC_LIST_PP> L;
+    L.list = c.B->listPP;
+    L.cnt = c.B->cntPP;
+    L.cap = c.P.N;
+    L.perm = nullptr;
+    return L;
+}
+
 static void ensure_pp(ScLaunchCtx &c) {
     ScBuffers &B = *c.B;
     if (B.validPP) return;
@@ -3105,18 +3223,12 @@ static void ensure_pp(ScLaunchCtx &c) {
     SC_BATCHED(k_build_pp)<<<nblocks(c.P.N), SC_THREADS, 0, c.st>>>(c.P, B.cellStartP, &B.ctr->nActive, F.pos, F.info, F.nb,
                                                          F.bonds, B.listPP, B.cntPP, c.P.N, B.classPP,
                                                          B.ctr->ppClassCount, B.ovfPP, &B.ctr->ovfPP, B.matchPP,
-                                                         B.matchN);
-    (*c.launches)++;
+                                                         B.matchN, B.geoPP);
+    k_bond_plan<<<std::min(nblocks(c.P.N), c.gridCap), SC_THREADS, 0, c.st>>>(
+        c.P, pp_list(c), B.classPP, B.ctr->ppClassCount, F.bonds, B.matchPP, B.matchN, B.bondRec);
+    (*c.launches) += 2;
     B.validPP = true;
-}
-
-static PairList<SC_LIST_PP> pp_list(const ScLaunchCtx &c) {
-    PairList<SC_LIST_PP> L;
-    L.list = c.B->listPP;
-    L.cnt = c.B->cntPP;
-    L.cap = c.P.N;
-    L.perm = nullptr;
-    return L;
+    B.relaxAge = 0;
 }
 
 void sc_phase_coordinate_noise(ScLaunchCtx &c, float frac) {
@@ -3158,30 +3270,30 @@ void sc_phase_relax(ScLaunchCtx &c) {
     PFields F = B.P(), X = B.Pnext();
     RelaxArgs A{B.cellStartP, &B.ctr->nActive, F.pos, F.info, F.nb, F.bonds, pp_list(c),
                 F.vel, F.rot, F.angvel, X.vel, X.rot, X.angvel, F.dbg, B.classPP, B.ctr->ppClassCount,
-                B.matchPP, B.matchN};
-    // The three classes write disjoint items and read only the input
-    // buffers: with side streams they run concurrently (bonded on st, the
-    // others on the side streams), so the classes fill each other's tails;
-    // each grid covers its class at most once.
-    const int g = std::min(nblocks(c.P.N), c.gridCap);
-    const bool fork = c.side[0] != nullptr;
-    if (fork) {
+                B.matchPP, B.matchN, B.geoPP, B.bondRec, B.ovfPP, &B.ctr->ovfPP, &B.ctr->ppClassCount[3], B.relaxAge};
+    const int nb = nblocks(c.P.N);
+    const bool batch = c.P.nRep > 1;
+    if (c.side[0]) {
+        // particles that fill the device: a kernel per class, each at its own
+        // occupancy, on three streams
         cudaEventRecord(c.fork, c.st);
         cudaStreamWaitEvent(c.side[0], c.fork, 0);
         cudaStreamWaitEvent(c.side[1], c.fork, 0);
-    }
-    const bool batch = c.P.nRep > 1;
-    (batch ? k_relax<0, true> : k_relax<0, false>)<<<g, SC_THREADS, 0, c.st>>>(c.P, A);
-    (batch ? k_relax<2, true> : k_relax<2, false>)<<<g, SC_THREADS, 0, fork ? c.side[0] : c.st>>>(c.P, A);
-    (batch ? k_relax<1, true> : k_relax<1, false>)<<<g, SC_THREADS, 0, fork ? c.side[1] : c.st>>>(c.P, A);
-    if (fork) {
+        const int g = std::min(nb, c.gridCap);
+        (batch ? k_relax<0, true> : k_relax<0, false>)<<<std::min(3 * nb + 1, c.gridCap), SC_THREADS, 0, c.st>>>(c.P, A);
+        (batch ? k_relax<2, true> : k_relax<2, false>)<<<g, SC_THREADS, 0, c.side[0]>>>(c.P, A);
+        (batch ? k_relax<1, true> : k_relax<1, false>)<<<g, SC_THREADS, 0, c.side[1]>>>(c.P, A);
         cudaEventRecord(c.join[0], c.side[0]);
         cudaEventRecord(c.join[1], c.side[1]);
         cudaStreamWaitEvent(c.st, c.join[0], 0);
         cudaStreamWaitEvent(c.st, c.join[1], 0);
+        (*c.launches) += 2;
+    } else {
+        // fewer: one launch
+        (batch ? k_relax<SC_RELAX_ALL, true>
+               : k_relax<SC_RELAX_ALL, false>)<<<std::min(3 * nb + 4, c.gridCap), SC_THREADS, 0, c.st>>>(c.P, A);
     }
-    SC_BATCHED(k_relax_overflow)<<<std::min(nblocks(c.P.N), c.gridCap / 4), SC_THREADS, 0, c.st>>>(c.P, A, B.ovfPP, &B.ctr->ovfPP);
-    (*c.launches) += 3;
+    B.relaxAge = std::min(B.relaxAge + 1, 2);
     B.cp[FP_VEL] ^= 1;
     B.cp[FP_ROT] ^= 1;
     B.cp[FP_ANGVEL] ^= 1;
