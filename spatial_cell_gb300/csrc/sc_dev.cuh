@@ -92,6 +92,7 @@ struct ScCounters {
     unsigned long long poolM;   // entries the metabolic list blocks asked of their pool (k_build_m)
     unsigned long long poolLM;  // the same for the lipid-metabolic lists (k_build_lm)
     int workCount;              // items in the particle work list (k_complexify_select)
+    int farMove;                // a metabolic item moved more than a cell along an axis since its sort
     int ovfD;                     // items whose diffusion list overflowed (k_build_d)
     unsigned long long poolOvfM;  // entries the overflowed metabolic items asked of their pool (k_build_m_ovf)
     unsigned long long poolOvfD;  // the same for the diffusion lists (k_build_d_ovf)
@@ -153,6 +154,11 @@ struct ScParams {
     // lipidP[slot] says "active lipid" (types and particle flags do not
     // change between sorts).
     int mAllActive;
+    // 1: the metabolic items have moved once since their sort (apply
+    // velocities); farMove then says whether one moved more than a cell along
+    // an axis
+    int movedOnce;
+    const int *farMove;
     int lipidValid;
     const uint8_t *lipidP;
 };
@@ -375,6 +381,164 @@ __device__ __forceinline__ void cells27(const ScParams &P, sc_f3 pos, const Reac
 template <class F>
 __device__ __forceinline__ void cells27(const ScParams &P, sc_f3 pos, F &&f) {
     cells27(P, pos, Reach(), f);
+}
+
+// Whether candidates of sets `need` may lie on either side of a periodic face
+// whatever cell they are listed in (scan_words).
+__device__ __forceinline__ bool scan_mixed(const ScParams &P, int need) {
+    return P.periodic && ((P.binned & need) != need || !(P.simSize >= 5.0f * P.cell));
+}
+// The same neighbourhood for the list builds, in two passes a thread takes
+// word by word.  A builder's thread spends its time on candidates that leave
+// at the cube test (three of four): visited one by one with the survivors
+// handled in place, a third of a warp's lanes were busy.  Here the first pass
+// tests up to 32 consecutive candidates without a branch and keeps the
+// survivors as a bit mask; the second walks the masks' bits, so the costly
+// part runs with a lane per survivor.  Candidates are visited in the
+// reference's order: cells of a column's z run are consecutive in `cand`, a
+// word's bits ascend, and when an item's words fill its slots they are walked
+// before the scan goes on.
+//
+// cand holds positions in cell order, start(key) the first candidate of cell
+// key (start(key + 1) the end of its run); up to seven records past a run's
+// end are read and masked off, so cand has SC_CAND_PAD records more than
+// candidates.  The first pass keeps a superset of what the cube |delta| <= lim
+// holds.  In the box's interior that is the cube itself.  A run across a
+// periodic face is tested against the item shifted by the box, with a margin:
+// a coordinate difference and its image differ from the box length by the
+// rounding of coordinates no larger than |pp| + 2 L + lim.  With `mixed`
+// (candidates that may lie on either side of a face: sets that have moved
+// since their sort, boxes under five cells) every candidate within that
+// margin directly or across a face is kept.  f(k, cand[k]) makes the exact
+// tests; without an image (Imager::wrap) the cube holds already.
+//
+// What bounds it is the latency of the candidates' loads at 32 warps per SM,
+// so SC_SCAN_GROUP of them are in flight at a time and a survivor's record is
+// loaded while the one before is handled.  524,288 + 2,097,152 items (a
+// quarter of the large workload), per step: k_build_m 1136 -> 604 us (groups
+// of four: 685; with the emission's four pairs in flight, which took 440 us
+// one by one), k_build_d 598 -> 508 us, k_build_lm 211 -> 150 us; the columns
+// advanced per lane instead of in step for the warp: 741 / 546 us.
+#define SC_SCAN_GROUP 8
+#define SC_CAND_PAD SC_SCAN_GROUP
+#define SC_SCAN_WORDS 10
+struct ScanWords {
+    uint32_t base[SC_SCAN_WORDS][SC_THREADS], mask[SC_SCAN_WORDS][SC_THREADS];
+};
+template <class Start, class F>
+__device__ __forceinline__ void scan_words(const ScParams &P, ScanWords &W, const float4 *__restrict__ cand,
+                                           Start &&start, sc_f3 pp, const Reach &R, float lim, bool mixed, F &&f) {
+    const int n = cell_limit(P), tid = threadIdx.x;
+    const int cx = (int)sc_grid_idx(pp.x, P.cell, n), cy = (int)sc_grid_idx(pp.y, P.cell, n),
+              cz = (int)sc_grid_idx(pp.z, P.cell, n);
+    const float L = P.simSize;
+    const float wide = lim + 1e-3f + 4e-6f * (L + fmaxf(fabsf(pp.x), fmaxf(fabsf(pp.y), fabsf(pp.z))));
+    // a periodic column's z run that crosses the face is taken in two parts:
+    // first the cells up to `cut`, then the rest
+    const int za = cz + R.zl, zb = cz + R.zh;
+    const bool split = P.periodic && (za < 0 || zb > n - 1);
+    const int cut = za < 0 ? -1 : n - 1;
+    int from = 0;             // where the scan goes on: the run, and its next candidate
+    uint32_t fromB = 0;
+    bool more;
+    do {
+        more = false;
+        int nw = 0;
+        // the columns in step for the whole warp (a lane without one idles), each in its two parts
+        for (int r = 0; r < 18; r++) {
+            const int ox = r / 6 - 1, oy = (r >> 1) % 3 - 1;
+            if (more || r < from || ((r & 1) && !split) || ox < R.xl || ox > R.xh || oy < R.yl || oy > R.yh) continue;
+            int gx = cx + ox, gy = cy + oy, z0 = za, z1 = zb;
+            sc_f3 q = pp;       // the item as this run's candidates see it
+            float far = lim;    // the first pass's cube
+            if (P.periodic) {
+                if (split) {
+                    if (r & 1) z0 = cut + 1;
+                    else z1 = cut;
+                }
+                if (gx < 0 || gx >= n || gy < 0 || gy >= n || z0 < 0 || z0 >= n) {
+                    q.x = gx < 0 ? pp.x + L : (gx >= n ? pp.x - L : pp.x);
+                    q.y = gy < 0 ? pp.y + L : (gy >= n ? pp.y - L : pp.y);
+                    q.z = z0 < 0 ? pp.z + L : (z0 >= n ? pp.z - L : pp.z);
+                    far = wide;
+                    const int len = z1 - z0;
+                    gx = (int)wrap_cell(gx, n);
+                    gy = (int)wrap_cell(gy, n);
+                    z0 = (int)wrap_cell(z0, n);
+                    z1 = z0 + len;
+                }
+            } else {
+                if (gx < 0 || gx >= n || gy < 0 || gy >= n) continue;
+                z0 = max(z0, 0);
+                z1 = min(z1, n - 1);
+            }
+            const uint32_t key = cell_key(P, (uint32_t)gx, (uint32_t)gy, 0);
+            uint32_t b = start(key + (uint32_t)z0);
+            const uint32_t e = start(key + (uint32_t)z1 + 1u);
+            if (r == from && fromB) b = fromB;
+            for (; b < e; b += 32u) {
+                if (nw == SC_SCAN_WORDS) {
+                    more = true;
+                    from = r;
+                    fromB = b;
+                    break;
+                }
+                const uint32_t m = min(32u, e - b);
+                const float4 *__restrict__ t = cand + b;
+                uint32_t mask = 0;
+                if (!mixed) {
+                    for (uint32_t u = 0; u < m; u += SC_SCAN_GROUP) {
+                        float4 c[SC_SCAN_GROUP];
+#pragma unroll
+                        for (int v = 0; v < SC_SCAN_GROUP; v++) c[v] = t[u + v];
+                        uint32_t bits = 0;
+#pragma unroll
+                        for (int v = 0; v < SC_SCAN_GROUP; v++)
+                            if (!(fmaxf(fabsf(c[v].x - q.x), fmaxf(fabsf(c[v].y - q.y), fabsf(c[v].z - q.z))) > far))
+                                bits |= 1u << v;
+                        mask |= bits << u;
+                    }
+                } else {
+                    for (uint32_t u = 0; u < m; u++) {
+                        const float4 c = t[u];
+                        const float dx = fabsf(c.x - pp.x), dy = fabsf(c.y - pp.y), dz = fabsf(c.z - pp.z);
+                        const float d = fmaxf(fminf(dx, fabsf(dx - L)),
+                                              fmaxf(fminf(dy, fabsf(dy - L)), fminf(dz, fabsf(dz - L))));
+                        if (!(d > wide)) mask |= 1u << u;
+                    }
+                }
+                if (m < 32u) mask &= (1u << m) - 1u;
+                if (mask) {
+                    W.base[nw][tid] = b - 1u;
+                    W.mask[nw][tid] = mask;
+                    nw++;
+                }
+            }
+        }
+        // the survivors so far, the next one's record on its way
+        uint32_t k = 0, base = 0, mask = 0;
+        int w = 0;
+        auto step = [&]() {
+            if (!mask) {
+                if (w == nw) return false;
+                base = W.base[w][tid];
+                mask = W.mask[w][tid];
+                w++;
+            }
+            k = base + (uint32_t)__ffs((int)mask);
+            mask &= mask - 1u;
+            return true;
+        };
+        bool any = step();
+        float4 c = cand[k];
+        while (any) {
+            const uint32_t kc = k;
+            const float4 cc = c;
+            any = step();
+            c = cand[k];
+            f((int)kc, cc);
+        }
+    } while (more);
 }
 
 __device__ __forceinline__ void set_error(ScCounters *c, int code) { atomicCAS(&c->error, 0, code); }

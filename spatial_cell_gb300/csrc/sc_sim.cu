@@ -414,6 +414,7 @@ void sort_metabolic(sc_sim *s) {
     MFields F = B.M();
     int cur = sc_launch_sort(s->st, F.pos, F.info, Nm, s->P, B.keysM, B.valsM, B.hist, B.lookback, B.ctr, &s->launches);
     B.sortCurM = cur;
+    cudaMemsetAsync(&B.ctr->farMove, 0, sizeof(int), s->st);
     sc_launch_cell_start(s->st, B.keysM[cur], Nm, s->P.cells, B.cellStartM, &s->launches);
     sc_launch_gather_metabolic(s->st, B.valsM[cur], Nm, s->P.SP / 4, B, &s->launches);
 }
@@ -441,7 +442,10 @@ void invalidate_after(ScBuffers &B, int phase) {
 void binned_after(ScParams &P, int phase) {
     if (phase == SC_PHASE_SORT_PARTICLES) P.binned |= SC_BINNED_P;
     if (phase == SC_PHASE_SORT_METABOLIC) P.binned |= SC_BINNED_M;
-    if (phase == SC_PHASE_APPLY_VELOCITIES) P.binned = 0;
+    if (phase == SC_PHASE_APPLY_VELOCITIES) {
+        P.movedOnce = (P.binned & SC_BINNED_M) != 0;
+        P.binned = 0;
+    }
     if (phase == SC_PHASE_SORT_METABOLIC) P.mAllActive = 1;  // inactive items sort past the cells
     if (phase == SC_PHASE_REMOVE_INTERFERING) P.mAllActive = 0;
     if (phase == SC_PHASE_SORT_PARTICLES) P.lipidValid = 1;  // marked by sort_particles
@@ -453,7 +457,7 @@ std::vector<int> host_state(const sc_sim *s) {
     std::vector<int> v(B.cp, B.cp + FP_COUNT);
     v.insert(v.end(), B.cm, B.cm + FM_COUNT);
     v.insert(v.end(), {B.sortCurP, B.sortCurM, (int)B.validPP, (int)B.validM, (int)B.validLM, (int)B.validD,
-                       s->P.binned, s->P.mAllActive, s->P.lipidValid, B.mParity, B.relaxAge});
+                       s->P.binned, s->P.mAllActive, s->P.lipidValid, B.mParity, B.relaxAge, s->P.movedOnce});
     return v;
 }
 void set_host_state(sc_sim *s, const std::vector<int> &v) {
@@ -472,6 +476,7 @@ void set_host_state(sc_sim *s, const std::vector<int> &v) {
     s->P.lipidValid = v[k++];
     B.setMParity(v[k++]);
     B.relaxAge = v[k++];
+    s->P.movedOnce = v[k++];
 }
 
 int run_phase(sc_sim *s, int phase, int arg) {
@@ -881,7 +886,7 @@ static int create_sim(const sc_config *cfg_in, const sc_replica *replicas, int32
     for (int b = 0; b < 2; b++) {
         PFields &f = B.p[b];
         MFields &m = B.m[b];
-        if ((rc = dalloc(s, &f.pos, N)) || (rc = dalloc(s, &f.vel, N)) || (rc = dalloc(s, &f.rot, N)) ||
+        if ((rc = dalloc(s, &f.pos, N + SC_CAND_PAD)) || (rc = dalloc(s, &f.vel, N)) || (rc = dalloc(s, &f.rot, N)) ||
             (rc = dalloc(s, &f.angvel, N)) || (rc = dalloc(s, &f.posnoise, N)) || (rc = dalloc(s, &f.angnoise, N)) ||
             (rc = dalloc(s, &f.dbg, N)) || (rc = dalloc(s, &f.info, N)) || (rc = dalloc(s, &f.state, N)) ||
             (rc = dalloc(s, &f.lscs, N)) || (rc = dalloc(s, &f.spoly, N)) || (rc = dalloc(s, &f.nb, N)) ||
@@ -892,7 +897,7 @@ static int create_sim(const sc_config *cfg_in, const sc_replica *replicas, int32
     }
     // the metabolic fields with one buffer each, and their spares
     for (int k = 0; k <= ScBuffers::kM4; k++)
-        if ((rc = dalloc(s, &B.mChain4[k], Nm))) return bail(rc);
+        if ((rc = dalloc(s, &B.mChain4[k], Nm + SC_CAND_PAD))) return bail(rc);
     for (int k = 0; k <= ScBuffers::kM1; k++)
         if ((rc = dalloc(s, &B.mChain1[k], Nm))) return bail(rc);
     B.setMParity(0);
@@ -922,7 +927,7 @@ static int create_sim(const sc_config *cfg_in, const sc_replica *replicas, int32
         (rc = dalloc(s, &B.ovfD, Nm)) || (rc = dalloc(s, &B.ovfOffD, Nm)) || (rc = dalloc(s, &B.ovfPoolD, 1)) ||
         (rc = dalloc(s, &B.claimP, P.pairClaim ? N : 1)) ||
         (rc = dalloc(s, &B.warpOffM, (size_t)Nm / 32 + 1)) || (rc = dalloc(s, &B.warpOffLM, (size_t)N / 32 + 1)) ||
-        (rc = dalloc(s, &B.lipidP, N)))
+        (rc = dalloc(s, &B.lipidP, N)) || (rc = dalloc(s, &B.comb, N + Nm + SC_CAND_PAD)))
         return bail(rc);
     // The LM list is built in the diffusion list's buffer when it fits.
     if (sc_list_words(SC_LIST_LM, (int)N) <= sc_list_words(SC_LIST_DBUF, (int)Nm)) {
@@ -937,6 +942,7 @@ static int create_sim(const sc_config *cfg_in, const sc_replica *replicas, int32
     if (cfg->pool_per_item >= 0)
         B.poolCapM = std::min(B.poolCapM, (size_t)cfg->pool_per_item * (size_t)std::max<int64_t>(Nm, 1));
     P.lipidP = B.lipidP;
+    P.farMove = &B.ctr->farMove;
     cudaMemsetAsync(B.ctr, 0, sizeof(ScCounters), s->st);
     cudaMemsetAsync(B.polyClaim, 0, std::max<size_t>(N, 1) * sizeof(int), s->st);
     cudaMemsetAsync(B.cellStartP, 0, ((size_t)P.cells + 1) * 4, s->st);
@@ -1039,6 +1045,7 @@ int sc_load_state(sc_sim *s, const sc_particle *particles, int32_t n, const sc_m
     B.invalidateLists();
     s->loaded = false;
     s->P.binned = 0;
+    s->P.movedOnce = 0;
     s->P.mAllActive = 0;
     s->P.lipidValid = 0;
     for (int k = 0; k < FP_COUNT; k++) B.cp[k] = 0;
@@ -1557,6 +1564,7 @@ static int generate_into(sc_sim *s, int n, int nm, uint64_t seed, const std::fun
     ScBuffers &B = s->B;
     B.invalidateLists();
     s->P.binned = 0;
+    s->P.movedOnce = 0;
     s->P.mAllActive = 0;
     s->P.lipidValid = 0;
     for (int k = 0; k < FP_COUNT; k++) B.cp[k] = 0;
@@ -1633,6 +1641,7 @@ int sc_generate_batch(sc_sim *s, const int32_t *n, const int32_t *nm, const int3
     ScBuffers &B = s->B;
     B.invalidateLists();
     s->P.binned = 0;
+    s->P.movedOnce = 0;
     s->P.mAllActive = 0;
     s->P.lipidValid = 0;
     for (int k = 0; k < FP_COUNT; k++) B.cp[k] = 0;
@@ -1718,6 +1727,7 @@ int sc_generate_scene_batch(sc_sim *s, const sc_scene_group *groups, int32_t n_g
     ScBuffers &B = s->B;
     B.invalidateLists();
     s->P.binned = 0;
+    s->P.movedOnce = 0;
     s->P.mAllActive = 0;
     s->P.lipidValid = 0;
     for (int k = 0; k < FP_COUNT; k++) B.cp[k] = 0;

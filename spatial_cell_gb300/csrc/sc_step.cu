@@ -71,7 +71,7 @@ template <bool BATCH>
 __global__ void __launch_bounds__(SC_THREADS) k_apply_velocities(const int *__restrict__ nActivePtr,
                                                                  const int4 *__restrict__ info, float4 *pos,
                                                                  float4 *vel, float4 *rot, float4 *angvel,
-                                                                 ScParams P, float f) {
+                                                                 ScParams P, float f, int *farMove) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= *nActivePtr) return;
     const int4 in = info[i];
@@ -80,6 +80,7 @@ __global__ void __launch_bounds__(SC_THREADS) k_apply_velocities(const int *__re
     float4 p4 = pos[i];
     sc_f3 p = sc_make_f3(p4.x, p4.y, p4.z);
     sc_f3 v = ld3(vel, i);
+    if (farMove && !(fmaxf(fabsf(v.x), fmaxf(fabsf(v.y), fabsf(v.z))) * f < 0.999f * P.cell)) *farMove = 1;
     p = P.periodic ? sc_wrap3(p + v * f, P.simSize)
                    : (P.walls ? sc_reflect3(p + v * f, P.simSize) : clamp(p + v * f, 0.0f, P.simSize));
     v *= P.velDecay;
@@ -172,7 +173,13 @@ __device__ __forceinline__ void emit_count_ordered(bool valid, int c, int limit,
         cnt[g] = max(cs, 0);
     }
     const int n = min(max(cs, 0), min(K, limit));
-    for (int k = 0; k < n; k++) list[sc_list4_at(K, g, k)] = scratch[sc_list_at(K, b0 + src, k)];
+    for (int k0 = 0; k0 < n; k0 += 8) {   // two chunks of four entries in flight together
+        uint32_t e[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) e[q] = k0 + q < n ? scratch[sc_list_at(K, b0 + src, k0 + q)] : 0u;
+        *reinterpret_cast<uint4 *>(list + sc_list4_at(K, g, k0)) = make_uint4(e[0], e[1], e[2], e[3]);
+        if (k0 + 4 < n) *reinterpret_cast<uint4 *>(list + sc_list4_at(K, g, k0 + 4)) = make_uint4(e[4], e[5], e[6], e[7]);
+    }
     if (ovf && cs > min(K, limit)) ovf[atomicAdd(ovfCount, 1)] = g;
 }
 
@@ -250,6 +257,7 @@ __global__ void __launch_bounds__(SC_THREADS) k_build_pp(ScParams P, const uint3
                                                          int *__restrict__ ovf, int *__restrict__ ovfCount,
                                                          uint32_t *__restrict__ match, int *__restrict__ matchN,
                                                          float4 *__restrict__ geo) {
+    __shared__ ScanWords W;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= *nActivePtr) return;
     int4 in = info[i];
@@ -270,17 +278,16 @@ __global__ void __launch_bounds__(SC_THREADS) k_build_pp(ScParams P, const uint3
         uint32_t any = 0;
         uint32_t *__restrict__ myMatch = match + (size_t)i * SC_MAX_ACTIVE_INTERACTIONS;
         const int K = min(SC_LIST_PP, P.listLimit);
-        auto add = [&](int j, uint32_t f, sc_f3 delta, float trad) {
+        auto add = [&](int j, uint32_t f, sc_f3 delta, float4 t4) {
             if (c < K) list[sc_list_at(SC_LIST_PP, i, c)] = (uint32_t)j | f;
             // a colliding pair's position-only part of dynamics.cuh:775-786,
             // tpos - normalize(tpos - pos) * collisionDistance: the first
             // float3 its velocity term evaluates, the same in every
             // relaxation sub-iteration
             if ((f & SC_PP_COLLIDE) && c < SC_GEO_PP) {
-                const float4 t4 = pos[j];
                 const sc_f3 tpos = IM(sc_make_f3(t4.x, t4.y, t4.z));
-                const sc_f3 a = tpos - normalize(delta) * (p4.w + trad);
-                geo[sc_list_at(SC_GEO_PP, i, c)] = make_float4(a.x, a.y, a.z, trad);
+                const sc_f3 a = tpos - normalize(delta) * (p4.w + t4.w);
+                geo[sc_list_at(SC_GEO_PP, i, c)] = make_float4(a.x, a.y, a.z, t4.w);
             }
             c++;
             any |= f;
@@ -292,35 +299,14 @@ __global__ void __launch_bounds__(SC_THREADS) k_build_pp(ScParams P, const uint3
                         myMatch[nm++] = (uint32_t)j | ((uint32_t)k << 29);
             }
         };
-        // 1. the candidates inside the interaction cube, in visiting order, held in the list's
-        // slots (a cheap loop: most candidates leave at the cube test)
-        int pc = 0;
-        scan27(P, cellStart, ppos, reach(P, ppos, P.maxInt, SC_BINNED_P), [&](int j) {
-            if (j == i) return;
-            const float4 t4 = pos[j];
-            if (outside_cube(IM(sc_make_f3(t4.x, t4.y, t4.z)) - ppos, P.maxInt)) return;
-            if (pc < K) list[sc_list_at(SC_LIST_PP, i, pc)] = (uint32_t)j;
-            pc++;
-        });
-        if (pc <= K) {
-            // 2. their remaining tests in order, the list compacted in place (entry c <= k)
-            for (int k = 0; k < pc; k++) {
-                const int j = (int)list[sc_list_at(SC_LIST_PP, i, k)];
-                const float4 t4 = pos[j];
-                const sc_f3 delta = IM(sc_make_f3(t4.x, t4.y, t4.z)) - ppos;
-                const uint32_t f = pp_flags_in_cube(delta, t4.w, j, p4.w, phydro, B, info);
-                if (f) add(j, f, delta, t4.w);
-            }
-        } else {
-            // more in-cube candidates than the list holds: every test in one scan
-            scan27(P, cellStart, ppos, reach(P, ppos, P.maxInt, SC_BINNED_P), [&](int j) {
-                const uint32_t f = pp_flags(P, IM, i, j, ppos, p4.w, phydro, B, pos, info);
-                if (f) {
-                    const float4 t4 = pos[j];
-                    add(j, f, IM(sc_make_f3(t4.x, t4.y, t4.z)) - ppos, t4.w);
-                }
-            });
-        }
+        scan_words(P, W, pos, [&](uint32_t key) { return cellStart[key]; }, ppos, reach(P, ppos, P.maxInt, SC_BINNED_P),
+                   P.maxInt, scan_mixed(P, SC_BINNED_P), [&](int j, float4 t4) {
+                       if (j == i) return;
+                       const sc_f3 delta = IM(sc_make_f3(t4.x, t4.y, t4.z)) - ppos;
+                       if (IM.wrap && outside_cube(delta, P.maxInt)) return;
+                       const uint32_t f = pp_flags_in_cube(delta, t4.w, j, p4.w, phydro, B, info);
+                       if (f) add(j, f, delta, t4);
+                   });
         cnt[i] = c;
         // A test bond rotates the particle itself, which its later terms
         // read: its relaxation takes the in-order scan with the overflowed
@@ -1214,21 +1200,85 @@ __device__ __forceinline__ void scan_m_item(const ScParams &P, const uint32_t *_
     });
 }
 
-__device__ __forceinline__ void build_m_item(const ScParams &P, const uint32_t *__restrict__ cellStartM,
-                                             const uint32_t *__restrict__ cellStartP, int i,
-                                             const float4 *__restrict__ mpos, const int4 *__restrict__ minfo,
-                                             const float4 *__restrict__ ppos_, const int4 *__restrict__ pinfo,
+// The M list's candidates in one array: cell by cell, the metabolic items'
+// positions, then the particles' (comb_start gives a cell's first), so that the
+// reference's visiting order -- per cell, metabolic items then lipids -- is one
+// run per column.  w holds the slot (SC_M_FROM_P for particles); what is no
+// candidate (particles other than active lipids, inactive items) lies at
+// infinity, which no cube reaches.  A radius other than its type's sets
+// SC_M_ODD: the tests of all others need no radius.
+#define SC_M_ODD 0x40000000u
+#define SC_M_SLOT 0x3FFFFFFFu
+__device__ __forceinline__ float type_radius(const ScParams &P, int type) {
+    return type < P.nTypes ? P.types[type].radius : 0.0f;
+}
+struct CombStart {
+    const uint32_t *__restrict__ m, *__restrict__ p;
+    __device__ __forceinline__ uint32_t operator()(uint32_t key) const { return m[key] + p[key]; }
+};
+__global__ void __launch_bounds__(SC_THREADS) k_combine(ScParams P, const uint32_t *__restrict__ keysM,
+                                                        const uint32_t *__restrict__ keysP, CombStart cs,
+                                                        const float4 *__restrict__ mpos, const int4 *__restrict__ minfo,
+                                                        const float4 *__restrict__ ppos_, const int4 *__restrict__ pinfo,
+                                                        float4 *__restrict__ comb) {
+    const long long total = (long long)P.N + P.Nm;
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
+        const bool m = t < P.Nm;
+        const int j = (int)(m ? t : t - P.Nm);
+        const uint32_t key = m ? keysM[j] : keysP[j];
+        if (key >= P.cells) continue;   // in no cell
+        const size_t at = m ? (size_t)j + cs.p[key] : (size_t)j + cs.m[key + 1];
+        if (at >= (size_t)total) continue;
+        float4 q = m ? mpos[j] : ppos_[j];
+        if (!(m ? active_m(P, minfo, j) : active_lipid(P, pinfo, j))) q.x = q.y = q.z = INFINITY;
+        const bool odd = !(q.w == type_radius(P, m ? SC_PARTICLE_TYPE_METABOLIC : SC_PARTICLE_TYPE_LIPID));
+        q.w = __uint_as_float((uint32_t)j | (m ? 0u : SC_M_FROM_P) | (odd ? SC_M_ODD : 0u));
+        comb[at] = q;
+    }
+}
+
+__device__ __forceinline__ void build_m_item(const ScParams &P, ScanWords &W, CombStart cs,
+                                             const float4 *__restrict__ comb, int i,
+                                             const float4 *__restrict__ mpos, const float4 *__restrict__ ppos_,
                                              uint32_t *list, int &c) {
-    float4 p4 = mpos[i];
+    const float4 p4 = mpos[i];
     const sc_f3 pp = sc_make_f3(p4.x, p4.y, p4.z);
     const Imager IM(P, pp, SC_BINNED_M | SC_BINNED_P);
-    CollisionDistCache cm, cp;
+    // the collision distances (metabolites.cuh:193-203, 230-240) to the two kinds of candidates
+    const sc_sqrt_le leM = sc_sqrt_le_make(sc_coll_dist(p4.w, type_radius(P, SC_PARTICLE_TYPE_METABOLIC))),
+                     leP = sc_sqrt_le_make(sc_coll_dist(p4.w, type_radius(P, SC_PARTICLE_TYPE_LIPID)));
     const int limit = min(SC_LIST_M, P.listLimit);
-    scan_m_item(P, cellStartM, cellStartP, i, mpos, minfo, ppos_, pinfo, IM, pp, p4.w, cm, cp,
-                [&](uint32_t j, bool fromP, float4) {
-                    if (c < limit) list[sc_list_at(SC_LIST_M, i, c)] = fromP ? (j | SC_M_FROM_P) : j;
-                    c++;
-                });
+    const float lim = P.maxInt;
+    const bool wrap = IM.wrap;
+    uint32_t *out = list + sc_list_at(SC_LIST_M, i, 0);
+    scan_words(P, W, comb, cs, pp, reach(P, pp, lim, SC_BINNED_M | SC_BINNED_P), lim, scan_mixed(P, SC_BINNED_M | SC_BINNED_P), [&](int, float4 t) {
+        const uint32_t e = __float_as_uint(t.w);
+        if ((e & ~SC_M_ODD) == (uint32_t)i) return;
+        sc_f3 delta;
+        if (wrap) {
+            delta = IM(sc_make_f3(t.x, t.y, t.z)) - pp;
+            if (outside_cube(delta, lim)) return;
+        } else {
+            delta = sc_make_f3(t.x, t.y, t.z) - pp;
+        }
+        const bool fromP = (e & SC_M_FROM_P) != 0;
+        const float x = sc_normsq3(delta);
+        bool hit;
+        if (e & SC_M_ODD) {
+            hit = sqrtf(x) <= sc_coll_dist(p4.w, (fromP ? ppos_ : mpos)[e & SC_M_SLOT].w);
+        } else {
+            sc_sqrt_le le;
+            le.d = fromP ? leP.d : leM.d;
+            le.lo = fromP ? leP.lo : leM.lo;
+            le.hi = fromP ? leP.hi : leM.hi;
+            hit = sc_sqrt_le_test(le, x);
+        }
+        if (hit) {
+            if (c < limit) *out = e & ~SC_M_ODD;
+            out += 32;
+            c++;
+        }
+    });
 }
 
 // The full pair lists of the metabolic items whose list overflowed (listed
@@ -1369,16 +1419,24 @@ __device__ __forceinline__ void emit_m_pairs(const ScParams &P0, bool valid, int
     const Imager IM(P, pp, SC_BINNED_M | SC_BINNED_P);
     const float prad = p4.w;
     CollisionDistCache cm, cp;
-    for (int k = 0; k < S.n; k++) {
-        const uint32_t e = scratch[sc_list_at(SC_LIST_M, i, k)];
-        const int j = (int)(e & SC_M_INDEX);
-        const bool fromP = (e & SC_M_FROM_P) != 0;
-        const float4 t4 = fromP ? ppos_[j] : mpos[j];
-        const sc_f3 tpos = IM(sc_make_f3(t4.x, t4.y, t4.z));
-        const sc_f3 nd = normalize(tpos - pp);
-        const float cd = fromP ? cp.get(prad, t4.w) : cm.get(prad, t4.w);
-        const sc_f3 a = tpos - nd * cd;
-        S.out[(size_t)k * 32] = make_uint4(e, __float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(a.z));
+    // four pairs' entries, then their positions, in flight together
+    for (int k0 = 0; k0 < S.n; k0 += 4) {
+        uint32_t e[4];
+        float4 t4[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) e[q] = k0 + q < S.n ? scratch[sc_list_at(SC_LIST_M, i, k0 + q)] : 0u;
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            t4[q] = k0 + q < S.n ? ((e[q] & SC_M_FROM_P) ? ppos_ : mpos)[e[q] & SC_M_INDEX] : p4;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (k0 + q >= S.n) break;
+            const sc_f3 tpos = IM(sc_make_f3(t4[q].x, t4[q].y, t4[q].z));
+            const sc_f3 nd = normalize(tpos - pp);
+            const float cd = (e[q] & SC_M_FROM_P) ? cp.get(prad, t4[q].w) : cm.get(prad, t4[q].w);
+            const sc_f3 a = tpos - nd * cd;
+            S.out[(size_t)(k0 + q) * 32] = make_uint4(e[q], __float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(a.z));
+        }
     }
 }
 
@@ -1400,17 +1458,17 @@ __device__ __forceinline__ void emit_m_pairs_lean(const ScParams &P, bool valid,
 }
 
 template <bool LEAN, bool BATCH>
-__global__ void __launch_bounds__(SC_THREADS) k_build_m(ScParams P0, const uint32_t *__restrict__ cellStartM,
-                                                        const uint32_t *__restrict__ cellStartP,
+__global__ void __launch_bounds__(SC_THREADS, 4) k_build_m(ScParams P0, CombStart cs, const float4 *__restrict__ comb,
                                                         const int *__restrict__ nActivePtr,
                                                         const float4 *__restrict__ mpos, const int4 *__restrict__ minfo,
-                                                        const float4 *__restrict__ ppos_, const int4 *__restrict__ pinfo,
+                                                        const float4 *__restrict__ ppos_,
                                                         uint32_t *__restrict__ pool, long long poolCap,
                                                         unsigned long long *__restrict__ poolUsed,
                                                         long long *__restrict__ warpOff, uint32_t *scratch,
                                                         int *__restrict__ cnt, int *__restrict__ perm, int cap,
                                                         int *__restrict__ ovf, int *__restrict__ ovfCount,
                                                         int *__restrict__ ovfN) {
+    __shared__ ScanWords W;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = i < *nActivePtr;
     int c = 0;
@@ -1418,7 +1476,7 @@ __global__ void __launch_bounds__(SC_THREADS) k_build_m(ScParams P0, const uint3
         const int4 mi = minfo[i];
         ScParams P = P0;
         rep_apply<BATCH>(P, mi.w);
-        if (mi.z & SC_ACTIVE) build_m_item(P, cellStartM, cellStartP, i, mpos, minfo, ppos_, pinfo, scratch, c);
+        if (mi.z & SC_ACTIVE) build_m_item(P, W, cs, comb, i, mpos, ppos_, scratch, c);
     }
     if (LEAN)
         emit_m_pairs_lean(P0, valid, c, scratch, pool, poolCap, poolUsed, warpOff, cnt, perm, cap, ovf, ovfCount, ovfN);
@@ -1995,7 +2053,7 @@ __global__ void __launch_bounds__(SC_THREADS) k_copy_tail(const uint32_t *__rest
 // ---- metabolites.cuh:266-350 relaxMetabolicParticlePartners ----------------
 // Only lipids change, and only their own velocity, which no other thread of
 // this kernel reads: updated in place.  List: the colliding metabolic items.
-__device__ __forceinline__ void build_lm_item(const ScParams &P, const uint32_t *__restrict__ cellStartM, int i,
+__device__ __forceinline__ void build_lm_item(const ScParams &P, ScanWords &W, const uint32_t *__restrict__ cellStartM, int i,
                                               const float4 *__restrict__ ppos_, const float4 *__restrict__ mpos,
                                               const int4 *__restrict__ minfo, uint32_t *list, int &c) {
     float4 p4 = ppos_[i];
@@ -2003,16 +2061,15 @@ __device__ __forceinline__ void build_lm_item(const ScParams &P, const uint32_t 
     const Imager IM(P, pp, SC_BINNED_M);
     const float prad = p4.w, lim = P.maxInt;
     CollisionDistCache cc;
-    scan27(P, cellStartM, pp, reach(P, pp, lim, SC_BINNED_M), [&](int j) {
-        if (!active_m(P, minfo, j)) return;
-        float4 t4 = mpos[j];
-        sc_f3 delta = IM(sc_make_f3(t4.x, t4.y, t4.z)) - pp;
-        if (outside_cube(delta, lim)) return;
-        if (cc.collides(prad, t4.w, delta)) {
-            if (c < min(SC_LIST_LM, P.listLimit)) list[sc_list_at(SC_LIST_LM, i, c)] = (uint32_t)j;
-            c++;
-        }
-    });
+    scan_words(P, W, mpos, [&](uint32_t key) { return cellStartM[key]; }, pp, reach(P, pp, lim, SC_BINNED_M), lim,
+               scan_mixed(P, SC_BINNED_M), [&](int j, float4 t4) {
+                   sc_f3 delta = IM(sc_make_f3(t4.x, t4.y, t4.z)) - pp;
+                   if ((IM.wrap && outside_cube(delta, lim)) || !active_m(P, minfo, j)) return;
+                   if (cc.collides(prad, t4.w, delta)) {
+                       if (c < min(SC_LIST_LM, P.listLimit)) list[sc_list_at(SC_LIST_LM, i, c)] = (uint32_t)j;
+                       c++;
+                   }
+               });
 }
 
 // LM pairs with their frozen geometry, as the M pairs: per pair
@@ -2042,7 +2099,7 @@ __global__ void __launch_bounds__(SC_THREADS) k_lipid_select(const int *__restri
 }
 
 template <bool BATCH>
-__global__ void __launch_bounds__(SC_THREADS) k_build_lm(ScParams P0, const uint32_t *__restrict__ cellStartM,
+__global__ void __launch_bounds__(SC_THREADS, 4) k_build_lm(ScParams P0, const uint32_t *__restrict__ cellStartM,
                                                          const int *__restrict__ lipids,
                                                          const int *__restrict__ lipidCount,
                                                          const int4 *__restrict__ pinfo,
@@ -2053,13 +2110,14 @@ __global__ void __launch_bounds__(SC_THREADS) k_build_lm(ScParams P0, const uint
                                                          long long *__restrict__ warpOff,
                                                          uint32_t *scratch, int *__restrict__ cnt,
                                                          int *__restrict__ perm, int cap) {
+    __shared__ ScanWords W;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = t < *lipidCount;
     int c = 0;
     if (valid) {
         ScParams P = P0;
         rep_apply<BATCH>(P, pinfo[lipids[t]].w);
-        build_lm_item(P, cellStartM, lipids[t], ppos_, mpos, minfo, scratch, c);
+        build_lm_item(P, W, cellStartM, lipids[t], ppos_, mpos, minfo, scratch, c);
     }
     const PoolSlot<uint4> S = pool_take<SC_LIST_LM>(P0, valid, c, pool, poolCap, poolUsed, warpOff, cnt, perm, cap,
                                                     nullptr, nullptr, lipids);
@@ -2071,13 +2129,21 @@ __global__ void __launch_bounds__(SC_THREADS) k_build_lm(ScParams P0, const uint
     const Imager IM(P, pp, SC_BINNED_M);
     const float prad = p4.w;
     CollisionDistCache cc;
-    for (int k = 0; k < S.n; k++) {
-        const uint32_t j = scratch[sc_list_at(SC_LIST_LM, S.i, k)];
-        const float4 t4 = mpos[j];
-        const sc_f3 tpos = IM(sc_make_f3(t4.x, t4.y, t4.z));
-        const sc_f3 nd = normalize(tpos - pp);
-        const sc_f3 a = tpos - nd * cc.get(prad, t4.w);
-        S.out[(size_t)k * 32] = make_uint4(j, __float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(a.z));
+    for (int k0 = 0; k0 < S.n; k0 += 4) {
+        uint32_t j[4];
+        float4 t4[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) j[q] = k0 + q < S.n ? scratch[sc_list_at(SC_LIST_LM, S.i, k0 + q)] : 0u;
+#pragma unroll
+        for (int q = 0; q < 4; q++) t4[q] = k0 + q < S.n ? mpos[j[q]] : p4;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (k0 + q >= S.n) break;
+            const sc_f3 tpos = IM(sc_make_f3(t4[q].x, t4[q].y, t4[q].z));
+            const sc_f3 nd = normalize(tpos - pp);
+            const sc_f3 a = tpos - nd * cc.get(prad, t4[q].w);
+            S.out[(size_t)(k0 + q) * 32] = make_uint4(j[q], __float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(a.z));
+        }
     }
 }
 
@@ -2832,33 +2898,52 @@ __global__ void __launch_bounds__(SC_THREADS) k_propagate_state(
 // ---- metabolites.cuh:352-431 diffuseMetabolites ------------------------------
 // List: the metabolic items within maxDiffusionDistance (cube, then sphere),
 // built after applyVelocities and read by all diffusion sub-iterations.
-__device__ __forceinline__ void build_d_item(const ScParams &P, const uint32_t *__restrict__ cellStart, int i,
+__device__ __forceinline__ void build_d_item(const ScParams &P, ScanWords &W, const uint32_t *__restrict__ cellStart, int i,
                                              const float4 *__restrict__ pos, const int4 *__restrict__ info,
                                              uint32_t *list, int &c) {
     float4 p4 = pos[i];
     const sc_f3 pp = sc_make_f3(p4.x, p4.y, p4.z);
-    const Imager IM(P, pp, SC_BINNED_M);
+    Imager IM(P, pp, SC_BINNED_M);
     const float lim = P.maxDiff;
+    // The items have moved since their sort.  When each moved once, by no
+    // more than a cell, the neighbours of an item two cells or more from
+    // every face (sorted into cells one or more from it) have not crossed
+    // one: no image is nearer than they are.
+    if (IM.wrap && P.movedOnce && P.simSize >= 7.0f * P.cell && *P.farMove == 0) {
+        const int n = P.nUsed;
+        const int cx = (int)sc_grid_idx(pp.x, P.cell, n), cy = (int)sc_grid_idx(pp.y, P.cell, n),
+                  cz = (int)sc_grid_idx(pp.z, P.cell, n);
+        IM.wrap = min(cx, min(cy, cz)) < 2 || max(cx, max(cy, cz)) > n - 3;
+    }
     const sc_sqrt_le within = sc_sqrt_le_make(lim);
-    scan27(P, cellStart, pp, reach(P, pp, lim, SC_BINNED_M), [&](int j) {
-        if (j == i || !active_m(P, info, j)) return;
-        float4 t4 = pos[j];
-        sc_f3 delta = IM(sc_make_f3(t4.x, t4.y, t4.z)) - pp;
-        if (outside_cube(delta, lim)) return;
-        if (sc_sqrt_le_test(within, sc_normsq3(delta))) {
-            if (c < min(SC_LIST_D, P.listLimit)) list[sc_list_at(SC_LIST_D, i, c)] = (uint32_t)j;
-            c++;
-        }
-    });
+    const int limit = min(SC_LIST_D, P.listLimit);
+    uint32_t *out = list + sc_list_at(SC_LIST_D, i, 0);
+    scan_words(P, W, pos, [&](uint32_t key) { return cellStart[key]; }, pp, reach(P, pp, lim, SC_BINNED_M), lim, IM.wrap,
+               [&](int j, float4 t4) {
+                   if (j == i || !active_m(P, info, j)) return;
+                   sc_f3 delta;
+                   if (IM.wrap) {
+                       delta = IM(sc_make_f3(t4.x, t4.y, t4.z)) - pp;
+                       if (outside_cube(delta, lim)) return;
+                   } else {
+                       delta = sc_make_f3(t4.x, t4.y, t4.z) - pp;
+                   }
+                   if (sc_sqrt_le_test(within, sc_normsq3(delta))) {
+                       if (c < limit) *out = (uint32_t)j;
+                       out += 32;
+                       c++;
+                   }
+               });
 }
 
 template <bool BATCH>
-__global__ void __launch_bounds__(SC_THREADS) k_build_d(ScParams P, const uint32_t *__restrict__ cellStart,
+__global__ void __launch_bounds__(SC_THREADS, 4) k_build_d(ScParams P, const uint32_t *__restrict__ cellStart,
                                                         const int *__restrict__ nActivePtr,
                                                         const float4 *__restrict__ pos, const int4 *__restrict__ info,
                                                         uint32_t *__restrict__ list, uint32_t *scratch,
                                                         int *__restrict__ cnt, int *__restrict__ perm, int cap,
                                                         int *__restrict__ ovf, int *__restrict__ ovfCount) {
+    __shared__ ScanWords W;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = i < *nActivePtr;
     int c = 0;
@@ -2866,7 +2951,7 @@ __global__ void __launch_bounds__(SC_THREADS) k_build_d(ScParams P, const uint32
         const int4 in = info[i];
         ScParams Q = P;
         rep_apply<BATCH>(Q, in.w);
-        if (in.z & SC_ACTIVE) build_d_item(Q, cellStart, i, pos, info, scratch, c);
+        if (in.z & SC_ACTIVE) build_d_item(Q, W, cellStart, i, pos, info, scratch, c);
     }
     emit_count_ordered<SC_LIST_D>(valid, c, P.listLimit, cap, scratch, list, cnt, perm, ovf, ovfCount);
 }
@@ -3326,11 +3411,15 @@ void sc_phase_build_m(ScLaunchCtx &c) {
                 B.cntM, B.ovfM, &B.ctr->ovfM);
         } else {
             cudaMemsetAsync(&B.ctr->poolM, 0, sizeof(B.ctr->poolM), c.st);
+            const CombStart cs{B.cellStartM, B.cellStartP};
+            k_combine<<<(int)std::min<long long>(((long long)c.P.N + c.P.Nm + SC_THREADS - 1) / SC_THREADS, 8 * c.gridCap),
+                        SC_THREADS, 0, c.st>>>(c.P, B.keysM[B.sortCurM], B.keysP[B.sortCurP], cs, M.pos, M.info, F.pos,
+                                               F.info, B.comb);
+            (*c.launches)++;
             (c.P.nRep > 1 ? (c.P.metabLean ? k_build_m<true, true> : k_build_m<false, true>)
                           : (c.P.metabLean ? k_build_m<true, false> : k_build_m<false, false>))<<<
                 nblocks(c.P.Nm), SC_THREADS, 0, c.st>>>(
-                c.P, B.cellStartM, B.cellStartP, &B.ctr->nActiveM, M.pos, M.info, F.pos, F.info, B.listM,
-                (long long)B.poolCapM, &B.ctr->poolM, B.warpOffM, B.listD, B.cntM, B.permM, c.P.Nm, B.ovfM, &B.ctr->ovfM,
+                c.P, cs, B.comb, &B.ctr->nActiveM, M.pos, M.info, F.pos, B.listM, (long long)B.poolCapM, &B.ctr->poolM, B.warpOffM, B.listD, B.cntM, B.permM, c.P.Nm, B.ovfM, &B.ctr->ovfM,
                 B.ovfNM);
             // the overflowed items' full lists
             cudaMemsetAsync(&B.ctr->poolOvfM, 0, sizeof(B.ctr->poolOvfM), c.st);
@@ -3424,13 +3513,13 @@ void sc_phase_apply_velocities(ScLaunchCtx &c) {
     if (c.P.N > 0) {
         PFields F = B.P();
         SC_BATCHED(k_apply_velocities)<<<nblocks(c.P.N), SC_THREADS, 0, c.st>>>(&B.ctr->nActive, F.info, F.pos, F.vel, F.rot,
-                                                                     F.angvel, c.P, 0.45f);
+                                                                     F.angvel, c.P, 0.45f, nullptr);
         (*c.launches)++;
     }
     if (c.P.Nm > 0) {
         MFields M = B.M();
         SC_BATCHED(k_apply_velocities)<<<nblocks(c.P.Nm), SC_THREADS, 0, c.st>>>(&B.ctr->nActiveM, M.info, M.pos, M.vel, M.rot,
-                                                                      M.angvel, c.P, 0.45f);
+                                                                      M.angvel, c.P, 0.45f, &B.ctr->farMove);
         (*c.launches)++;
     }
 }
