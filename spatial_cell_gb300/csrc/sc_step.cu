@@ -2406,29 +2406,64 @@ __device__ __forceinline__ unsigned long long claim_key(sc_f3 delta, int i) {
     return ((unsigned long long)sc_f2u(sc_normsq3(delta)) << 32) | (unsigned)i;
 }
 
+// Whether some rule of a type (partner-mapped rules [cs, ce)) can bond it to
+// type b at all: the part of claim_rule that needs no more of the candidate.
+__device__ __forceinline__ bool claim_types(const ScParams &P, int type, int cs, int ce, int b) {
+    for (int k = cs; k < ce; k++) {
+        const sc_rule &pii = P.prules[k];
+        if (((type == pii.first_partner_type && b == pii.second_partner_type) ||
+             (type == pii.second_partner_type && b == pii.first_partner_type)) &&
+            !pii.only_via_transition)
+            return true;
+    }
+    return false;
+}
+
+// A warp per open item, a lane per neighbour cell: offers are taken by
+// atomicMin, so their order is free.  With a thread per item 6 of a warp's 32
+// lanes were busy and an item's 27 cells were one chain of dependent loads;
+// and a candidate's records are only read once its type has a rule (10 % of
+// the candidates in the cube at the measured mix).  A quarter of the large
+// workload: 174 -> 126 us; a step of 4,096 + 8,192 items is 0.13 ms shorter.
 template <bool BATCH>
-__global__ void __launch_bounds__(SC_THREADS, 3) k_claim_offer(
+__global__ void __launch_bounds__(SC_THREADS) k_claim_offer(
     ScParams P, const uint32_t *__restrict__ cellStart, const int *__restrict__ work, const int *__restrict__ workCount,
     const float4 *__restrict__ pos, const float4 *__restrict__ rot, const int4 *__restrict__ info,
     const int *__restrict__ state, const int *__restrict__ nbIn, const int *__restrict__ bonds,
     const int *__restrict__ stepPtr, int prep, unsigned long long *claim) {
   const int step = prep ? -1 : *stepPtr;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < *workCount; t += gridDim.x * blockDim.x) {
+  const int lane = threadIdx.x & 31;
+  const int ox = lane / 9 - 1, oy = lane / 3 % 3 - 1, oz = lane % 3 - 1;
+  const int n = *workCount;
+  for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < n; t += (gridDim.x * blockDim.x) >> 5) {
     const int i = work[t];
     rep_apply<BATCH>(P, info[i].w);
     const ClaimItem a = claim_item(P, pos, rot, info, state, nbIn, bonds, i);
-    if (a.nb >= SC_MAX_ACTIVE_INTERACTIONS) continue;
-    const Imager IM(P, a.pos, SC_BINNED_P);
+    if (a.nb >= SC_MAX_ACTIVE_INTERACTIONS || lane >= 27) continue;
     const float lim = P.maxInt;
-    scan27(P, cellStart, a.pos, reach(P, a.pos, lim, SC_BINNED_P), [&](int j) {
-        if (j == i) return;
+    const Reach R = reach(P, a.pos, lim, SC_BINNED_P);
+    if (ox < R.xl || ox > R.xh || oy < R.yl || oy > R.yh || oz < R.zl || oz > R.zh) continue;
+    const int g = cell_limit(P);
+    int gx = (int)sc_grid_idx(a.pos.x, P.cell, g) + ox, gy = (int)sc_grid_idx(a.pos.y, P.cell, g) + oy,
+        gz = (int)sc_grid_idx(a.pos.z, P.cell, g) + oz;
+    if (P.periodic) {
+        gx = (int)wrap_cell(gx, g);
+        gy = (int)wrap_cell(gy, g);
+        gz = (int)wrap_cell(gz, g);
+    } else if (min(gx, min(gy, gz)) < 0 || max(gx, max(gy, gz)) >= g) {
+        continue;
+    }
+    const Imager IM(P, a.pos, SC_BINNED_P);
+    const uint32_t key = cell_key(P, (uint32_t)gx, (uint32_t)gy, (uint32_t)gz);
+    for (int j = (int)cellStart[key], e = (int)cellStart[key + 1]; j < e; j++) {
         const float4 t4 = pos[j];
+        const int4 in = info[j];
+        if (j == i) continue;
         const sc_f3 delta = IM(sc_make_f3(t4.x, t4.y, t4.z)) - a.pos;
-        if (outside_cube(delta, lim)) return;
-        if (!(info[j].z & SC_ACTIVE)) return;
+        if (outside_cube(delta, lim) || !(in.z & SC_ACTIVE) || !claim_types(P, a.type, a.cs, a.ce, in.y)) continue;
         const ClaimItem b = claim_item(P, pos, rot, info, state, nbIn, bonds, j);
         if (claim_rule(P, a, b, delta, step) >= 0) atomicMin(&claim[j], claim_key(delta, i));
-    });
+    }
   }
 }
 
@@ -3538,7 +3573,7 @@ void sc_phase_complexify(ScLaunchCtx &c, bool prep) {
         (*c.launches) += 2;
     } else {
         cudaMemsetAsync(B.claimP, 0xff, (size_t)c.P.N * sizeof(unsigned long long), c.st);
-        SC_BATCHED(k_claim_offer)<<<blocks, SC_THREADS, 0, c.st>>>(c.P, B.cellStartP, B.workP, &B.ctr->workCount, F.pos, F.rot,
+        SC_BATCHED(k_claim_offer)<<<std::min(nblocks(c.P.N) * 8, 4 * c.gridCap), SC_THREADS, 0, c.st>>>(c.P, B.cellStartP, B.workP, &B.ctr->workCount, F.pos, F.rot,
                                                        F.info, F.state, F.nb, F.bonds, &B.ctr->step, prep, B.claimP);
         SC_BATCHED(k_claim_bind)<<<blocks, SC_THREADS, 0, c.st>>>(c.P, B.workP, &B.ctr->workCount, F.pos, F.rot, F.info, F.state,
                                                       F.nb, X.nb, F.bonds, &B.ctr->step, prep, B.claimP);
