@@ -1067,7 +1067,8 @@ extern "C" {
 
 #if !defined(SC_PORT_FP64)
 // ---- scmath.h entry points for the CPU tests ---------------------------------
-// fn: 0 sin, 1 cos, 2 acos, 3 log, 4 exp, 5 pow(x, y)
+// fn: 0 sin, 1 cos, 2 acos, 3 log, 4 exp, 5 pow(x, y), 6 / 7 sin / cos of
+// sc_sincosf, 8 / 9 the first / last sine of sc_sin3(x, y, -x)
 void scp_math_eval(int fn, const float *x, const float *y, float *out, int n) {
     for (int i = 0; i < n; i++) {
         switch (fn) {
@@ -1076,6 +1077,10 @@ void scp_math_eval(int fn, const float *x, const float *y, float *out, int n) {
             case 2: out[i] = sc_acosf(x[i]); break;
             case 3: out[i] = sc_logf(x[i]); break;
             case 4: out[i] = sc_expf(x[i]); break;
+            case 6: out[i] = sc_sincosf(x[i]).x; break;
+            case 7: out[i] = sc_sincosf(x[i]).y; break;
+            case 8: out[i] = sc_sin3(x[i], y[i], -x[i]).x; break;
+            case 9: out[i] = sc_sin3(y[i], x[i], -x[i]).z; break;
             default: out[i] = sc_powf(x[i], y[i]); break;
         }
     }

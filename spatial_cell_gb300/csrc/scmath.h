@@ -182,6 +182,47 @@ SC_HD_COLD float sc_cosf(float x) {
     return q == 0 ? c : q == 1 ? -s : q == 2 ? -c : s;
 }
 
+// sc_sinf(x) and sc_cosf(x) of one argument, reduced once: the same bits.
+SC_HD_COLD sc_f2 sc_sincosf(float x) {
+    sc_f2 o;
+    float r, s, c;
+    if (!sc_isfinitef(x)) {
+        o.x = o.y = x - x;
+        return o;
+    }
+    int q = sc_reduce_pio2(x, &r);
+    s = sc_sin_poly(r);
+    c = sc_cos_poly(r);
+    o.x = x == 0.0f ? x : (q == 0 ? s : q == 1 ? c : q == 2 ? -s : -c);
+    o.y = q == 0 ? c : q == 1 ? -s : q == 2 ? -c : s;
+    return o;
+}
+// sc_sinf of three arguments, their evaluations side by side: one argument's
+// is a chain of some forty dependent operations.
+typedef struct {
+    float x, y, z;
+} sc_sin3_t;
+SC_HD sc_sin3_t sc_sin3(float a, float b, float c) {
+    sc_sin3_t o;
+    if (!(fabsf(a) <= 1000.0f && fabsf(b) <= 1000.0f && fabsf(c) <= 1000.0f)) {
+        o.x = sc_sinf(a);
+        o.y = sc_sinf(b);
+        o.z = sc_sinf(c);
+        return o;
+    }
+    const float v[3] = {a, b, c};
+    float r[3], s[3], k[3];
+    int q[3];
+    for (int i = 0; i < 3; i++) q[i] = sc_reduce_pio2(v[i], &r[i]);
+    for (int i = 0; i < 3; i++) s[i] = sc_sin_poly(r[i]);
+    for (int i = 0; i < 3; i++) k[i] = sc_cos_poly(r[i]);
+    for (int i = 0; i < 3; i++) s[i] = v[i] == 0.0f ? v[i] : (q[i] == 0 ? s[i] : q[i] == 1 ? k[i] : q[i] == 2 ? -s[i] : -k[i]);
+    o.x = s[0];
+    o.y = s[1];
+    o.z = s[2];
+    return o;
+}
+
 // asin on [0, 0.5]: z + z^3 * sum_n c_n z^(2n-2), c_n = (2n)!/(4^n (n!)^2 (2n+1)).
 SC_HD float sc_asin_poly(float z) {
     float w = z * z;
@@ -455,8 +496,8 @@ SC_HD float sc_angle3(sc_f3 a, sc_f3 b) {
 
 // math.cuh:143-155
 SC_HD sc_f4 sc_quat(sc_f3 axis, float angle) {
-    float s = sc_sinf(angle * 0.5f);
-    float c = sc_cosf(angle * 0.5f);
+    const sc_f2 sc = sc_sincosf(angle * 0.5f);
+    const float s = sc.x, c = sc.y;
     return normalize(sc_make_f4(axis.x * s, axis.y * s, axis.z * s, c));
 }
 
@@ -473,9 +514,10 @@ SC_HD sc_f4 sc_qinv(sc_f4 a) {
 // The weights of slerp for an angle whose cosine is cosO (not near 1).
 SC_HD_COLD sc_f2 sc_slerp_weights(float cosO, float t, bool flip) {
     float omega = sc_acosf(cosO);
-    float invSin = 1.0f / sc_sinf(omega);
-    float s1 = sc_sinf((1.0f - t) * omega) * invSin;
-    float s2 = flip ? -sc_sinf(t * omega) * invSin : sc_sinf(t * omega) * invSin;
+    const sc_sin3_t sn = sc_sin3(omega, (1.0f - t) * omega, t * omega);
+    float invSin = 1.0f / sn.x;
+    float s1 = sn.y * invSin;
+    float s2 = flip ? -sn.z * invSin : sn.z * invSin;
     sc_f2 r;
     r.x = s1;
     r.y = s2;
@@ -503,7 +545,8 @@ SC_HD sc_f4 sc_slerp(sc_f4 a, sc_f4 b, float t) {
 SC_HD sc_f4 sc_random_rotation(float u, float v, float w) {
     float su = sqrtf(u), su1 = sqrtf(1.0f - u);
     float tp = 2.0f * SC_PI_REF;
-    return sc_make_f4(su1 * sc_sinf(tp * v), su1 * sc_cosf(tp * v), su * sc_sinf(tp * w), su * sc_cosf(tp * w));
+    const sc_f2 a = sc_sincosf(tp * v), b = sc_sincosf(tp * w);
+    return sc_make_f4(su1 * a.x, su1 * a.y, su * b.x, su * b.y);
 }
 
 // math.cuh:309-338 (rotation-matrix form; evaluated literally so signed zeros
