@@ -422,8 +422,11 @@ void sort_metabolic(sc_sim *s) {
 // Which pair lists a phase invalidates (it changes positions, flags, types,
 // radii or interactions their tests read, or re-sorts slots they index).
 void invalidate_after(ScBuffers &B, int phase) {
-    // only the relaxation loop's phases leave rot and angvel to relax alone
-    if (phase != SC_PHASE_RELAX && phase != SC_PHASE_RELAX_METAB && phase != SC_PHASE_RELAX_PARTNERS) B.relaxAge = 0;
+    // only the relaxation loop's phases leave rot and angvel to relax alone,
+    // and the metabolic velocities to relax_metab
+    if (phase != SC_PHASE_RELAX && phase != SC_PHASE_RELAX_METAB && phase != SC_PHASE_RELAX_PARTNERS)
+        B.relaxAge = B.relaxMAge = 0;
+    if (phase != SC_PHASE_DIFFUSE) B.diffuseAge = 0;
     switch (phase) {
         case SC_PHASE_SORT_PARTICLES: B.validPP = B.validM = B.validLM = false; break;
         case SC_PHASE_SORT_METABOLIC: B.validM = B.validLM = B.validD = false; break;
@@ -457,7 +460,8 @@ std::vector<int> host_state(const sc_sim *s) {
     std::vector<int> v(B.cp, B.cp + FP_COUNT);
     v.insert(v.end(), B.cm, B.cm + FM_COUNT);
     v.insert(v.end(), {B.sortCurP, B.sortCurM, (int)B.validPP, (int)B.validM, (int)B.validLM, (int)B.validD,
-                       s->P.binned, s->P.mAllActive, s->P.lipidValid, B.mParity, B.relaxAge, s->P.movedOnce});
+                       s->P.binned, s->P.mAllActive, s->P.lipidValid, B.mParity, B.relaxAge, s->P.movedOnce, B.relaxMAge,
+                       B.diffuseAge});
     return v;
 }
 void set_host_state(sc_sim *s, const std::vector<int> &v) {
@@ -477,6 +481,8 @@ void set_host_state(sc_sim *s, const std::vector<int> &v) {
     B.setMParity(v[k++]);
     B.relaxAge = v[k++];
     s->P.movedOnce = v[k++];
+    B.relaxMAge = v[k++];
+    B.diffuseAge = v[k++];
 }
 
 int run_phase(sc_sim *s, int phase, int arg) {

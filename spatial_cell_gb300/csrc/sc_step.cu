@@ -1499,6 +1499,14 @@ struct RelaxMArgs {
     const float4 *__restrict__ pvel;
     const uint4 *__restrict__ pool;     // pairs with their geometry (emit_m_pairs)
     const long long *__restrict__ warpOff;
+    // the items whose list overflowed (k_build_m), with their pair counts and
+    // regions of the overflow pool (ovfOff null: none is kept whole)
+    const int *__restrict__ ovf, *__restrict__ ovfCount, *__restrict__ ovfN;
+    const long long *__restrict__ ovfOff;
+    const uint4 *__restrict__ ovfPool;
+    // launches since the sort: from the second on both velocity buffers hold
+    // the inactive items' velocities
+    int age;
 };
 
 // The contribution of one colliding neighbour (a metabolic item, or a lipid
@@ -1517,54 +1525,205 @@ __device__ __forceinline__ float4 metab_pair_vel(const RelaxMArgs &A, uint32_t e
     return ((e & SC_M_FROM_P) ? A.pvel : A.mvelIn)[e & SC_M_INDEX];
 }
 
-// Items whose list fits, in count order: each pair adds its precomputed
-// geometry and the neighbour's current velocity, in list order.  Pairs are
-// taken SC_METAB_GROUP at a time: the group's neighbour velocities and the
-// next group's entries are all in flight together, so a thread waits about
-// one memory latency per group instead of one per pair.  Entries are read
-// once per launch (evict-first); velocities are re-read by nearby items.
-#define SC_METAB_GROUP 4
-__global__ void __launch_bounds__(SC_THREADS, 4) k_relax_metab(ScParams P, RelaxMArgs A) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;   // list position (count-ordered)
-    if (g >= *A.nActivePtr) return;
-    const int i = A.L.perm[g];
+// One pair of a pool: its precomputed geometry and the neighbour's current
+// velocity (metabolites.cuh:196-203 / 235-242).
+__device__ __forceinline__ void metab_pool_term(uint4 E, float4 tv, sc_f3 ppv, sc_f3 &dV, float &w) {
+    const float kw = (E.x & SC_M_FROM_P) ? 2.0f : 1.0f;
+    const sc_f3 a = sc_make_f3(__uint_as_float(E.y), __uint_as_float(E.z), __uint_as_float(E.w));
+    w += kw;
+    dV += (a + sc_make_f3(tv.x, tv.y, tv.z) - ppv) * 0.9f * kw;
+}
+
+// An item whose list overflowed: the reference's loops over the 27 cells.
+template <bool BATCH>
+__device__ __noinline__ void relax_metab_scan_item(const ScParams &P0, const RelaxMArgs &A, int i) {
     if (i < 0) return;
-    const float4 v4 = A.mvelIn[i];
+    const int4 mi = A.minfo[i];
+    if (!(mi.z & SC_ACTIVE)) return;
+    ScParams P = P0;
+    rep_apply<BATCH>(P, mi.w);
+    float4 v4 = A.mvelIn[i];
+    float4 p4 = A.mpos[i];
+    const sc_f3 pp = sc_make_f3(p4.x, p4.y, p4.z);
+    const Imager IM(P, pp, SC_BINNED_M | SC_BINNED_P);
+    const float prad = p4.w;
+    const sc_f3 pv = sc_make_f3(v4.x, v4.y, v4.z);
+    const sc_f3 ppv = pp + pv;
+    sc_f3 dV = sc_zero3();
+    float w = 0.0f;
+    CollisionDistCache cm, cp;
+    const float lim = P.maxInt;
+    cells27(P, pp, reach(P, pp, lim, SC_BINNED_M | SC_BINNED_P), [&](uint32_t key) {
+        for (uint32_t j = A.cellStartM[key], e = A.cellStartM[key + 1]; j < e; j++) {
+            if ((int)j == i) continue;
+            if (!active_m(P, A.minfo, (int)j)) continue;
+            float4 t4 = A.mpos[j];
+            sc_f3 delta = IM(sc_make_f3(t4.x, t4.y, t4.z)) - pp;
+            if (outside_cube(delta, lim)) continue;
+            if (cm.collides(prad, t4.w, delta))
+                metab_pair(IM, pp, ppv, t4, A.mvelIn[j], cm.get(prad, t4.w), false, dV, w);
+        }
+        for (uint32_t j = A.cellStartP[key], e = A.cellStartP[key + 1]; j < e; j++) {
+            if (!active_lipid(P, A.pinfo, (int)j)) continue;
+            float4 t4 = A.ppos[j];
+            sc_f3 delta = IM(sc_make_f3(t4.x, t4.y, t4.z)) - pp;
+            if (outside_cube(delta, lim)) continue;
+            if (cp.collides(prad, t4.w, delta))
+                metab_pair(IM, pp, ppv, t4, A.pvel[j], cp.get(prad, t4.w), true, dV, w);
+        }
+    });
+    st3(A.mvelOut, i, pv + dV / fmaxf(w, 1.0f), v4.w);
+}
+
+// Lists of the overflow pool longer than this are walked by a whole warp,
+// shorter ones by one thread (both in relax_metab_overflow): a list that
+// overflowed because the main pool had no room for its block fits the list
+// capacity, one that outgrew the capacity (a wall pile's) holds hundreds to
+// thousands of pairs.  With the list capacity capped (pair_list_limit, the
+// tests' way into the overflow paths) the bound is four times the cap, so
+// ordinary lists take both walks.
+#define SC_POOL_WARP_MIN SC_LIST_M
+__device__ __forceinline__ int pool_warp_min(const ScParams &P) {
+    return P.listLimit < SC_POOL_WARP_MIN / 4 ? 4 * P.listLimit : SC_POOL_WARP_MIN;
+}
+
+// The items whose list overflowed, by `blocks` blocks of which this is block
+// `blk`.  First a thread each: an item the overflow pool had no room for
+// scans its neighbourhood; one whose region there is short walks it as
+// k_relax_metab walks the main pool.  Then a warp for each longer region,
+// warp-stride so the long lists of a wall pile spread over the device: the
+// lanes load 32 entries and the neighbours' velocities at once and each forms
+// its pair's term and weight; lanes 0-2 add the terms' components and lane 3
+// the weights in list order from shared memory -- the sums a thread walking
+// the list forms, at one gather latency per 32 pairs.
+#define SC_TERM_ROW 5   // x, y, z, weight (odd row length: no bank conflicts)
+template <bool BATCH>
+__device__ __noinline__ void relax_metab_overflow(const ScParams &P, const RelaxMArgs &A, int blk, int blocks,
+                                                  float (*sTerm)[32][SC_TERM_ROW]) {
+    const int nOvf = *A.ovfCount, warpMin = pool_warp_min(P);
+    for (int t = blk * SC_THREADS + threadIdx.x; t < nOvf; t += blocks * SC_THREADS) {
+        const int i = A.ovf[t];
+        const long long off = A.ovfOff ? A.ovfOff[t] : -1;
+        if (off < 0) {
+            relax_metab_scan_item<BATCH>(P, A, i);
+            continue;
+        }
+        const int n = A.ovfN[t];
+        if (i < 0 || n > warpMin || !(A.minfo[i].z & SC_ACTIVE)) continue;
+        const float4 v4 = A.mvelIn[i], p4 = A.mpos[i];
+        const sc_f3 pv = sc_make_f3(v4.x, v4.y, v4.z);
+        const sc_f3 ppv = sc_make_f3(p4.x, p4.y, p4.z) + pv;
+        sc_f3 dV = sc_zero3();
+        float w = 0.0f;
+        const uint4 *__restrict__ e = A.ovfPool + off;
+        for (int k0 = 0; k0 < n; k0 += 4) {
+            uint4 E[4];
+            float4 tv[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) E[q] = k0 + q < n ? e[k0 + q] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+            for (int q = 0; q < 4; q++) tv[q] = k0 + q < n ? metab_pair_vel(A, E[q].x) : make_float4(0, 0, 0, 0);
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (k0 + q < n) metab_pool_term(E[q], tv[q], ppv, dV, w);
+        }
+        st3(A.mvelOut, i, pv + dV / fmaxf(w, 1.0f), v4.w);
+    }
+    if (!A.ovfOff) return;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (int t = blk * (SC_THREADS / 32) + wid; t < nOvf; t += blocks * (SC_THREADS / 32)) {
+        const int i = A.ovf[t], n = A.ovfN[t];
+        const long long off = A.ovfOff[t];
+        if (off < 0 || i < 0 || n <= warpMin || !(A.minfo[i].z & SC_ACTIVE)) continue;   // warp-uniform
+        const float4 v4 = A.mvelIn[i], p4 = A.mpos[i];
+        const sc_f3 pv = sc_make_f3(v4.x, v4.y, v4.z);
+        const sc_f3 ppv = sc_make_f3(p4.x, p4.y, p4.z) + pv;
+        const uint4 *__restrict__ e = A.ovfPool + off;
+        float acc = 0.0f;   // lanes 0-2: dV's components; lane 3: the weight
+        for (int b = 0; b < n; b += 32) {
+            float term[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            if (b + lane < n) {
+                const uint4 E = e[b + lane];
+                const float4 tv = metab_pair_vel(A, E.x);
+                const float kw = (E.x & SC_M_FROM_P) ? 2.0f : 1.0f;
+                const sc_f3 a = sc_make_f3(__uint_as_float(E.y), __uint_as_float(E.z), __uint_as_float(E.w));
+                const sc_f3 d = (a + sc_make_f3(tv.x, tv.y, tv.z) - ppv) * 0.9f * kw;
+                term[0] = d.x;
+                term[1] = d.y;
+                term[2] = d.z;
+                term[3] = kw;
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) sTerm[wid][lane][k] = term[k];
+            __syncwarp();
+            if (lane < 4) {
+                const int m = min(32, n - b);
+                for (int u = 0; u < m; u++) acc += sTerm[wid][u][lane];
+            }
+            __syncwarp();
+        }
+        const float dy = __shfl_sync(0xffffffffu, acc, 1), dz = __shfl_sync(0xffffffffu, acc, 2),
+                    w = __shfl_sync(0xffffffffu, acc, 3);
+        if (lane == 0) st3(A.mvelOut, i, pv + sc_make_f3(acc, dy, dz) / fmaxf(w, 1.0f), v4.w);
+    }
+}
+
+// The metabolic sweep: the items whose list fits, in count order; at G = 8 the
+// first `extra` blocks take the overflowed items (the longest lists start
+// first).  Pairs are taken G at a time: the group's neighbour velocities and
+// the next group's entries are all in flight together, so a thread waits
+// about one memory latency per group instead of one per pair.  Entries are
+// read once per launch (evict-first) and lie at a place known from the list
+// position, so they are on their way with the item's own records; velocities
+// are re-read by nearby items.  Inactive items' velocities are copied until
+// both buffers hold them.
+//
+// G = 4 keeps four blocks per SM for sims that fill the device, where the
+// pool's stream from HBM bounds the launch; G = 8 halves the rounds of sims
+// that do not, where the rounds' latency does.
+template <int G, bool BATCH>
+__global__ void __launch_bounds__(SC_THREADS, G == 4 ? 4 : 2) k_relax_metab(ScParams P, RelaxMArgs A, int extra) {
+    if constexpr (G == 8) {
+        __shared__ float sTerm[SC_THREADS / 32][32][SC_TERM_ROW];
+        if ((int)blockIdx.x < extra) {
+            if (*A.ovfCount > 0) relax_metab_overflow<BATCH>(P, A, blockIdx.x, extra, sTerm);
+            return;
+        }
+    }
+    const int g = ((int)blockIdx.x - extra) * SC_THREADS + threadIdx.x;   // list position (count-ordered)
+    if (g >= *A.nActivePtr) return;
+    const int i = A.L.perm[g], c = A.L.cnt[g];
+    const uint4 *pairs = A.pool + A.warpOff[g >> 5] + (g & 31);
     // after the sort the active items are exactly the binned ones
-    const bool act = P.mAllActive ? i < (int)A.cellStartM[P.cells] : (A.minfo[i].z & SC_ACTIVE) != 0;
+    const int binned = P.mAllActive ? (int)A.cellStartM[P.cells] : 0;
+    if (i < 0) return;
+    const bool act = P.mAllActive ? i < binned : (A.minfo[i].z & SC_ACTIVE) != 0;
     if (!act) {
-        A.mvelOut[i] = v4;
+        if (A.age == 0) A.mvelOut[i] = A.mvelIn[i];
         return;
     }
-    const int c = A.L.cnt[g];
     if (c > min(SC_LIST_M, P.listLimit)) return;
-    const float4 p4 = A.mpos[i];
+    const float4 v4 = A.mvelIn[i], p4 = A.mpos[i];
+    uint4 E[G];
+#pragma unroll
+    for (int q = 0; q < G; q++) E[q] = q < c ? __ldcs(pairs + (size_t)q * 32) : make_uint4(0, 0, 0, 0);
     const sc_f3 pv = sc_make_f3(v4.x, v4.y, v4.z);
     const sc_f3 ppv = sc_make_f3(p4.x, p4.y, p4.z) + pv;
     sc_f3 dV = sc_zero3();
     float w = 0.0f;
-    const uint4 *pairs = A.pool + A.warpOff[g >> 5] + (g & 31);
-    uint4 E[SC_METAB_GROUP];
+    for (int k0 = 0; k0 < c; k0 += G) {
+        float4 tv[G];
+        uint4 En[G];
 #pragma unroll
-    for (int q = 0; q < SC_METAB_GROUP; q++) E[q] = q < c ? __ldcs(pairs + (size_t)q * 32) : make_uint4(0, 0, 0, 0);
-    for (int k0 = 0; k0 < c; k0 += SC_METAB_GROUP) {
-        float4 tv[SC_METAB_GROUP];
-        uint4 En[SC_METAB_GROUP];
+        for (int q = 0; q < G; q++) tv[q] = k0 + q < c ? metab_pair_vel(A, E[q].x) : make_float4(0, 0, 0, 0);
 #pragma unroll
-        for (int q = 0; q < SC_METAB_GROUP; q++) tv[q] = k0 + q < c ? metab_pair_vel(A, E[q].x) : make_float4(0, 0, 0, 0);
-#pragma unroll
-        for (int q = 0; q < SC_METAB_GROUP; q++) {
-            const int k = k0 + SC_METAB_GROUP + q;
+        for (int q = 0; q < G; q++) {
+            const int k = k0 + G + q;
             En[q] = k < c ? __ldcs(pairs + (size_t)k * 32) : make_uint4(0, 0, 0, 0);
         }
 #pragma unroll
-        for (int q = 0; q < SC_METAB_GROUP; q++) {
-            if (k0 + q < c) {
-                const float kw = (E[q].x & SC_M_FROM_P) ? 2.0f : 1.0f;
-                const sc_f3 a = sc_make_f3(__uint_as_float(E[q].y), __uint_as_float(E[q].z), __uint_as_float(E[q].w));
-                w += kw;
-                dV += (a + sc_make_f3(tv[q].x, tv[q].y, tv[q].z) - ppv) * 0.9f * kw;
-            }
+        for (int q = 0; q < G; q++) {
+            if (k0 + q < c) metab_pool_term(E[q], tv[q], ppv, dV, w);
             E[q] = En[q];
         }
     }
@@ -1577,19 +1736,25 @@ __global__ void __launch_bounds__(SC_THREADS, 4) k_relax_metab(ScParams P, Relax
 // periodic box is decided once per item (Imager), the collision distance per
 // neighbour kind (the lipids' and the metabolic items' radii are each one
 // value in practice, CollisionDistCache recomputes it when they are not).
+#define SC_METAB_GROUP 4
 template <bool BATCH>
-__global__ void __launch_bounds__(SC_THREADS, 4) k_relax_metab_lean(ScParams P, RelaxMArgs A) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;   // list position (count-ordered)
+__global__ void __launch_bounds__(SC_THREADS, 4) k_relax_metab_lean(ScParams P, RelaxMArgs A, int extra) {
+    __shared__ float sTerm[SC_THREADS / 32][32][SC_TERM_ROW];
+    if ((int)blockIdx.x < extra) {
+        if (*A.ovfCount > 0) relax_metab_overflow<BATCH>(P, A, blockIdx.x, extra, sTerm);
+        return;
+    }
+    const int g = ((int)blockIdx.x - extra) * SC_THREADS + threadIdx.x;   // list position (count-ordered)
     if (g >= *A.nActivePtr) return;
     const int i = A.L.perm[g];
     if (i < 0) return;
     if (BATCH) rep_apply<BATCH>(P, A.minfo[i].w);
-    const float4 v4 = A.mvelIn[i];
     const bool act = P.mAllActive ? i < (int)A.cellStartM[P.cells] : (A.minfo[i].z & SC_ACTIVE) != 0;
     if (!act) {
-        A.mvelOut[i] = v4;
+        if (A.age == 0) A.mvelOut[i] = A.mvelIn[i];
         return;
     }
+    const float4 v4 = A.mvelIn[i];
     const int c = A.L.cnt[g];
     if (c > min(SC_LIST_M, P.listLimit)) return;
     const float4 p4 = A.mpos[i];
@@ -1633,168 +1798,11 @@ __global__ void __launch_bounds__(SC_THREADS, 4) k_relax_metab_lean(ScParams P, 
     st3(A.mvelOut, i, pv + dV / fmaxf(w, 1.0f), v4.w);
 }
 
-// An item whose list overflowed: the reference's loops over the 27 cells.
+// The overflowed items in a launch of their own.
 template <bool BATCH>
-__device__ __forceinline__ void relax_metab_scan_item(const ScParams &P0, const RelaxMArgs &A, int i) {
-    if (i < 0) return;
-    const int4 mi = A.minfo[i];
-    if (!(mi.z & SC_ACTIVE)) return;
-    ScParams P = P0;
-    rep_apply<BATCH>(P, mi.w);
-    float4 v4 = A.mvelIn[i];
-    float4 p4 = A.mpos[i];
-    const sc_f3 pp = sc_make_f3(p4.x, p4.y, p4.z);
-    const Imager IM(P, pp, SC_BINNED_M | SC_BINNED_P);
-    const float prad = p4.w;
-    const sc_f3 pv = sc_make_f3(v4.x, v4.y, v4.z);
-    const sc_f3 ppv = pp + pv;
-    sc_f3 dV = sc_zero3();
-    float w = 0.0f;
-    CollisionDistCache cm, cp;
-    const float lim = P.maxInt;
-    cells27(P, pp, reach(P, pp, lim, SC_BINNED_M | SC_BINNED_P), [&](uint32_t key) {
-        for (uint32_t j = A.cellStartM[key], e = A.cellStartM[key + 1]; j < e; j++) {
-            if ((int)j == i) continue;
-            if (!active_m(P, A.minfo, (int)j)) continue;
-            float4 t4 = A.mpos[j];
-            sc_f3 delta = IM(sc_make_f3(t4.x, t4.y, t4.z)) - pp;
-            if (outside_cube(delta, lim)) continue;
-            if (cm.collides(prad, t4.w, delta))
-                metab_pair(IM, pp, ppv, t4, A.mvelIn[j], cm.get(prad, t4.w), false, dV, w);
-        }
-        for (uint32_t j = A.cellStartP[key], e = A.cellStartP[key + 1]; j < e; j++) {
-            if (!active_lipid(P, A.pinfo, (int)j)) continue;
-            float4 t4 = A.ppos[j];
-            sc_f3 delta = IM(sc_make_f3(t4.x, t4.y, t4.z)) - pp;
-            if (outside_cube(delta, lim)) continue;
-            if (cp.collides(prad, t4.w, delta))
-                metab_pair(IM, pp, ppv, t4, A.pvel[j], cp.get(prad, t4.w), true, dV, w);
-        }
-    });
-    st3(A.mvelOut, i, pv + dV / fmaxf(w, 1.0f), v4.w);
-}
-
-// Lists of the overflow pool longer than this are walked by a whole warp,
-// shorter ones by one thread (both in k_relax_metab_pool): a list that
-// overflowed because the main pool had no room for its block fits the list
-// capacity, one that outgrew the capacity (a wall pile's) holds hundreds to
-// thousands of pairs.  With the list capacity capped (pair_list_limit, the
-// tests' way into the overflow paths) the bound is four times the cap, so
-// ordinary lists take both walks.
-#define SC_POOL_WARP_MIN SC_LIST_M
-__device__ __forceinline__ int pool_warp_min(const ScParams &P) {
-    return P.listLimit < SC_POOL_WARP_MIN / 4 ? 4 * P.listLimit : SC_POOL_WARP_MIN;
-}
-
-// The items whose list overflowed (listed by k_build_m), a thread each,
-// grid-stride: an item the overflow pool had no room for scans its
-// neighbourhood; one whose region there is short walks it as k_relax_metab
-// walks the main pool (the same terms in the same order, SC_METAB_GROUP pairs
-// in flight); the long regions are k_relax_metab_pool's.
-template <bool BATCH>
-__global__ void __launch_bounds__(SC_THREADS) k_relax_metab_overflow(ScParams P, RelaxMArgs A,
-                                                                     const int *__restrict__ ovf,
-                                                                     const int *__restrict__ ovfCount,
-                                                                     const int *__restrict__ ovfN,
-                                                                     const long long *__restrict__ ovfOff,
-                                                                     const uint4 *__restrict__ ovfPool) {
-    const int warpMin = pool_warp_min(P);
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < *ovfCount; t += gridDim.x * blockDim.x) {
-        const int i = ovf[t];
-        const long long off = ovfOff ? ovfOff[t] : -1;
-        if (off < 0) {
-            relax_metab_scan_item<BATCH>(P, A, i);
-            continue;
-        }
-        const int n = ovfN[t];
-        if (i < 0 || n > warpMin || !(A.minfo[i].z & SC_ACTIVE)) continue;
-        const float4 v4 = A.mvelIn[i], p4 = A.mpos[i];
-        const sc_f3 pv = sc_make_f3(v4.x, v4.y, v4.z);
-        const sc_f3 ppv = sc_make_f3(p4.x, p4.y, p4.z) + pv;
-        sc_f3 dV = sc_zero3();
-        float w = 0.0f;
-        const uint4 *__restrict__ e = ovfPool + off;
-        uint4 E[SC_METAB_GROUP];
-#pragma unroll
-        for (int q = 0; q < SC_METAB_GROUP; q++) E[q] = q < n ? e[q] : make_uint4(0, 0, 0, 0);
-        for (int k0 = 0; k0 < n; k0 += SC_METAB_GROUP) {
-            float4 tv[SC_METAB_GROUP];
-            uint4 En[SC_METAB_GROUP];
-#pragma unroll
-            for (int q = 0; q < SC_METAB_GROUP; q++)
-                tv[q] = k0 + q < n ? metab_pair_vel(A, E[q].x) : make_float4(0, 0, 0, 0);
-#pragma unroll
-            for (int q = 0; q < SC_METAB_GROUP; q++) {
-                const int k = k0 + SC_METAB_GROUP + q;
-                En[q] = k < n ? e[k] : make_uint4(0, 0, 0, 0);
-            }
-#pragma unroll
-            for (int q = 0; q < SC_METAB_GROUP; q++) {
-                if (k0 + q < n) {
-                    const float kw = (E[q].x & SC_M_FROM_P) ? 2.0f : 1.0f;
-                    const sc_f3 a = sc_make_f3(__uint_as_float(E[q].y), __uint_as_float(E[q].z),
-                                               __uint_as_float(E[q].w));
-                    w += kw;
-                    dV += (a + sc_make_f3(tv[q].x, tv[q].y, tv[q].z) - ppv) * 0.9f * kw;
-                }
-                E[q] = En[q];
-            }
-        }
-        st3(A.mvelOut, i, pv + dV / fmaxf(w, 1.0f), v4.w);
-    }
-}
-
-// The overflowed items whose list is kept whole in the overflow pool
-// (k_build_m_ovf) and is longer than pool_warp_min, a warp each, warp-stride
-// over the items so the long lists of a wall pile spread over the device:
-// the lanes load 32 entries and the neighbours' velocities at once and each
-// forms its pair's term and weight; lanes 0-2 add the terms' components and
-// lane 3 the weights in list order from shared memory -- the sums a thread
-// walking the list forms, at one gather latency per 32 pairs.
-__global__ void __launch_bounds__(SC_THREADS) k_relax_metab_pool(ScParams P, RelaxMArgs A, const int *__restrict__ ovf,
-                                                                 const int *__restrict__ ovfCount,
-                                                                 const int *__restrict__ ovfN,
-                                                                 const long long *__restrict__ ovfOff,
-                                                                 const uint4 *__restrict__ ovfPool) {
-    __shared__ float sTerm[SC_THREADS / 32][32][5];   // x, y, z, weight (odd row length: no bank conflicts)
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int nOvf = *ovfCount;
-    const int warpMin = pool_warp_min(P);
-    for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < nOvf; t += (gridDim.x * blockDim.x) >> 5) {
-        const int i = ovf[t], n = ovfN[t];
-        const long long off = ovfOff[t];
-        if (off < 0 || i < 0 || n <= warpMin || !(A.minfo[i].z & SC_ACTIVE)) continue;   // warp-uniform
-        const float4 v4 = A.mvelIn[i], p4 = A.mpos[i];
-        const sc_f3 pv = sc_make_f3(v4.x, v4.y, v4.z);
-        const sc_f3 ppv = sc_make_f3(p4.x, p4.y, p4.z) + pv;
-        const uint4 *__restrict__ e = ovfPool + off;
-        float acc = 0.0f;   // lanes 0-2: dV's components; lane 3: the weight
-        for (int b = 0; b < n; b += 32) {
-            float term[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            if (b + lane < n) {
-                const uint4 E = e[b + lane];
-                const float4 tv = metab_pair_vel(A, E.x);
-                const float kw = (E.x & SC_M_FROM_P) ? 2.0f : 1.0f;
-                const sc_f3 a = sc_make_f3(__uint_as_float(E.y), __uint_as_float(E.z), __uint_as_float(E.w));
-                const sc_f3 d = (a + sc_make_f3(tv.x, tv.y, tv.z) - ppv) * 0.9f * kw;
-                term[0] = d.x;
-                term[1] = d.y;
-                term[2] = d.z;
-                term[3] = kw;
-            }
-#pragma unroll
-            for (int k = 0; k < 4; k++) sTerm[wid][lane][k] = term[k];
-            __syncwarp();
-            if (lane < 4) {
-                const int m = min(32, n - b);
-                for (int u = 0; u < m; u++) acc += sTerm[wid][u][lane];
-            }
-            __syncwarp();
-        }
-        const float dy = __shfl_sync(0xffffffffu, acc, 1), dz = __shfl_sync(0xffffffffu, acc, 2),
-                    w = __shfl_sync(0xffffffffu, acc, 3);
-        if (lane == 0) st3(A.mvelOut, i, pv + sc_make_f3(acc, dy, dz) / fmaxf(w, 1.0f), v4.w);
-    }
+__global__ void __launch_bounds__(SC_THREADS) k_relax_metab_overflow(ScParams P, RelaxMArgs A) {
+    __shared__ float sTerm[SC_THREADS / 32][32][SC_TERM_ROW];
+    if (*A.ovfCount > 0) relax_metab_overflow<BATCH>(P, A, blockIdx.x, gridDim.x, sTerm);
 }
 
 // ---- the same sweep on column-segment tiles (sc_tile.cuh) ---------------------
@@ -2159,21 +2167,18 @@ __global__ void __launch_bounds__(SC_THREADS) k_relax_partners(
     const float4 *__restrict__ mpos, const int4 *__restrict__ minfo, const float4 *__restrict__ mvel) {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;   // list position (count-ordered)
     if (g >= *nActivePtr) return;
-    const int i = L.perm[g];
+    // the positions are those of active lipids, -1 past them (k_build_lm)
+    const int i = L.perm[g], c = L.cnt[g];
+    const uint4 *pairs = pool + warpOff[g >> 5] + (g & 31);
     if (i < 0) return;
-    int4 in = pinfo[i];
-    if (!(in.z & SC_ACTIVE) || in.y != SC_PARTICLE_TYPE_LIPID) return;
-    rep_apply<BATCH>(P, in.w);
     float4 p4 = ppos_[i];
+    float4 v4 = pvel_[i];
     const sc_f3 pp = sc_make_f3(p4.x, p4.y, p4.z);
     const float prad = p4.w;
-    float4 v4 = pvel_[i];
     const sc_f3 pv = sc_make_f3(v4.x, v4.y, v4.z);
     sc_f3 dV = sc_zero3();
     float w = 0.0f;
-    const int c = L.cnt[g];
     if (c <= min(SC_LIST_LM, P.listLimit)) {
-        const uint4 *pairs = pool + warpOff[g >> 5] + (g & 31);
         for (int k0 = 0; k0 < c; k0 += 4) {
             uint4 E[4];
             float4 tv[4];
@@ -2191,6 +2196,7 @@ __global__ void __launch_bounds__(SC_THREADS) k_relax_partners(
             }
         }
     } else {
+        rep_apply<BATCH>(P, pinfo[i].w);
         const Imager IM(P, pp, SC_BINNED_M);
         CollisionDistCache cc;
         const float lim = P.maxInt;
@@ -2994,7 +3000,7 @@ __global__ void __launch_bounds__(SC_THREADS, 4) k_build_d(ScParams P, const uin
 // The full diffusion lists of the overflowed positions (listed by k_build_d;
 // their counts are in cnt): each takes a contiguous region of the overflow
 // pool by atomicAdd and writes its neighbours there in build_d_item's order,
-// for k_diffuse_pool; a position the pool has no room for keeps offset -1 (it
+// for diffuse_pool; a position the pool has no room for keeps offset -1 (it
 // scans).  The demand is counted in full for the pool's growth at the next
 // synchronisation.
 template <bool BATCH>
@@ -3074,106 +3080,35 @@ __device__ __forceinline__ void diffuse_term(const float4 (&v)[SP / 4], const fl
     }
 }
 
-template <int SP, bool BATCH>
-__global__ void __launch_bounds__(SC_THREADS) k_diffuse(ScParams P, const uint32_t *__restrict__ cellStart,
-                                                        const int *__restrict__ nActivePtr,
-                                                        const float4 *__restrict__ pos, const int4 *__restrict__ info,
-                                                        PairList<SC_LIST_D> L, const float4 *__restrict__ metIn,
-                                                        float4 *__restrict__ metOut, const long long *__restrict__ ovfOff,
-                                                        const uint32_t *__restrict__ ovfPool) {
-    constexpr int Q = SP / 4;
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;   // list position (count-ordered)
-    if (g >= *nActivePtr) return;
-    const int i = L.perm[g];
-    if (i < 0) return;
-    if (BATCH) rep_apply<BATCH>(P, info[i].w);
-    float pm[SP];
-    {
-        float4 v[Q];
-        met_row<Q>(metIn, i, v);
-#pragma unroll
-        for (int q = 0; q < Q; q++) {
-            pm[4 * q] = v[q].x; pm[4 * q + 1] = v[q].y; pm[4 * q + 2] = v[q].z; pm[4 * q + 3] = v[q].w;
-        }
-    }
-    // after the sort the active items are exactly the binned ones
-    const bool act = P.mAllActive ? i < (int)cellStart[P.cells] : (info[i].z & SC_ACTIVE) != 0;
-    if (!act) {
-        met_store<SP>(metOut, i, pm);   // the amounts' bits, unchanged
-        return;
-    }
-    float dm[SP];
-#pragma unroll
-    for (int k = 0; k < SP; k++) dm[k] = 0.0f;
-    const int S = P.S;
-    const int c = L.cnt[g];
-    if (c <= min(SC_LIST_D, P.listLimit)) {
-        // four entries per list load; their amounts are gathered together and
-        // the next chunk of the list is loaded while this one is applied
-        const uint4 *__restrict__ chunks = sc_list4_chunks(L.list, SC_LIST_D, g);
-        uint4 E = c > 0 ? chunks[0] : make_uint4(0, 0, 0, 0);
-        for (int k0 = 0; k0 < c; k0 += 4) {
-            const uint4 En = k0 + 4 < c ? chunks[(size_t)(k0 / 4 + 1) * 32] : make_uint4(0, 0, 0, 0);
-            const int e[4] = {(int)E.x, (int)E.y, (int)E.z, (int)E.w};
-            float4 v[4][Q];
-#pragma unroll
-            for (int kk = 0; kk < 4; kk++)
-                if (k0 + kk < c) met_row<Q>(metIn, e[kk], v[kk]);
-#pragma unroll
-            for (int kk = 0; kk < 4; kk++) {
-                if (k0 + kk >= c) break;
-                diffuse_term<SP>(v[kk], pm, dm, S);
-            }
-            E = En;
-        }
-    } else if (ovfOff && ovfOff[g] >= 0) {
-        return;   // an overflowed list kept whole in the overflow pool: k_diffuse_pool
-    } else {
-        float4 p4 = pos[i];
-        const sc_f3 pp = sc_make_f3(p4.x, p4.y, p4.z);
-        const Imager IM(P, pp, SC_BINNED_M);
-        const float lim = P.maxDiff;
-        const sc_sqrt_le within = sc_sqrt_le_make(lim);
-        scan27(P, cellStart, pp, reach(P, pp, lim, SC_BINNED_M), [&](int j) {
-            if (j == i) return;
-            if (!active_m(P, info, j)) return;
-            float4 t4 = pos[j];
-            sc_f3 delta = IM(sc_make_f3(t4.x, t4.y, t4.z)) - pp;
-            if (outside_cube(delta, lim)) return;
-            if (sc_sqrt_le_test(within, sc_normsq3(delta))) {
-                float4 v[Q];
-                met_row<Q>(metIn, j, v);
-                diffuse_term<SP>(v, pm, dm, S);
-            }
-        });
-    }
-#pragma unroll
-    for (int k = 0; k < SP; k++)
-        if (k < S) pm[k] += dm[k];
-    met_store<SP>(metOut, i, pm);
-}
+// The overflowed diffusion positions (k_build_d), the first entry of each one's
+// region of the overflow pool by position (-1: it scans).
+struct DiffuseOvf {
+    const int *__restrict__ ovf, *__restrict__ count;
+    const long long *__restrict__ off;
+    const uint32_t *__restrict__ pool;
+};
 
 // The positions whose overflowed list is kept whole in the overflow pool
-// (k_build_d_ovf), one warp per position: the lanes gather 32 neighbours'
+// (k_build_d_ovf), one warp per position, by `blocks` blocks of which this is
+// block `blk`: the lanes gather 32 neighbours'
 // amounts at once and each computes its neighbour's terms (zero where the
 // threshold drops the pair; a kept term is never zero), then lane k adds the
 // kept terms of amount k in list order from shared memory -- the sums a
 // thread walking the list forms, term by term, while the list's pile-sized
 // length costs one gather latency per 32 neighbours instead of per 4.
 template <int SP>
-__global__ void __launch_bounds__(SC_THREADS) k_diffuse_pool(ScParams P, const int4 *__restrict__ info,
-                                                             PairList<SC_LIST_D> L, const int *__restrict__ ovf,
-                                                             const int *__restrict__ ovfCount,
-                                                             const long long *__restrict__ ovfOff,
-                                                             const uint32_t *__restrict__ ovfPool,
-                                                             const float4 *__restrict__ metIn,
-                                                             float4 *__restrict__ metOut) {
+__device__ __forceinline__ void diffuse_pool(const ScParams &P, const int4 *__restrict__ info,
+                                             const PairList<SC_LIST_D> &L, const DiffuseOvf &O,
+                                             const float4 *__restrict__ metIn, float4 *__restrict__ metOut, int blk,
+                                             int blocks, float (*sTerm)[32][SP + 1]) {
     constexpr int Q = SP / 4;
-    __shared__ float sTerm[SC_THREADS / 32][32][SP + 1];   // odd row length: no bank conflicts either way
+    const int *__restrict__ ovf = O.ovf;
+    const long long *__restrict__ ovfOff = O.off;
+    const uint32_t *__restrict__ ovfPool = O.pool;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int S = P.S;
-    const int n = *ovfCount;
-    for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < n; t += (gridDim.x * blockDim.x) >> 5) {
+    const int n = *O.count;
+    for (int t = blk * (SC_THREADS / 32) + wid; t < n; t += blocks * (SC_THREADS / 32)) {
         const int g = ovf[t];
         const long long off = ovfOff[g];
         const int i = L.perm[g];
@@ -3229,6 +3164,108 @@ __global__ void __launch_bounds__(SC_THREADS) k_diffuse_pool(ScParams P, const i
         }
         if (lane < SP) reinterpret_cast<float *>(metOut)[(size_t)i * SP + lane] = mine;
     }
+}
+
+template <int SP>
+__global__ void __launch_bounds__(SC_THREADS) k_diffuse_pool(ScParams P, const int4 *__restrict__ info,
+                                                             PairList<SC_LIST_D> L, DiffuseOvf O,
+                                                             const float4 *__restrict__ metIn,
+                                                             float4 *__restrict__ metOut) {
+    __shared__ float sTerm[SC_THREADS / 32][32][SP + 1];
+    if (*O.count > 0) diffuse_pool<SP>(P, info, L, O, metIn, metOut, blockIdx.x, gridDim.x, sTerm);
+}
+
+// With POOL the first `extra` blocks take the positions of the overflow pool
+// (they write other items and read what the others read; the longest lists
+// start first); k_diffuse_pool takes them otherwise: its shared memory in this
+// kernel takes L1 from the gathers that bound it (large workload: 330 -> 361 us
+// a launch), while a sim that does not fill the device saves a launch.
+// Inactive items' amounts are copied until both buffers hold them (age:
+// launches since the amounts were last out of step).
+template <int SP, bool BATCH, bool POOL>
+__global__ void __launch_bounds__(SC_THREADS) k_diffuse(ScParams P, const uint32_t *__restrict__ cellStart,
+                                                        const int *__restrict__ nActivePtr,
+                                                        const float4 *__restrict__ pos, const int4 *__restrict__ info,
+                                                        PairList<SC_LIST_D> L, const float4 *__restrict__ metIn,
+                                                        float4 *__restrict__ metOut, DiffuseOvf O, int extra, int age) {
+    constexpr int Q = SP / 4;
+    if constexpr (POOL) {
+        __shared__ float sTerm[SC_THREADS / 32][32][SP + 1];   // odd row length: no bank conflicts either way
+        if ((int)blockIdx.x < extra) {
+            if (*O.count > 0) diffuse_pool<SP>(P, info, L, O, metIn, metOut, blockIdx.x, extra, sTerm);
+            return;
+        }
+    }
+    const int g = ((int)blockIdx.x - extra) * SC_THREADS + threadIdx.x;   // list position (count-ordered)
+    if (g >= *nActivePtr) return;
+    const int i = L.perm[g];
+    if (i < 0) return;
+    if (BATCH) rep_apply<BATCH>(P, info[i].w);
+    float pm[SP];
+    {
+        float4 v[Q];
+        met_row<Q>(metIn, i, v);
+#pragma unroll
+        for (int q = 0; q < Q; q++) {
+            pm[4 * q] = v[q].x; pm[4 * q + 1] = v[q].y; pm[4 * q + 2] = v[q].z; pm[4 * q + 3] = v[q].w;
+        }
+    }
+    // after the sort the active items are exactly the binned ones
+    const bool act = P.mAllActive ? i < (int)cellStart[P.cells] : (info[i].z & SC_ACTIVE) != 0;
+    if (!act) {
+        if (age > 0) return;
+        met_store<SP>(metOut, i, pm);   // the amounts' bits, unchanged
+        return;
+    }
+    float dm[SP];
+#pragma unroll
+    for (int k = 0; k < SP; k++) dm[k] = 0.0f;
+    const int S = P.S;
+    const int c = L.cnt[g];
+    if (c <= min(SC_LIST_D, P.listLimit)) {
+        const uint4 *__restrict__ chunks = sc_list4_chunks(L.list, SC_LIST_D, g);
+        uint4 E = c > 0 ? chunks[0] : make_uint4(0, 0, 0, 0);
+        // four entries per list load; their amounts are gathered together and
+        // the next chunk of the list is loaded while this one is applied
+        for (int k0 = 0; k0 < c; k0 += 4) {
+            const uint4 En = k0 + 4 < c ? chunks[(size_t)(k0 / 4 + 1) * 32] : make_uint4(0, 0, 0, 0);
+            const int e[4] = {(int)E.x, (int)E.y, (int)E.z, (int)E.w};
+            float4 v[4][Q];
+#pragma unroll
+            for (int kk = 0; kk < 4; kk++)
+                if (k0 + kk < c) met_row<Q>(metIn, e[kk], v[kk]);
+#pragma unroll
+            for (int kk = 0; kk < 4; kk++) {
+                if (k0 + kk >= c) break;
+                diffuse_term<SP>(v[kk], pm, dm, S);
+            }
+            E = En;
+        }
+    } else if (O.off && O.off[g] >= 0) {
+        return;   // an overflowed list kept whole in the overflow pool: diffuse_pool
+    } else {
+        float4 p4 = pos[i];
+        const sc_f3 pp = sc_make_f3(p4.x, p4.y, p4.z);
+        const Imager IM(P, pp, SC_BINNED_M);
+        const float lim = P.maxDiff;
+        const sc_sqrt_le within = sc_sqrt_le_make(lim);
+        scan27(P, cellStart, pp, reach(P, pp, lim, SC_BINNED_M), [&](int j) {
+            if (j == i) return;
+            if (!active_m(P, info, j)) return;
+            float4 t4 = pos[j];
+            sc_f3 delta = IM(sc_make_f3(t4.x, t4.y, t4.z)) - pp;
+            if (outside_cube(delta, lim)) return;
+            if (sc_sqrt_le_test(within, sc_normsq3(delta))) {
+                float4 v[Q];
+                met_row<Q>(metIn, j, v);
+                diffuse_term<SP>(v, pm, dm, S);
+            }
+        });
+    }
+#pragma unroll
+    for (int k = 0; k < SP; k++)
+        if (k < S) pm[k] += dm[k];
+    met_store<SP>(metOut, i, pm);
 }
 
 // ---- metabolites.cuh:18-88 removeInterferingMetabolicParticles -------------
@@ -3481,26 +3518,32 @@ void sc_phase_relax_metab(ScLaunchCtx &c) {
     L.cap = c.P.Nm;
     L.perm = tiles ? nullptr : B.permM;
     RelaxMArgs A{B.cellStartM, B.cellStartP, &B.ctr->nActiveM, M.pos, M.info, L, M.vel, X.vel, F.pos, F.info, F.vel,
-                 reinterpret_cast<const uint4 *>(B.listM), B.warpOffM};
+                 reinterpret_cast<const uint4 *>(B.listM), B.warpOffM, B.ovfM, &B.ctr->ovfM, B.ovfNM,
+                 tiles ? nullptr : B.ovfOffM, B.ovfPoolM, B.relaxMAge};
+    const int nb = nblocks(c.P.Nm);
     if (tiles) {
         k_relax_metab_tile<<<tile_blocks(c.P), SC_THREADS, sc_tile_bytes(c.P.tileCapM, c.P.tileCapP, 32), c.st>>>(
             c.P, A, reinterpret_cast<const uint16_t *>(B.listM), &B.ctr->error);
         k_copy_tail<<<std::max(1, c.gridCap / 8), SC_THREADS, 0, c.st>>>(
             B.cellStartM + c.P.cells, &B.ctr->nActiveM, M.vel, X.vel);
-        (*c.launches) += 2;
+        SC_BATCHED(k_relax_metab_overflow)<<<std::min(nb, c.gridCap / 4), SC_THREADS, 0, c.st>>>(c.P, A);
+        (*c.launches) += 3;
     } else {
-        (c.P.metabLean ? (c.P.nRep > 1 ? k_relax_metab_lean<true> : k_relax_metab_lean<false>) : k_relax_metab)<<<
-            nblocks(c.P.Nm), SC_THREADS, 0, c.st>>>(c.P, A);
+        const bool batch = c.P.nRep > 1, small = nb <= c.gridCap / 4;   // at most two blocks per SM: all resident at G = 8
+        const int extra = small || c.P.metabLean ? std::min(nb, c.gridCap / 2) : 0;
+        if (c.P.metabLean)
+            SC_BATCHED(k_relax_metab_lean)<<<extra + nb, SC_THREADS, 0, c.st>>>(c.P, A, extra);
+        else if (small)
+            (batch ? k_relax_metab<8, true> : k_relax_metab<8, false>)<<<extra + nb, SC_THREADS, 0, c.st>>>(c.P, A, extra);
+        else
+            (batch ? k_relax_metab<4, true> : k_relax_metab<4, false>)<<<nb, SC_THREADS, 0, c.st>>>(c.P, A, 0);
         (*c.launches)++;
+        if (!extra) {
+            SC_BATCHED(k_relax_metab_overflow)<<<std::min(nb, c.gridCap), SC_THREADS, 0, c.st>>>(c.P, A);
+            (*c.launches)++;
+        }
     }
-    SC_BATCHED(k_relax_metab_overflow)<<<std::min(nblocks(c.P.Nm), c.gridCap / 4), SC_THREADS, 0, c.st>>>(
-        c.P, A, B.ovfM, &B.ctr->ovfM, B.ovfNM, tiles ? nullptr : B.ovfOffM, B.ovfPoolM);
-    (*c.launches)++;
-    if (!tiles) {
-        k_relax_metab_pool<<<std::min(nblocks(c.P.Nm), c.gridCap), SC_THREADS, 0, c.st>>>(
-            c.P, A, B.ovfM, &B.ctr->ovfM, B.ovfNM, B.ovfOffM, B.ovfPoolM);
-        (*c.launches)++;
-    }
+    B.relaxMAge = 1;
     B.cm[FM_VEL] ^= 1;
 }
 
@@ -3643,48 +3686,31 @@ void sc_phase_diffuse(ScLaunchCtx &c) {
     L.cnt = B.cntD;
     L.cap = c.P.Nm;
     L.perm = B.permD;
-    // the positions of the overflow pool run beside the others (on a side
-    // stream when there is one): they write other items and read what the
-    // others read
-    const bool fork = c.side[0] != nullptr;
-    cudaStream_t ps = fork ? c.side[0] : c.st;
-    if (fork) {
+    const DiffuseOvf O{B.ovfD, &B.ctr->ovfD, B.ovfOffD, B.ovfPoolD};
+    const int nb = nblocks(c.P.Nm);
+    const bool batch = c.P.nRep > 1, fork = c.side[0] != nullptr;
+    const int extra = fork ? 0 : std::min(nb, c.gridCap / 2);
+    if (fork) {   // beside the others on a side stream
         cudaEventRecord(c.fork, c.st);
-        cudaStreamWaitEvent(ps, c.fork, 0);
+        cudaStreamWaitEvent(c.side[0], c.fork, 0);
+        auto pool = c.P.SP == 4 ? k_diffuse_pool<4> : c.P.SP == 8 ? k_diffuse_pool<8> : k_diffuse_pool<12>;
+        pool<<<std::min(nb, c.gridCap), SC_THREADS, 0, c.side[0]>>>(c.P, M.info, L, O, M.met, X.met);
+        (*c.launches)++;
     }
-    const int pg = std::min(nblocks(c.P.Nm), c.gridCap);
-    switch (c.P.SP) {
-        case 4:
-            k_diffuse_pool<4><<<pg, SC_THREADS, 0, ps>>>(c.P, M.info, L, B.ovfD, &B.ctr->ovfD, B.ovfOffD, B.ovfPoolD,
-                                                         M.met, X.met);
-            break;
-        case 8:
-            k_diffuse_pool<8><<<pg, SC_THREADS, 0, ps>>>(c.P, M.info, L, B.ovfD, &B.ctr->ovfD, B.ovfOffD, B.ovfPoolD,
-                                                         M.met, X.met);
-            break;
-        default:
-            k_diffuse_pool<12><<<pg, SC_THREADS, 0, ps>>>(c.P, M.info, L, B.ovfD, &B.ctr->ovfD, B.ovfOffD,
-                                                          B.ovfPoolD, M.met, X.met);
-    }
-    (*c.launches)++;
-    switch (c.P.SP) {
-        case 4:
-            (c.P.nRep > 1 ? k_diffuse<4, true> : k_diffuse<4, false>)<<<nblocks(c.P.Nm), SC_THREADS, 0, c.st>>>(c.P, B.cellStartM, &B.ctr->nActiveM, M.pos, M.info,
-                                                                   L, M.met, X.met, B.ovfOffD, B.ovfPoolD);
-            break;
-        case 8:
-            (c.P.nRep > 1 ? k_diffuse<8, true> : k_diffuse<8, false>)<<<nblocks(c.P.Nm), SC_THREADS, 0, c.st>>>(c.P, B.cellStartM, &B.ctr->nActiveM, M.pos, M.info,
-                                                                   L, M.met, X.met, B.ovfOffD, B.ovfPoolD);
-            break;
-        default:
-            (c.P.nRep > 1 ? k_diffuse<12, true> : k_diffuse<12, false>)<<<nblocks(c.P.Nm), SC_THREADS, 0, c.st>>>(c.P, B.cellStartM, &B.ctr->nActiveM, M.pos,
-                                                                    M.info, L, M.met, X.met, B.ovfOffD, B.ovfPoolD);
-            break;
-    }
+    auto kern =
+        c.P.SP == 4 ? (fork ? (batch ? k_diffuse<4, true, false> : k_diffuse<4, false, false>)
+                            : (batch ? k_diffuse<4, true, true> : k_diffuse<4, false, true>))
+        : c.P.SP == 8 ? (fork ? (batch ? k_diffuse<8, true, false> : k_diffuse<8, false, false>)
+                              : (batch ? k_diffuse<8, true, true> : k_diffuse<8, false, true>))
+                      : (fork ? (batch ? k_diffuse<12, true, false> : k_diffuse<12, false, false>)
+                              : (batch ? k_diffuse<12, true, true> : k_diffuse<12, false, true>));
+    kern<<<extra + nb, SC_THREADS, 0, c.st>>>(c.P, B.cellStartM, &B.ctr->nActiveM, M.pos, M.info, L, M.met, X.met, O,
+                                              extra, B.diffuseAge);
     if (fork) {
-        cudaEventRecord(c.join[0], ps);
+        cudaEventRecord(c.join[0], c.side[0]);
         cudaStreamWaitEvent(c.st, c.join[0], 0);
     }
+    B.diffuseAge = 1;
     B.cm[FM_MET] ^= 1;
     (*c.launches)++;
 }
