@@ -797,6 +797,96 @@ __device__ __forceinline__ void relax_polar(const ScParams &P0, const RelaxArgs 
     st4(A.avOut, i, pav);
 }
 
+// The same by SC_POLAR_LANES threads per item, for sims that do not fill the
+// device: each thread forms the terms of every SC_POLAR_LANES-th pair, and
+// the group's threads add them all in list order (so each holds the sums).
+// One thread per item was the longest chain of a small sim's launch (the
+// powf, roots and divisions of some eight entries one after another).
+#define SC_POLAR_LANES 4
+template <bool BATCH>
+__device__ __forceinline__ void relax_polar_lanes(const ScParams &P0, const RelaxArgs &A, int i) {
+    const int lane = threadIdx.x & 31, sub = lane & (SC_POLAR_LANES - 1), first = lane & ~(SC_POLAR_LANES - 1);
+    const unsigned group = ((1u << SC_POLAR_LANES) - 1u) << first;
+    const int c = A.L.cnt[i];
+    const float4 v4 = A.velIn[i], r4 = A.rotIn[i], a4 = A.avIn[i], p4 = A.pos[i];
+    uint32_t e = A.L.list[sc_list_at(SC_LIST_PP, i, sub)];
+    if (c > min(SC_LIST_PP, P0.listLimit)) return;   // left to the scan
+    ScParams P = P0;
+    if (BATCH) rep_apply<BATCH>(P, A.info[i].w);
+    const sc_f3 ppos = sc_make_f3(p4.x, p4.y, p4.z);
+    const Imager IM(P, ppos, SC_BINNED_P);
+    const float prad = p4.w;
+    const sc_f3 pvel = sc_make_f3(v4.x, v4.y, v4.z);
+    const sc_f3 ppv = ppos + pvel;
+    const sc_f4 prot = sc_make_f4(r4.x, r4.y, r4.z, r4.w);
+    sc_f4 pav = sc_make_f4(a4.x, a4.y, a4.z, a4.w);
+    sc_f3 dV = sc_zero3();
+    const sc_f4 dAV = sc_qid();
+    sc_f3 phobPos = sc_zero3();
+    float phobSum = 0.0f;
+    float w = 0.0f;
+    const sc_f3 up = sc_rotate(sc_up(), prot);
+    const sc_f3 nextUp = sc_rotate(up, pav);
+    for (int k0 = 0; k0 < c; k0 += SC_POLAR_LANES) {
+        if (k0 > 0) e = k0 + sub < c ? A.L.list[sc_list_at(SC_LIST_PP, i, k0 + sub)] : 0u;
+        const uint32_t fl = k0 + sub < c ? e : 0u;
+        sc_f3 polar = sc_zero3(), pull = sc_zero3(), push = sc_zero3();
+        float pap = 0.0f;
+        if (fl) {
+            const int j = (int)(fl & SC_PP_INDEX);
+            const float4 t4 = A.pos[j], tv = A.velIn[j];
+            if (fl & SC_PP_POLAR) {
+                // dynamics.cuh:478-582: polar (lipid) head / tail attraction
+                const float4 tr = A.rotIn[j];
+                const sc_f3 tpos = IM(sc_make_f3(t4.x, t4.y, t4.z));
+                const float trad = t4.w;
+                const sc_f3 tvel = sc_make_f3(tv.x, tv.y, tv.z);
+                sc_f3 nextTup = sc_rotate(sc_rotate(sc_up(), sc_make_f4(tr.x, tr.y, tr.z, tr.w)), pav);
+                sc_f3 pPV = -nextUp * prad + ppos + pvel;
+                sc_f3 tpPV = -nextTup * trad + tpos + tvel;
+                float Lr = length(tpPV - pPV) / (prad + trad);
+                float attr = sc_polar_attr(Lr);
+                polar = (tpPV - pPV) * 0.05f * attr * 1.0f;
+                pap = sc_powf(fminf(1.0f / fmaxf(Lr, 1e-6f), 10.0f) / 10.0f, 0.2f);
+                pull = tpPV * pap;
+            }
+            if (fl & SC_PP_COLLIDE) push = collide_term(collide_geo(IM, ppos, prad, t4), tv, ppv, prad);
+        }
+        __syncwarp(group);
+#pragma unroll
+        for (int u = 0; u < SC_POLAR_LANES; u++) {
+            const uint32_t f = __shfl_sync(group, fl, first + u);
+            const sc_f3 a = sc_make_f3(__shfl_sync(group, polar.x, first + u), __shfl_sync(group, polar.y, first + u),
+                                       __shfl_sync(group, polar.z, first + u));
+            const sc_f3 b = sc_make_f3(__shfl_sync(group, pull.x, first + u), __shfl_sync(group, pull.y, first + u),
+                                       __shfl_sync(group, pull.z, first + u));
+            const sc_f3 d = sc_make_f3(__shfl_sync(group, push.x, first + u), __shfl_sync(group, push.y, first + u),
+                                       __shfl_sync(group, push.z, first + u));
+            const float q = __shfl_sync(group, pap, first + u);
+            if (f & SC_PP_POLAR) {
+                w += 1.0f;
+                dV += a;
+                phobSum += q;
+                phobPos += b;
+            }
+            if (f & SC_PP_COLLIDE) {
+                w += 1.0f;
+                dV += d;
+            }
+        }
+    }
+    sc_f3 nv = pvel + dV / fmaxf(w, 1.0f);
+    pav = sc_qmul(sc_slerp(sc_qid(), dAV, 1.0f / fmaxf(w, 1.0f)), pav);
+    if (phobSum > 0.0f) {
+        sc_f3 dir = normalize(phobPos / phobSum - (ppos + nv));
+        pav = sc_slerp(pav, sc_quat_from_to(-up, dir), 0.2f);
+    }
+    if (sub) return;
+    st3(A.velOut, i, nv, v4.w);
+    if (A.age == 0) A.rotOut[i] = r4;
+    st4(A.avOut, i, pav);
+}
+
 // The bonded class's items in the order its blocks relax them: each block of
 // SC_BOND_ITEMS ranked by bond-match count, chain-bonded items apart from
 // rule-bonded ones (their pose terms are different code), so that a warp's
@@ -943,9 +1033,14 @@ __device__ __forceinline__ sc_f3 bond_velocity(const ScParams &P, const BondSelf
 // scheduler; two threads per item cut the chain in two, and the record takes
 // two dependent loads out of it.  The class alone, 524,288 + 2,097,152 items
 // (a quarter of the large workload): 37 -> 22 us a launch.
-template <bool BATCH>
+//
+// List entries are loaded two together; with EARLY (sims that do not fill the
+// device) four, the first of them while the bonds' terms are formed, which
+// costs registers the larger sims want.
+template <bool BATCH, bool EARLY>
 __device__ __forceinline__ void relax_bonded_block(const ScParams &P0, const RelaxArgs &A, int base, int n,
                                                    float4 *s_av) {
+    constexpr int G = EARLY ? 4 : 2;
     const bool turner = threadIdx.x < SC_BOND_ITEMS;
     const int slot = turner ? threadIdx.x : threadIdx.x - SC_BOND_ITEMS;
     const int t = base + slot;
@@ -1000,6 +1095,23 @@ __device__ __forceinline__ void relax_bonded_block(const ScParams &P0, const Rel
             else st4(A.avOut, i, pav);
         } else {
             const sc_f3 ppv = S.ppos + S.pvel;
+            auto load = [&](int k0, uint32_t (&e)[G], float4 (&g)[G], float4 (&tv)[G]) {
+                const bool kept = k0 < SC_GEO_PP;
+#pragma unroll
+                for (int q = 0; q < G; q++)
+                    e[q] = k0 + q < c ? A.L.list[sc_list_at(SC_LIST_PP, i, k0 + q)] : 0u;
+#pragma unroll
+                for (int q = 0; q < G; q++) {
+                    g[q] = make_float4(0, 0, 0, 0);
+                    tv[q] = g[q];
+                    if (e[q] & SC_PP_COLLIDE)
+                        g[q] = kept ? A.geo[sc_list_at(SC_GEO_PP, i, k0 + q)] : A.pos[(int)(e[q] & SC_PP_INDEX)];
+                    if (e[q] & (SC_PP_COLLIDE | SC_PP_POLAR)) tv[q] = A.velIn[(int)(e[q] & SC_PP_INDEX)];
+                }
+            };
+            uint32_t e0[G];
+            float4 g0[G], tv0[G];
+            if (EARLY) load(0, e0, g0, tv0);
             // 1. the bonds' velocity terms: the first stays in registers (most
             // bonded items have one), the rest go to a per-thread array
             sc_f3 T0 = sc_zero3(), T[SC_MAX_ACTIVE_INTERACTIONS - 1];
@@ -1028,23 +1140,10 @@ __device__ __forceinline__ void relax_bonded_block(const ScParams &P0, const Rel
             // 2. every velocity term in the reference's order
             sc_f3 dV = sc_zero3(), phobPos = sc_zero3();
             int ut = 0, mi = 0;
-            for (int k0 = 0; k0 < c; k0 += SC_POLAR_GROUP) {
-                uint32_t e[SC_POLAR_GROUP];
-                float4 g[SC_POLAR_GROUP], tv[SC_POLAR_GROUP];
+            auto walk = [&](int k0, const uint32_t (&e)[G], const float4 (&g)[G], const float4 (&tv)[G]) {
                 const bool kept = k0 < SC_GEO_PP;
 #pragma unroll
-                for (int q = 0; q < SC_POLAR_GROUP; q++)
-                    e[q] = k0 + q < c ? A.L.list[sc_list_at(SC_LIST_PP, i, k0 + q)] : 0u;
-#pragma unroll
-                for (int q = 0; q < SC_POLAR_GROUP; q++) {
-                    g[q] = make_float4(0, 0, 0, 0);
-                    tv[q] = g[q];
-                    if (e[q] & SC_PP_COLLIDE)
-                        g[q] = kept ? A.geo[sc_list_at(SC_GEO_PP, i, k0 + q)] : A.pos[(int)(e[q] & SC_PP_INDEX)];
-                    if (e[q] & (SC_PP_COLLIDE | SC_PP_POLAR)) tv[q] = A.velIn[(int)(e[q] & SC_PP_INDEX)];
-                }
-#pragma unroll
-                for (int q = 0; q < SC_POLAR_GROUP; q++) {
+                for (int q = 0; q < G; q++) {
                     const uint32_t fl = e[q];
                     const int j = (int)(fl & SC_PP_INDEX);
                     if (fl & SC_PP_POLAR) {
@@ -1077,6 +1176,17 @@ __device__ __forceinline__ void relax_bonded_block(const ScParams &P0, const Rel
                     }
                     if (fl & SC_PP_COLLIDE)
                         dV += collide_term(kept ? g[q] : collide_geo(IM, S.ppos, S.prad, g[q]), tv[q], ppv, S.prad);
+                }
+            };
+            for (int k0 = 0; k0 < c; k0 += G) {
+                if (EARLY) {
+                    if (k0 > 0) load(k0, e0, g0, tv0);
+                    walk(k0, e0, g0, tv0);
+                } else {
+                    uint32_t e[G];
+                    float4 g[G], tv[G];
+                    load(k0, e, g, tv);
+                    walk(k0, e, g, tv);
                 }
             }
             const sc_f3 nv = S.pvel + dV / fmaxf((float)(r.w >> 16), 1.0f);
@@ -1112,21 +1222,26 @@ __device__ __forceinline__ void relax_bonded_block(const ScParams &P0, const Rel
 // take 27.5 ms with a kernel per class and 30.7 ms with one launch, whose two
 // blocks per SM starve the plain and polar items.
 #define SC_RELAX_ALL 3
+#define SC_RELAX_ALL_LANES 4   // the same with SC_POLAR_LANES threads per polar item
 template <int CLS, bool BATCH>
 __global__ void __launch_bounds__(SC_THREADS, CLS == 1 ? 4 : CLS == 2 ? 5 : 2) k_relax(ScParams P, RelaxArgs A) {
-    __shared__ float4 s_av[CLS == 0 || CLS == SC_RELAX_ALL ? SC_BOND_ITEMS : 1];
-    constexpr bool B0 = CLS == 0 || CLS == SC_RELAX_ALL, B1 = CLS == 1 || CLS == SC_RELAX_ALL,
-                   B2 = CLS == 2 || CLS == SC_RELAX_ALL;
+    constexpr bool ALL = CLS >= SC_RELAX_ALL, B0 = CLS == 0 || ALL, B1 = CLS == 1 || ALL, B2 = CLS == 2 || ALL;
+    __shared__ float4 s_av[B0 ? SC_BOND_ITEMS : 1];
     const int n0 = B0 ? A.classCount[0] : 0, n1 = B1 ? A.classCount[1] : 0, n2 = B2 ? A.classCount[2] : 0,
               nv = B0 ? *A.ovfCount : 0;
-    const int b0 = (n0 + SC_BOND_ITEMS - 1) / SC_BOND_ITEMS, b1 = b0 + (n1 + SC_THREADS - 1) / SC_THREADS,
+    constexpr int PL = CLS == SC_RELAX_ALL_LANES ? SC_POLAR_LANES : 1;   // threads per polar item
+    const int b0 = (n0 + SC_BOND_ITEMS - 1) / SC_BOND_ITEMS, b1 = b0 + (n1 * PL + SC_THREADS - 1) / SC_THREADS,
               b2 = b1 + (n2 + SC_THREADS - 1) / SC_THREADS, b3 = b2 + (nv + SC_THREADS - 1) / SC_THREADS;
     for (int b = blockIdx.x; b < b3; b += gridDim.x) {
         if (B0 && b < b0) {
-            relax_bonded_block<BATCH>(P, A, b * SC_BOND_ITEMS, n0, s_av);
+            relax_bonded_block<BATCH, CLS == SC_RELAX_ALL_LANES>(P, A, b * SC_BOND_ITEMS, n0, s_av);
         } else if (B1 && b < b1) {
             const int t = (b - b0) * SC_THREADS + threadIdx.x;
-            if (t < n1) relax_polar<BATCH>(P, A, A.classIdx[(size_t)A.L.cap + t]);
+            if (PL > 1) {
+                if (t < n1 * PL) relax_polar_lanes<BATCH>(P, A, A.classIdx[(size_t)A.L.cap + t / PL]);
+            } else if (t < n1) {
+                relax_polar<BATCH>(P, A, A.classIdx[(size_t)A.L.cap + t]);
+            }
         } else if (B2 && b < b2) {
             const int t = (b - b1) * SC_THREADS + threadIdx.x;
             if (t < n2) relax_plain<BATCH>(P, A, A.classIdx[2 * (size_t)A.L.cap + t]);
@@ -3446,9 +3561,14 @@ void sc_phase_relax(ScLaunchCtx &c) {
         cudaStreamWaitEvent(c.st, c.join[1], 0);
         (*c.launches) += 2;
     } else {
-        // fewer: one launch
-        (batch ? k_relax<SC_RELAX_ALL, true>
-               : k_relax<SC_RELAX_ALL, false>)<<<std::min(3 * nb + 4, c.gridCap), SC_THREADS, 0, c.st>>>(c.P, A);
+        // fewer: one launch, with more threads per polar item while the
+        // particles take less than a block per SM (milliseconds a step with
+        // and without, at 1 : 2 metabolic items: 4,096 0.86 / 0.95, 32,000
+        // 1.03 / 1.09, 45,000 1.20 / 1.21, 65,536 1.41 / 1.30)
+        const bool lanes = nb <= c.gridCap / (2048 / SC_THREADS);
+        auto kern = lanes ? (batch ? k_relax<SC_RELAX_ALL_LANES, true> : k_relax<SC_RELAX_ALL_LANES, false>)
+                          : (batch ? k_relax<SC_RELAX_ALL, true> : k_relax<SC_RELAX_ALL, false>);
+        kern<<<std::min((2 + (lanes ? SC_POLAR_LANES : 1)) * nb + 4, c.gridCap), SC_THREADS, 0, c.st>>>(c.P, A);
     }
     B.relaxAge = std::min(B.relaxAge + 1, 2);
     B.cp[FP_VEL] ^= 1;
