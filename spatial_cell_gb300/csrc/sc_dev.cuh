@@ -85,17 +85,18 @@ struct ScCounters {
     int polyCreates;  // of those, the ones whose rule creates a monomer
     int polyConflict; // 1: two listed items touch the same particle (k_poly_plan)
     int step;         // the step loop counter (main.cu:347)
-    int tileCounter[4];
+    // what one builder resets lies together, so one memset resets it
+    int tileCounter[4];   // k_onesweep, per pass
+    int farMove;          // a metabolic item moved more than a cell along an axis since its sort
     int ppClassCount[4];  // items per relax work class (k_build_pp); [3]: RelaxArgs::unsettled
-    int ovfPP, ovfM;      // items whose particle / metabolic list overflowed (k_build_pp, k_build_m)
-    int _pad;
-    unsigned long long poolM;   // entries the metabolic list blocks asked of their pool (k_build_m)
-    unsigned long long poolLM;  // the same for the lipid-metabolic lists (k_build_lm)
-    int workCount;              // items in the particle work list (k_complexify_select)
-    int farMove;                // a metabolic item moved more than a cell along an axis since its sort
-    int ovfD;                     // items whose diffusion list overflowed (k_build_d)
-    unsigned long long poolOvfM;  // entries the overflowed metabolic items asked of their pool (k_build_m_ovf)
-    unsigned long long poolOvfD;  // the same for the diffusion lists (k_build_d_ovf)
+    int ovfPP;            // items whose particle list overflowed (k_build_pp)
+    int ovfD;             // items whose diffusion list overflowed (k_build_d)
+    int ovfM;             // items whose metabolic list overflowed (k_build_m)
+    unsigned long long poolOvfD;  // entries the overflowed diffusion lists asked of their pool (k_build_d_ovf)
+    unsigned long long poolM;     // entries the metabolic list blocks asked of their pool (k_build_m)
+    unsigned long long poolOvfM;  // the same for the overflowed metabolic items (k_build_m_ovf)
+    unsigned long long poolLM;    // the same for the lipid-metabolic lists (k_build_lm)
+    int workCount;                // items in the particle work list (k_complexify_select, k_lipid_select)
 };
 
 // Relax work classes: 0 bonded items, 1 items with polar (lipid) pairs and no

@@ -269,7 +269,8 @@ int sc_launch_sort(cudaStream_t st, const float4 *pos, const int4 *info, int n, 
     size_t lbWords = (size_t)tiles * 256;
     cudaMemsetAsync(hist, 0, 4 * 256 * sizeof(uint32_t), st);
     cudaMemsetAsync(lookback, 0, (size_t)passes * lbWords * sizeof(uint32_t), st);
-    cudaMemsetAsync(ctr->tileCounter, 0, sizeof(ctr->tileCounter), st);
+    // the tile counters and farMove behind them
+    cudaMemsetAsync(ctr->tileCounter, 0, sizeof(ctr->tileCounter) + sizeof(ctr->farMove), st);
     int blocks = (n + SC_THREADS - 1) / SC_THREADS;
     if (n > 0) {
         (P.nRep > 1 ? k_sort_keys<true> : k_sort_keys<false>)<<<blocks, SC_THREADS, 0, st>>>(

@@ -56,6 +56,7 @@ struct ScBuffers {
     float4 *geoPP;                // collision geometry of the particle list's first SC_GEO_PP entries
     uint4 *bondRec;               // bonded class: a record per item, in the blocks' ranked order (k_bond_plan)
     int relaxAge;                 // relax launches since rot / angvel were last out of step (RelaxArgs::age)
+    int noiseAge;                 // coordinate_noise launches since the noises were last out of step (0, 1)
     int relaxMAge;                // relax_metab launches since the metabolic velocities were last out of step (0, 1)
     int diffuseAge;               // the same for the amounts
     int *permM, *permLM, *permD;  // count-ordered list position -> item
@@ -85,7 +86,7 @@ struct ScBuffers {
     float4 *comb;                 // candidates of the metabolic list build, cell by cell (k_combine)
     uint8_t *lipidP;              // per sorted particle slot: active lipid (after each particle sort)
     bool validPP, validM, validLM, validD;
-    void invalidateLists() { validPP = validM = validLM = validD = false; relaxAge = relaxMAge = diffuseAge = 0; }
+    void invalidateLists() { validPP = validM = validLM = validD = false; relaxAge = noiseAge = relaxMAge = diffuseAge = 0; }
     // polymerisation list
     // polymerize: the scheduled items in index order, per slot the rank of
     // its new monomer and its previous monomer, per item a claim count, per
@@ -201,6 +202,7 @@ struct ScLaunchCtx {
     ScParams P;
     ScBuffers *B;
     long long *launches;
+    bool mayPolymerize;  // an item may be scheduled to polymerise
     int gridCap;  // blocks of SC_THREADS resident on the whole device (grid-stride kernels)
     // Two more streams for independent kernels of one phase: forked from st
     // at `fork`, joined back into st through join[0..1] before the phase ends

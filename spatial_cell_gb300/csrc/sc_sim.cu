@@ -76,7 +76,8 @@ __global__ void k_gen_metabolic(uint8_t *aos, int nm, float box, int species, fl
 
 // Slots [0, cap) of F (records i < n from aos, the rest empty).  With `bad`,
 // the lowest record index (plus base) whose interaction count is outside
-// 0..8 is recorded there by atomicMin.
+// 0..8 is recorded there by atomicMin, and bad[1] set when a record has a
+// scheduled polymerisation.
 __global__ void k_unpack_particles(const uint8_t *__restrict__ aos, int n, int cap, PFields F, int *bad = nullptr,
                                    int base = 0) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -99,6 +100,7 @@ __global__ void k_unpack_particles(const uint8_t *__restrict__ aos, int n, int c
     F.angnoise[i] = rd4(r, 112);
     int nb = rdi(r, 128);
     if (bad && (nb < 0 || nb > SC_MAX_ACTIVE_INTERACTIONS)) atomicMin(bad, base + i);
+    if (bad && rdi(r, 228) >= 0) bad[1] = 1;
     F.nb[i] = nb;
     for (int k = 0; k < 24; k++) F.bonds[(size_t)i * 24 + k] = k < 3 * min(max(nb, 0), 8) ? rdi(r, 132 + 4 * k) : 0;
     F.spoly[i] = rdi(r, 228);
@@ -221,8 +223,6 @@ __global__ void k_pack_metabolic(uint8_t *__restrict__ aos, const int *nActivePt
     for (int k = 0; k < SC_AOS_NUM_METABOLITES && k < SP; k++) wrf(r, 256 + 4 * k, met[k]);
 }
 
-__global__ void k_after_sort(ScCounters *c) { c->lastActive = c->nActive - 1; }
-
 // The replica of every slot of a batch just loaded: the loaded items are the
 // replicas' items one replica after another (offsets: nRep + 1 prefix
 // sums); slots past them get the replica id nRep, which names no replica.
@@ -241,13 +241,13 @@ __global__ void k_set_reps(int4 *__restrict__ info, int cap, const int *__restri
     info[i] = in;
 }
 // Per sorted particle slot: 1 for an active lipid (the metabolic kernels'
-// candidate test); slots past the active ones are cleared.
-__global__ void k_mark_lipids(const int *__restrict__ nActivePtr, int cap, const int4 *__restrict__ info,
-                              uint8_t *__restrict__ lipid) {
+// candidate test); slots past the active ones are cleared.  Sets lastActive.
+__global__ void k_mark_lipids(ScCounters *c, int cap, const int4 *__restrict__ info, uint8_t *__restrict__ lipid) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) c->lastActive = c->nActive - 1;
     if (i >= cap) return;
     const int4 in = info[i];
-    lipid[i] = (i < *nActivePtr && (in.z & SC_ACTIVE) && in.y == SC_PARTICLE_TYPE_LIPID) ? 1 : 0;
+    lipid[i] = (i < c->nActive && (in.z & SC_ACTIVE) && in.y == SC_PARTICLE_TYPE_LIPID) ? 1 : 0;
 }
 __global__ void k_end_step(ScCounters *c) { c->step++; }
 
@@ -261,6 +261,8 @@ struct sc_sim {
     cudaStream_t copySt = nullptr;          // frame copies to the host
     cudaStream_t side[2] = {nullptr, nullptr};  // concurrent kernels of one phase (ScLaunchCtx)
     cudaEvent_t fork = nullptr, join[2] = {nullptr, nullptr};
+    bool rulesPolymerize = false;           // some rule may schedule a polymerisation
+    bool loadScheduled = false;             // the loaded state held scheduled polymerisations
     bool forkClasses = false;               // run independent kernels of a phase on the side streams
     cudaEvent_t reduced[2] = {nullptr, nullptr}, copied[2] = {nullptr, nullptr};
     int64_t frames = 0;                     // frames enqueued by sc_reduce_frame_async
@@ -370,6 +372,7 @@ ScLaunchCtx ctx(sc_sim *s) {
     c.B = &s->B;
     c.launches = &s->launches;
     c.gridCap = s->gridCap;
+    c.mayPolymerize = s->rulesPolymerize || s->loadScheduled;
     c.side[0] = s->forkClasses ? s->side[0] : nullptr;
     c.side[1] = s->forkClasses ? s->side[1] : nullptr;
     c.fork = s->fork;
@@ -403,9 +406,8 @@ void sort_particles(sc_sim *s) {
     sc_launch_cell_start(s->st, B.keysP[cur], N, s->P.cells, B.cellStartP, &s->launches);
     sc_launch_gather_particles(s->st, B.valsP[cur], N, B.P(), B.Pnext(), &s->launches);
     B.flipAllP();
-    k_after_sort<<<1, 1, 0, s->st>>>(B.ctr);
-    k_mark_lipids<<<nb_of(N), SC_THREADS, 0, s->st>>>(&B.ctr->nActive, N, B.P().info, B.lipidP);
-    s->launches += 2;
+    k_mark_lipids<<<std::max(nb_of(N), 1), SC_THREADS, 0, s->st>>>(B.ctr, N, B.P().info, B.lipidP);
+    s->launches++;
 }
 
 void sort_metabolic(sc_sim *s) {
@@ -414,7 +416,6 @@ void sort_metabolic(sc_sim *s) {
     MFields F = B.M();
     int cur = sc_launch_sort(s->st, F.pos, F.info, Nm, s->P, B.keysM, B.valsM, B.hist, B.lookback, B.ctr, &s->launches);
     B.sortCurM = cur;
-    cudaMemsetAsync(&B.ctr->farMove, 0, sizeof(int), s->st);
     sc_launch_cell_start(s->st, B.keysM[cur], Nm, s->P.cells, B.cellStartM, &s->launches);
     sc_launch_gather_metabolic(s->st, B.valsM[cur], Nm, s->P.SP / 4, B, &s->launches);
 }
@@ -427,6 +428,7 @@ void invalidate_after(ScBuffers &B, int phase) {
     if (phase != SC_PHASE_RELAX && phase != SC_PHASE_RELAX_METAB && phase != SC_PHASE_RELAX_PARTNERS)
         B.relaxAge = B.relaxMAge = 0;
     if (phase != SC_PHASE_DIFFUSE) B.diffuseAge = 0;
+    if (phase != SC_PHASE_COORDINATE_NOISE) B.noiseAge = 0;
     switch (phase) {
         case SC_PHASE_SORT_PARTICLES: B.validPP = B.validM = B.validLM = false; break;
         case SC_PHASE_SORT_METABOLIC: B.validM = B.validLM = B.validD = false; break;
@@ -443,6 +445,8 @@ void invalidate_after(ScBuffers &B, int phase) {
 // set, moving positions unbins both (particles a polymerisation creates are in
 // no cell, so they are never found as neighbours).
 void binned_after(ScParams &P, int phase) {
+    // either sort clears farMove, which movedOnce's reader needs
+    if (phase == SC_PHASE_SORT_PARTICLES && !(P.binned & SC_BINNED_M)) P.movedOnce = 0;
     if (phase == SC_PHASE_SORT_PARTICLES) P.binned |= SC_BINNED_P;
     if (phase == SC_PHASE_SORT_METABOLIC) P.binned |= SC_BINNED_M;
     if (phase == SC_PHASE_APPLY_VELOCITIES) {
@@ -461,7 +465,7 @@ std::vector<int> host_state(const sc_sim *s) {
     v.insert(v.end(), B.cm, B.cm + FM_COUNT);
     v.insert(v.end(), {B.sortCurP, B.sortCurM, (int)B.validPP, (int)B.validM, (int)B.validLM, (int)B.validD,
                        s->P.binned, s->P.mAllActive, s->P.lipidValid, B.mParity, B.relaxAge, s->P.movedOnce, B.relaxMAge,
-                       B.diffuseAge});
+                       B.diffuseAge, B.noiseAge});
     return v;
 }
 void set_host_state(sc_sim *s, const std::vector<int> &v) {
@@ -483,6 +487,7 @@ void set_host_state(sc_sim *s, const std::vector<int> &v) {
     s->P.movedOnce = v[k++];
     B.relaxMAge = v[k++];
     B.diffuseAge = v[k++];
+    B.noiseAge = v[k++];
 }
 
 int run_phase(sc_sim *s, int phase, int arg) {
@@ -836,6 +841,8 @@ static int create_sim(const sc_config *cfg_in, const sc_replica *replicas, int32
         if (id < 0 || seen[(size_t)id]) continue;
         seen[(size_t)id] = 1;
         flat[(size_t)id] = rules[i];
+        // (a transition to an id without a rule reads the zero rule, whose polymerize is 0)
+        if (rules[i].polymerize >= 0 || rules[i].transition_to >= 0) s->rulesPolymerize = true;
         if (!cfg->rule_probabilities) {  // padding in the reference's records
             flat[(size_t)id].use_probability = 0;
             flat[(size_t)id].probability = 0.0f;
@@ -1057,8 +1064,9 @@ int sc_load_state(sc_sim *s, const sc_particle *particles, int32_t n, const sc_m
     for (int k = 0; k < FP_COUNT; k++) B.cp[k] = 0;
     for (int k = 0; k < FM_COUNT; k++) B.cm[k] = 0;
     // mcFlag: [0] a metabolic record differs from the first, [1] the lowest
-    // particle index with an interaction count outside 0..8
-    const int flags0[2] = {0, INT_MAX};
+    // particle index with an interaction count outside 0..8, [2] a particle is
+    // scheduled to polymerise
+    const int flags0[3] = {0, INT_MAX, 0};
     SC_CK(s, cudaMemcpyAsync(B.mcFlag, flags0, sizeof flags0, cudaMemcpyHostToDevice, s->st));
     const uint8_t *hp = reinterpret_cast<const uint8_t *>(particles);
     const int perP = (int)(kStageBytes / sizeof(sc_particle));
@@ -1097,10 +1105,11 @@ int sc_load_state(sc_sim *s, const sc_particle *particles, int32_t n, const sc_m
                 s->staging, 0, Nm - nm, s->P.SP, shift_m(B.m[0], (size_t)nm, Q), mirrors ? B.mcLscs + nm : nullptr,
                 mirrors ? B.mcSpoly + nm : nullptr, mirrors ? B.mcNb + nm : nullptr,
                 mirrors ? B.mcBonds + (size_t)nm * 24 : nullptr, nm);
-        int flags[2] = {0, INT_MAX};
+        int flags[3] = {0, INT_MAX, 0};
         SC_CK(s, cudaMemcpyAsync(flags, B.mcFlag, sizeof flags, cudaMemcpyDeviceToHost, s->st));
         SC_CK(s, cudaStreamSynchronize(s->st));
         if ((rc = check_launch(s))) return rc;
+        s->loadScheduled = flags[2] != 0;
         if (flags[1] != INT_MAX)
             return set_err(s, SC_E_INVALID, "particle " + std::to_string(flags[1]) + " has more than 8 interactions");
         if (mirrors || !flags[0]) {

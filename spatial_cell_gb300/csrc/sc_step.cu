@@ -420,33 +420,27 @@ __device__ __forceinline__ void coordinate_noise_item(
 
 
 // Runs over the bonded work class (items with at least one bond), the new
-// noise of class position t going to pnTmp[t] / anTmp[t]; every other
-// item's noise is unchanged.
+// noise going to the fields' other buffers; every other item's noise is
+// unchanged and copied there by the first launch of a run (age 0), after which
+// both buffers hold it.
 template <bool BATCH>
 __global__ void __launch_bounds__(SC_THREADS) k_coordinate_noise(
-    ScParams P, const uint32_t *__restrict__ cellStart, const int *__restrict__ classIdx,
-    const int *__restrict__ classCount, const float4 *__restrict__ pos, const int4 *__restrict__ info,
-    const int *__restrict__ nb, const int *__restrict__ bonds, PairList<SC_LIST_PP> L,
+    ScParams P, const uint32_t *__restrict__ cellStart, const int *__restrict__ nActivePtr,
+    const int *__restrict__ classIdx, const int *__restrict__ classCount, const float4 *__restrict__ pos,
+    const int4 *__restrict__ info, const int *__restrict__ nb, const int *__restrict__ bonds, PairList<SC_LIST_PP> L,
     const uint32_t *__restrict__ match, const int *__restrict__ matchN, const float4 *__restrict__ pnIn,
-    const float4 *__restrict__ anIn, float4 *__restrict__ pnTmp, float4 *__restrict__ anTmp, float frac) {
-    const int n0 = classCount[0];
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n0; t += gridDim.x * blockDim.x)
-        coordinate_noise_item<BATCH>(P, cellStart, classIdx[t], pos, info, nb, bonds, L, match, matchN, pnIn, anIn,
-                              pnTmp + t, anTmp + t, frac);
-}
-
-// The bonded class's new noise written back in place (after every read of
-// the old values).
-__global__ void __launch_bounds__(SC_THREADS) k_noise_writeback(const int *__restrict__ classIdx,
-                                                                const int *__restrict__ classCount,
-                                                                const float4 *__restrict__ pnTmp,
-                                                                const float4 *__restrict__ anTmp,
-                                                                float4 *__restrict__ pn, float4 *__restrict__ an) {
-    const int n0 = classCount[0];
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n0; t += gridDim.x * blockDim.x) {
+    const float4 *__restrict__ anIn, float4 *__restrict__ pnOut, float4 *__restrict__ anOut, float frac, int age) {
+    const int n0 = classCount[0], first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    for (int t = first; t < n0; t += stride) {
         const int i = classIdx[t];
-        pn[i] = pnTmp[t];
-        an[i] = anTmp[t];
+        coordinate_noise_item<BATCH>(P, cellStart, i, pos, info, nb, bonds, L, match, matchN, pnIn, anIn, pnOut + i,
+                                     anOut + i, frac);
+    }
+    if (age > 0) return;
+    for (int i = first, n = *nActivePtr; i < n; i += stride) {
+        if ((info[i].z & SC_ACTIVE) && nb[i] >= 1) continue;
+        pnOut[i] = pnIn[i];
+        anOut[i] = anIn[i];
     }
 }
 
@@ -3490,8 +3484,7 @@ static void ensure_pp(ScLaunchCtx &c) {
     ScBuffers &B = *c.B;
     if (B.validPP) return;
     PFields F = B.P();
-    cudaMemsetAsync(B.ctr->ppClassCount, 0, sizeof(B.ctr->ppClassCount), c.st);
-    cudaMemsetAsync(&B.ctr->ovfPP, 0, sizeof(int), c.st);
+    cudaMemsetAsync(B.ctr->ppClassCount, 0, sizeof(B.ctr->ppClassCount) + sizeof(B.ctr->ovfPP), c.st);
     SC_BATCHED(k_build_pp)<<<nblocks(c.P.N), SC_THREADS, 0, c.st>>>(c.P, B.cellStartP, &B.ctr->nActive, F.pos, F.info, F.nb,
                                                          F.bonds, B.listPP, B.cntPP, c.P.N, B.classPP,
                                                          B.ctr->ppClassCount, B.ovfPP, &B.ctr->ovfPP, B.matchPP,
@@ -3500,23 +3493,22 @@ static void ensure_pp(ScLaunchCtx &c) {
         c.P, pp_list(c), B.classPP, B.ctr->ppClassCount, F.bonds, B.matchPP, B.matchN, B.bondRec);
     (*c.launches) += 2;
     B.validPP = true;
-    B.relaxAge = 0;
+    B.relaxAge = B.noiseAge = 0;
 }
 
 void sc_phase_coordinate_noise(ScLaunchCtx &c, float frac) {
     ScBuffers &B = *c.B;
     if (c.P.N <= 0) return;
     ensure_pp(c);
-    // the other buffers of the two noise fields hold the bonded class's new
-    // values by class position until they are written back in place
     PFields F = B.P(), X = B.Pnext();
     const int g = std::min(nblocks(c.P.N), c.gridCap);
-    SC_BATCHED(k_coordinate_noise)<<<g, SC_THREADS, 0, c.st>>>(c.P, B.cellStartP, B.classPP, B.ctr->ppClassCount, F.pos, F.info,
-                                                    F.nb, F.bonds, pp_list(c), B.matchPP, B.matchN, F.posnoise,
-                                                    F.angnoise, X.posnoise, X.angnoise, frac);
-    k_noise_writeback<<<g, SC_THREADS, 0, c.st>>>(B.classPP, B.ctr->ppClassCount, X.posnoise, X.angnoise,
-                                                   F.posnoise, F.angnoise);
-    (*c.launches) += 2;
+    SC_BATCHED(k_coordinate_noise)<<<g, SC_THREADS, 0, c.st>>>(
+        c.P, B.cellStartP, &B.ctr->nActive, B.classPP, B.ctr->ppClassCount, F.pos, F.info, F.nb, F.bonds, pp_list(c),
+        B.matchPP, B.matchN, F.posnoise, F.angnoise, X.posnoise, X.angnoise, frac, B.noiseAge);
+    (*c.launches)++;
+    B.noiseAge = 1;
+    B.cp[FP_POSNOISE] ^= 1;
+    B.cp[FP_ANGNOISE] ^= 1;
 }
 
 void sc_phase_apply_noise(ScLaunchCtx &c) {
@@ -3597,12 +3589,12 @@ void sc_phase_build_m(ScLaunchCtx &c) {
         // the diffusion list's buffer is the build scratch (that list is rebuilt after the next move anyway)
         B.validD = false;
         cudaMemsetAsync(&B.ctr->ovfM, 0, sizeof(int), c.st);
+        cudaMemsetAsync(&B.ctr->poolM, 0, sizeof(B.ctr->poolM) + sizeof(B.ctr->poolOvfM), c.st);
         if (tiles) {
             k_build_m_tile<<<tile_blocks(c.P), SC_THREADS, sc_tile_bytes(c.P.tileCapM, c.P.tileCapP, 17), c.st>>>(
                 c.P, B.cellStartM, B.cellStartP, M.pos, M.info, F.pos, F.info, reinterpret_cast<uint16_t *>(B.listM),
                 B.cntM, B.ovfM, &B.ctr->ovfM);
         } else {
-            cudaMemsetAsync(&B.ctr->poolM, 0, sizeof(B.ctr->poolM), c.st);
             const CombStart cs{B.cellStartM, B.cellStartP};
             k_combine<<<(int)std::min<long long>(((long long)c.P.N + c.P.Nm + SC_THREADS - 1) / SC_THREADS, 8 * c.gridCap),
                         SC_THREADS, 0, c.st>>>(c.P, B.keysM[B.sortCurM], B.keysP[B.sortCurP], cs, M.pos, M.info, F.pos,
@@ -3614,7 +3606,6 @@ void sc_phase_build_m(ScLaunchCtx &c) {
                 c.P, cs, B.comb, &B.ctr->nActiveM, M.pos, M.info, F.pos, B.listM, (long long)B.poolCapM, &B.ctr->poolM, B.warpOffM, B.listD, B.cntM, B.permM, c.P.Nm, B.ovfM, &B.ctr->ovfM,
                 B.ovfNM);
             // the overflowed items' full lists
-            cudaMemsetAsync(&B.ctr->poolOvfM, 0, sizeof(B.ctr->poolOvfM), c.st);
             SC_BATCHED(k_build_m_ovf)<<<std::min(nblocks(c.P.Nm), c.gridCap / 4), SC_THREADS, 0, c.st>>>(
                 c.P, B.cellStartM, B.cellStartP, M.pos, M.info, F.pos, F.info, B.ovfM, &B.ctr->ovfM, B.ovfNM,
                 B.ovfOffM, B.ovfPoolM, (long long)B.ovfPoolCapM, &B.ctr->poolOvfM);
@@ -3675,8 +3666,7 @@ void sc_phase_build_lm(ScLaunchCtx &c) {
     PFields F = B.P();
     if (!B.validLM) {
         if (B.scratchLM == B.listD) B.validD = false;
-        cudaMemsetAsync(&B.ctr->poolLM, 0, sizeof(B.ctr->poolLM), c.st);
-        cudaMemsetAsync(&B.ctr->workCount, 0, sizeof(int), c.st);
+        cudaMemsetAsync(&B.ctr->poolLM, 0, sizeof(B.ctr->poolLM) + sizeof(B.ctr->workCount), c.st);
         k_lipid_select<<<nblocks(c.P.N), SC_THREADS, 0, c.st>>>(&B.ctr->nActive, F.info, B.workP, &B.ctr->workCount);
         SC_BATCHED(k_build_lm)<<<nblocks(c.P.N), SC_THREADS, 0, c.st>>>(
             c.P, B.cellStartM, B.workP, &B.ctr->workCount, F.info, F.pos, M.pos, M.info,
@@ -3760,7 +3750,7 @@ void sc_phase_transition(ScLaunchCtx &c) {
 
 void sc_phase_polymerize(ScLaunchCtx &c) {
     ScBuffers &B = *c.B;
-    if (c.P.N <= 0) return;
+    if (c.P.N <= 0 || !c.mayPolymerize) return;
     PFields F = B.P();
     const int nb = nblocks(c.P.N);
     k_poly_count<<<nb, SC_THREADS, 0, c.st>>>(c.P, F, B.ctr, B.polyBlk);
@@ -3791,10 +3781,10 @@ void sc_phase_diffuse(ScLaunchCtx &c) {
     if (!B.validD) {
         // the build scratch follows the list in the same buffer
         cudaMemsetAsync(&B.ctr->ovfD, 0, sizeof(int), c.st);
+        cudaMemsetAsync(&B.ctr->poolOvfD, 0, sizeof(B.ctr->poolOvfD), c.st);
         SC_BATCHED(k_build_d)<<<nblocks(c.P.Nm), SC_THREADS, 0, c.st>>>(c.P, B.cellStartM, &B.ctr->nActiveM, M.pos, M.info,
                                                              B.listD, B.listD + sc_list_words(SC_LIST_D, c.P.Nm),
                                                              B.cntD, B.permD, c.P.Nm, B.ovfD, &B.ctr->ovfD);
-        cudaMemsetAsync(&B.ctr->poolOvfD, 0, sizeof(B.ctr->poolOvfD), c.st);
         SC_BATCHED(k_build_d_ovf)<<<std::min(nblocks(c.P.Nm), c.gridCap / 4), SC_THREADS, 0, c.st>>>(
             c.P, B.cellStartM, M.pos, M.info, B.ovfD, &B.ctr->ovfD, B.cntD, B.permD, B.ovfOffD, B.ovfPoolD,
             (long long)B.ovfPoolCapD, &B.ctr->poolOvfD);
