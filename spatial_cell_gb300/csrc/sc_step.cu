@@ -2521,63 +2521,95 @@ __device__ __forceinline__ unsigned long long claim_key(sc_f3 delta, int i) {
     return ((unsigned long long)sc_f2u(sc_normsq3(delta)) << 32) | (unsigned)i;
 }
 
-// Whether some rule of a type (partner-mapped rules [cs, ce)) can bond it to
-// type b at all: the part of claim_rule that needs no more of the candidate.
-__device__ __forceinline__ bool claim_types(const ScParams &P, int type, int cs, int ce, int b) {
-    for (int k = cs; k < ce; k++) {
+// Whether some rule of item a's type can bond it to an item of type b with
+// the bonds bb[0, nbb): the part of claim_rule that needs no more of it.
+__device__ __forceinline__ bool claim_open(const ScParams &P, const ClaimItem &a, int b, int nbb,
+                                           const int *__restrict__ bb) {
+    for (int k = a.cs; k < a.ce; k++) {
         const sc_rule &pii = P.prules[k];
-        if (((type == pii.first_partner_type && b == pii.second_partner_type) ||
-             (type == pii.second_partner_type && b == pii.first_partner_type)) &&
-            !pii.only_via_transition)
-            return true;
+        if (!((a.type == pii.first_partner_type && b == pii.second_partner_type) ||
+              (a.type == pii.second_partner_type && b == pii.first_partner_type)) ||
+            pii.only_via_transition)
+            continue;
+        if (pii.group >= 0 && (group_active_in(a.b, a.nb, pii.group) || group_active_in(bb, nbb, pii.group))) continue;
+        return true;
     }
     return false;
 }
 
-// A warp per open item, a lane per neighbour cell: offers are taken by
-// atomicMin, so their order is free.  With a thread per item 6 of a warp's 32
-// lanes were busy and an item's 27 cells were one chain of dependent loads;
-// and a candidate's records are only read once its type has a rule (10 % of
-// the candidates in the cube at the measured mix).  A quarter of the large
-// workload: 174 -> 126 us; a step of 4,096 + 8,192 items is 0.13 ms shorter.
+// Three open items per warp, a lane per column of an item's neighbourhood:
+// offers are taken by atomicMin, so their order is free.  With a thread per
+// item 6 of a warp's 32 lanes were busy and an item's 27 cells were one chain
+// of dependent loads; a lane's column takes its candidates' positions four at
+// a time, and a candidate's records are only read once its type and bonds
+// leave a rule open (under 10 % of the candidates in the cube at the measured
+// mix).  A batch of 24 replicas (0.9 M particles): 290 us a step with a warp per
+// item and a lane per cell, 117 us so; the large workload's third step 637 and
+// 275 us (477 us with the four candidates' tests unrolled, at 115 registers).
 template <bool BATCH>
-__global__ void __launch_bounds__(SC_THREADS) k_claim_offer(
-    ScParams P, const uint32_t *__restrict__ cellStart, const int *__restrict__ work, const int *__restrict__ workCount,
+__global__ void __launch_bounds__(SC_THREADS, 4) k_claim_offer(
+    ScParams P0, const uint32_t *__restrict__ cellStart, const int *__restrict__ work, const int *__restrict__ workCount,
     const float4 *__restrict__ pos, const float4 *__restrict__ rot, const int4 *__restrict__ info,
     const int *__restrict__ state, const int *__restrict__ nbIn, const int *__restrict__ bonds,
     const int *__restrict__ stepPtr, int prep, unsigned long long *claim) {
   const int step = prep ? -1 : *stepPtr;
-  const int lane = threadIdx.x & 31;
-  const int ox = lane / 9 - 1, oy = lane / 3 % 3 - 1, oz = lane % 3 - 1;
-  const int n = *workCount;
-  for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < n; t += (gridDim.x * blockDim.x) >> 5) {
+  const int lane = threadIdx.x & 31, col = lane % 9;
+  const int ox = col / 3 - 1, oy = col % 3 - 1;
+  const int n = lane < 27 ? *workCount : 0;
+  const int stride = ((gridDim.x * blockDim.x) >> 5) * 3;
+  for (int t = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 3 + lane / 9; t < n; t += stride) {
     const int i = work[t];
-    rep_apply<BATCH>(P, info[i].w);
+    ScParams P = P0;
+    if (BATCH) rep_apply<BATCH>(P, info[i].w);
     const ClaimItem a = claim_item(P, pos, rot, info, state, nbIn, bonds, i);
-    if (a.nb >= SC_MAX_ACTIVE_INTERACTIONS || lane >= 27) continue;
     const float lim = P.maxInt;
     const Reach R = reach(P, a.pos, lim, SC_BINNED_P);
-    if (ox < R.xl || ox > R.xh || oy < R.yl || oy > R.yh || oz < R.zl || oz > R.zh) continue;
+    if (a.nb >= SC_MAX_ACTIVE_INTERACTIONS || ox < R.xl || ox > R.xh || oy < R.yl || oy > R.yh) continue;
     const int g = cell_limit(P);
-    int gx = (int)sc_grid_idx(a.pos.x, P.cell, g) + ox, gy = (int)sc_grid_idx(a.pos.y, P.cell, g) + oy,
-        gz = (int)sc_grid_idx(a.pos.z, P.cell, g) + oz;
+    int gx = (int)sc_grid_idx(a.pos.x, P.cell, g) + ox, gy = (int)sc_grid_idx(a.pos.y, P.cell, g) + oy;
+    const int cz = (int)sc_grid_idx(a.pos.z, P.cell, g);
+    // the column's z run, in two parts where a periodic one crosses the face
+    int z0 = cz + R.zl, z1 = cz + R.zh, y0 = 0, y1 = -1;
     if (P.periodic) {
         gx = (int)wrap_cell(gx, g);
         gy = (int)wrap_cell(gy, g);
-        gz = (int)wrap_cell(gz, g);
-    } else if (min(gx, min(gy, gz)) < 0 || max(gx, max(gy, gz)) >= g) {
-        continue;
+        if (z0 < 0) {
+            y0 = y1 = g - 1;
+            z0 = 0;
+        } else if (z1 >= g) {
+            y0 = y1 = 0;
+            z1 = g - 1;
+        }
+    } else {
+        if (min(gx, gy) < 0 || max(gx, gy) >= g) continue;
+        z0 = max(z0, 0);
+        z1 = min(z1, g - 1);
     }
     const Imager IM(P, a.pos, SC_BINNED_P);
-    const uint32_t key = cell_key(P, (uint32_t)gx, (uint32_t)gy, (uint32_t)gz);
-    for (int j = (int)cellStart[key], e = (int)cellStart[key + 1]; j < e; j++) {
-        const float4 t4 = pos[j];
-        const int4 in = info[j];
-        if (j == i) continue;
-        const sc_f3 delta = IM(sc_make_f3(t4.x, t4.y, t4.z)) - a.pos;
-        if (outside_cube(delta, lim) || !(in.z & SC_ACTIVE) || !claim_types(P, a.type, a.cs, a.ce, in.y)) continue;
-        const ClaimItem b = claim_item(P, pos, rot, info, state, nbIn, bonds, j);
-        if (claim_rule(P, a, b, delta, step) >= 0) atomicMin(&claim[j], claim_key(delta, i));
+    const uint32_t key = cell_key(P, (uint32_t)gx, (uint32_t)gy, 0);
+    for (int part = 0; part < 2; part++) {
+        if (part && y1 < y0) break;
+        const int e = (int)cellStart[key + (uint32_t)(part ? y1 : z1) + 1u];
+        for (int j0 = (int)cellStart[key + (uint32_t)(part ? y0 : z0)]; j0 < e; j0 += 4) {
+            uint32_t near = 0;   // of the next four (reading up to three past the run: SC_CAND_PAD)
+            float4 t4[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) t4[u] = pos[j0 + u];
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (j0 + u < e && j0 + u != i &&
+                    !outside_cube(IM(sc_make_f3(t4[u].x, t4[u].y, t4[u].z)) - a.pos, lim))
+                    near |= 1u << u;
+            while (near) {
+                const int j = j0 + __ffs((int)near) - 1;
+                near &= near - 1u;
+                const int4 in = info[j];
+                if (!(in.z & SC_ACTIVE) || !claim_open(P, a, in.y, nbIn[j], bonds + (size_t)j * 24)) continue;
+                const ClaimItem b = claim_item(P, pos, rot, info, state, nbIn, bonds, j);
+                const sc_f3 delta = IM(b.pos) - a.pos;
+                if (claim_rule(P, a, b, delta, step) >= 0) atomicMin(&claim[j], claim_key(delta, i));
+            }
+        }
     }
   }
 }
@@ -3726,7 +3758,7 @@ void sc_phase_complexify(ScLaunchCtx &c, bool prep) {
         (*c.launches) += 2;
     } else {
         cudaMemsetAsync(B.claimP, 0xff, (size_t)c.P.N * sizeof(unsigned long long), c.st);
-        SC_BATCHED(k_claim_offer)<<<std::min(nblocks(c.P.N) * 8, 4 * c.gridCap), SC_THREADS, 0, c.st>>>(c.P, B.cellStartP, B.workP, &B.ctr->workCount, F.pos, F.rot,
+        SC_BATCHED(k_claim_offer)<<<std::min(nblocks(c.P.N) * 11, 4 * c.gridCap), SC_THREADS, 0, c.st>>>(c.P, B.cellStartP, B.workP, &B.ctr->workCount, F.pos, F.rot,
                                                        F.info, F.state, F.nb, F.bonds, &B.ctr->step, prep, B.claimP);
         SC_BATCHED(k_claim_bind)<<<blocks, SC_THREADS, 0, c.st>>>(c.P, B.workP, &B.ctr->workCount, F.pos, F.rot, F.info, F.state,
                                                       F.nb, X.nb, F.bonds, &B.ctr->step, prep, B.claimP);
