@@ -881,8 +881,8 @@ __device__ __forceinline__ void relax_polar_lanes(const ScParams &P0, const Rela
     st4(A.avOut, i, pav);
 }
 
-// The bonded class's items in the order its blocks relax them: each block of
-// SC_BOND_ITEMS ranked by bond-match count, chain-bonded items apart from
+// The bonded class's items in the order they are relaxed: each block of
+// SC_THREADS ranked by bond-match count, chain-bonded items apart from
 // rule-bonded ones (their pose terms are different code), so that a warp's
 // lanes walk about as many bond terms of the same kind, with what an item's
 // first loads depend on beside its index:
@@ -891,7 +891,6 @@ __device__ __forceinline__ void relax_polar_lanes(const ScParams &P0, const Rela
 //   z  that bond's interaction type
 //   w  match count (bits 0-3) | first bond forward (4) | has polar pairs (5) |
 //      list count (8-15) | terms in all (16-31)
-#define SC_BOND_ITEMS (SC_THREADS / 2)
 __global__ void __launch_bounds__(SC_THREADS) k_bond_plan(ScParams P, PairList<SC_LIST_PP> L,
                                                           const int *__restrict__ classIdx,
                                                           const int *__restrict__ classCount,
@@ -1011,11 +1010,10 @@ __device__ __forceinline__ sc_f3 bond_velocity(const ScParams &P, const BondSelf
     return (pDV - (pDV + tpDV) / 2.0f) * 0.9f * prad / (prad + trad) * 1.0f;
 }
 
-// A block of bonded particles (work class 0): SC_BOND_ITEMS items, each
-// relaxed by two threads in different warps.  Only bond terms turn dAV, and
-// the velocity needs none of it, so the block's first half of threads carries
-// the orientation -- the slerp targets of the item's bond matches and dAV's
-// chain over them -- and the second half the velocity: the matches' velocity
+// A block of bonded particles (work class 0), each relaxed by two threads in
+// different warps.  Only bond terms turn dAV, and the velocity needs none of
+// it, so one warp of a pair carries the orientation -- the slerp targets of the
+// items' bond matches and dAV's chain over them -- and the other the velocity: the matches' velocity
 // terms, then the list walked once to add every term in the reference's order
 // (a test bond rotates the particle itself, which later terms read: such
 // particles take the in-order scan).  The divisor of dAV's last slerp is a
@@ -1031,13 +1029,21 @@ __device__ __forceinline__ sc_f3 bond_velocity(const ScParams &P, const BondSelf
 // List entries are loaded two together; with EARLY (sims that do not fill the
 // device) four, the first of them while the bonds' terms are formed, which
 // costs registers the larger sims want.
-template <bool BATCH, bool EARLY>
-__device__ __forceinline__ void relax_bonded_block(const ScParams &P0, const RelaxArgs &A, int base, int n,
+template <bool BATCH, bool EARLY, int T>
+__device__ __forceinline__ void relax_bonded_block(const ScParams &P0, const RelaxArgs &A, int b, int n,
                                                    float4 *s_av) {
     constexpr int G = EARLY ? 4 : 2;
-    const bool turner = threadIdx.x < SC_BOND_ITEMS;
-    const int slot = turner ? threadIdx.x : threadIdx.x - SC_BOND_ITEMS;
-    const int t = base + slot;
+    // warps in pairs: one turns, the other moves the pair's 32 items (the
+    // first half of a block's warps turns, so its schedulers hold both kinds)
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, pair = warp % (T / 64);
+    const bool turner = warp < T / 64;
+    const int slot = pair * 32 + lane;
+    // The plan ranks every 256 items by their bonds, so its 32-item groups
+    // come as eight weights: one-pair blocks take all the heaviest groups
+    // first, and no launch ends on one (vesicle at 1/16: 134 us a launch in
+    // plan order, 114 us so).
+    const int ranked = (n + SC_THREADS - 1) / SC_THREADS;
+    const int t = T == 64 ? (b % ranked * 8 + b / ranked) * 32 + lane : b * (T / 2) + slot;
     const uint4 r = t < n ? A.bondRec[t] : make_uint4(0xffffffffu, 0, 0, 0);
     const int i = (int)r.x;
     const bool polar = (r.w >> 5) & 1u;
@@ -1108,7 +1114,7 @@ __device__ __forceinline__ void relax_bonded_block(const ScParams &P0, const Rel
             if (EARLY) load(0, e0, g0, tv0);
             // 1. the bonds' velocity terms: the first stays in registers (most
             // bonded items have one), the rest go to a per-thread array
-            sc_f3 T0 = sc_zero3(), T[SC_MAX_ACTIVE_INTERACTIONS - 1];
+            sc_f3 V0 = sc_zero3(), V[SC_MAX_ACTIVE_INTERACTIONS - 1];
             sc_f4 pdbg = sc_make_f4(0, 0, 0, 0);
             bool dbgTouched = false;
             int nt = 0;
@@ -1126,8 +1132,8 @@ __device__ __forceinline__ void relax_bonded_block(const ScParams &P0, const Rel
                     pdbg.y = (float)((double)pdbg.y + (double)dd.y * (1.0 - (double)0.9f));
                     pdbg.z = (float)((double)pdbg.z + (double)dd.z * (1.0 - (double)0.9f));
                 }
-                if (nt == 0) T0 = dv;
-                else T[nt - 1] = dv;
+                if (nt == 0) V0 = dv;
+                else V[nt - 1] = dv;
                 nt++;
             }
             if (dbgTouched) st4(A.dbg, i, pdbg);
@@ -1163,7 +1169,7 @@ __device__ __forceinline__ void relax_bonded_block(const ScParams &P0, const Rel
                             if ((int)(me & SC_PP_INDEX) != j) break;
                             const int it = mi == 0 ? (int)r.z : myBonds[3 * (int)(me >> 29)];
                             if (bond_turns(it)) {
-                                dV += ut == 0 ? T0 : T[ut - 1];
+                                dV += ut == 0 ? V0 : V[ut - 1];
                                 ut++;
                             }
                         }
@@ -1217,30 +1223,41 @@ __device__ __forceinline__ void relax_bonded_block(const ScParams &P0, const Rel
 // blocks per SM starve the plain and polar items.
 #define SC_RELAX_ALL 3
 #define SC_RELAX_ALL_LANES 4   // the same with SC_POLAR_LANES threads per polar item
+//
+// The bonded kernel's blocks are one pair of warps: an item's time goes with
+// its bonds (a lattice complex's particles hold up to seven), and in blocks of
+// four pairs the others' registers waited for the longest (vesicle at 1/16:
+// 141 us a launch so, 134 us in pairs).  Ten pairs, three and four blocks per SM:
+// batch of 24 replicas, two steps 11.3 ms at 2 / 4 / 5 blocks of 256, 11.0 ms
+// so; sub-iteration of the large workload 170 us at 3 / 3 / 3, 181 us at
+// 2 / 5 / 6.
+__host__ __device__ constexpr int relax_threads(int cls) { return cls == 0 ? 64 : SC_THREADS; }
 template <int CLS, bool BATCH>
-__global__ void __launch_bounds__(SC_THREADS, CLS == 1 ? 4 : CLS == 2 ? 5 : 2) k_relax(ScParams P, RelaxArgs A) {
+__global__ void __launch_bounds__(relax_threads(CLS), CLS == 0 ? 10 : CLS == 1 ? 3 : CLS == 2 ? 4 : 2)
+    k_relax(ScParams P, RelaxArgs A) {
     constexpr bool ALL = CLS >= SC_RELAX_ALL, B0 = CLS == 0 || ALL, B1 = CLS == 1 || ALL, B2 = CLS == 2 || ALL;
-    __shared__ float4 s_av[B0 ? SC_BOND_ITEMS : 1];
+    constexpr int T = relax_threads(CLS);
+    __shared__ float4 s_av[B0 ? T / 2 : 1];
     const int n0 = B0 ? A.classCount[0] : 0, n1 = B1 ? A.classCount[1] : 0, n2 = B2 ? A.classCount[2] : 0,
               nv = B0 ? *A.ovfCount : 0;
     constexpr int PL = CLS == SC_RELAX_ALL_LANES ? SC_POLAR_LANES : 1;   // threads per polar item
-    const int b0 = (n0 + SC_BOND_ITEMS - 1) / SC_BOND_ITEMS, b1 = b0 + (n1 * PL + SC_THREADS - 1) / SC_THREADS,
-              b2 = b1 + (n2 + SC_THREADS - 1) / SC_THREADS, b3 = b2 + (nv + SC_THREADS - 1) / SC_THREADS;
+    const int b0 = T == 64 ? (n0 + SC_THREADS - 1) / SC_THREADS * 8 : (n0 + T / 2 - 1) / (T / 2), b1 = b0 + (n1 * PL + T - 1) / T, b2 = b1 + (n2 + T - 1) / T,
+              b3 = b2 + (nv + T - 1) / T;
     for (int b = blockIdx.x; b < b3; b += gridDim.x) {
         if (B0 && b < b0) {
-            relax_bonded_block<BATCH, CLS == SC_RELAX_ALL_LANES>(P, A, b * SC_BOND_ITEMS, n0, s_av);
+            relax_bonded_block<BATCH, CLS == SC_RELAX_ALL_LANES, T>(P, A, b, n0, s_av);
         } else if (B1 && b < b1) {
-            const int t = (b - b0) * SC_THREADS + threadIdx.x;
+            const int t = (b - b0) * T + threadIdx.x;
             if (PL > 1) {
                 if (t < n1 * PL) relax_polar_lanes<BATCH>(P, A, A.classIdx[(size_t)A.L.cap + t / PL]);
             } else if (t < n1) {
                 relax_polar<BATCH>(P, A, A.classIdx[(size_t)A.L.cap + t]);
             }
         } else if (B2 && b < b2) {
-            const int t = (b - b1) * SC_THREADS + threadIdx.x;
+            const int t = (b - b1) * T + threadIdx.x;
             if (t < n2) relax_plain<BATCH>(P, A, A.classIdx[2 * (size_t)A.L.cap + t]);
         } else if (B0) {
-            const int t = (b - b2) * SC_THREADS + threadIdx.x;
+            const int t = (b - b2) * T + threadIdx.x;
             if (t < nv) {
                 const int i = A.ovf[t];
                 const int4 in = A.info[i];
@@ -3576,7 +3593,8 @@ void sc_phase_relax(ScLaunchCtx &c) {
         cudaStreamWaitEvent(c.side[0], c.fork, 0);
         cudaStreamWaitEvent(c.side[1], c.fork, 0);
         const int g = std::min(nb, c.gridCap);
-        (batch ? k_relax<0, true> : k_relax<0, false>)<<<std::min(3 * nb + 1, c.gridCap), SC_THREADS, 0, c.st>>>(c.P, A);
+        (batch ? k_relax<0, true> : k_relax<0, false>)<<<std::min(12 * nb, 6 * c.gridCap), relax_threads(0), 0,
+                                                         c.st>>>(c.P, A);
         (batch ? k_relax<2, true> : k_relax<2, false>)<<<g, SC_THREADS, 0, c.side[0]>>>(c.P, A);
         (batch ? k_relax<1, true> : k_relax<1, false>)<<<g, SC_THREADS, 0, c.side[1]>>>(c.P, A);
         cudaEventRecord(c.join[0], c.side[0]);
