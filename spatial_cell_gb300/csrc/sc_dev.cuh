@@ -83,7 +83,7 @@ struct ScCounters {
     int error;        // first device-side error code
     int polyCount;    // scheduled polymerisations listed this step (k_poly_offsets)
     int polyCreates;  // of those, the ones whose rule creates a monomer
-    int polyConflict; // 1: two listed items touch the same particle (k_poly_plan)
+    int polyConflict; // 1: an item holds two bonds of its rule's group (k_poly_plan)
     int step;         // the step loop counter (main.cu:347)
     // what one builder resets lies together, so one memset resets it
     int tileCounter[4];   // k_onesweep, per pass

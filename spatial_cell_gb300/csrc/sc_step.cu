@@ -469,9 +469,9 @@ struct RelaxArgs {
     int age;
 };
 
-// The relaxation of a particle whose list overflowed or that holds a test
-// bond: its 27 cells are visited and the list's tests applied to each
-// candidate.  The bond loop reads the particle's bonds from memory one at a
+// The relaxation of a particle that holds a test bond, pair by pair, or whose
+// list overflowed: then its 27 cells are visited and the list's tests applied
+// to each candidate.  The bond loop reads the particle's bonds from memory one at a
 // time, so its body is emitted once; out of line, so that the lists' code
 // does not carry its registers.
 __device__ __noinline__ void relax_scan_item(const ScParams &P, const RelaxArgs &A, int i, int4 in, float4 v4, float4 r4,
@@ -599,12 +599,22 @@ __device__ __noinline__ void relax_scan_item(const ScParams &P, const RelaxArgs 
             dV += (tpos - nd * cd + tvel - (ppos + pvel)) * 0.9f * trad / (prad + trad) * 1.0f;
         }
     };
-    BondRegs B;
-    B.load(A.nb, A.bonds, i);
-    scan27(P, A.cellStart, ppos, reach(P, ppos, P.maxInt, SC_BINNED_P), [&](int j) {
-        uint32_t fl = pp_flags(P, IM, i, j, ppos, prad, phydro, B, A.pos, A.info);
-        if (fl) body(j, fl);
-    });
+    // the pairs in the reference's order, from the list where there is one
+    // (a test bond's item: its list holds what the scan would find)
+    const int c = A.L.cnt[i];
+    if (c <= min(SC_LIST_PP, P.listLimit)) {
+        for (int k = 0; k < c; k++) {
+            const uint32_t e = A.L.list[sc_list_at(SC_LIST_PP, i, k)];
+            body((int)(e & SC_PP_INDEX), e);
+        }
+    } else {
+        BondRegs B;
+        B.load(A.nb, A.bonds, i);
+        scan27(P, A.cellStart, ppos, reach(P, ppos, P.maxInt, SC_BINNED_P), [&](int j) {
+            uint32_t fl = pp_flags(P, IM, i, j, ppos, prad, phydro, B, A.pos, A.info);
+            if (fl) body(j, fl);
+        });
+    }
     sc_f3 nv = pvel + dV / fmaxf(w, 1.0f);
     pav = sc_qmul(sc_slerp(sc_qid(), dAV, 1.0f / fmaxf(w, 1.0f)), pav);
     if (phobSum > 0.0f) {
@@ -2784,11 +2794,13 @@ __global__ void __launch_bounds__(SC_THREADS) k_transition(
 //    the index is below the capacity), so neither needs a serial counter;
 //  * an item's processing reads and writes its own bonds and those of its
 //    previous monomer (pmi, found by id among the binned particles, whose
-//    ids no processing changes) and writes its new monomer's slot.  When no
-//    listed item's previous monomer is itself listed or shared with another
-//    item, the footprints are disjoint and every item runs at once
-//    (k_poly_apply); otherwise one thread runs them all in slot order
-//    (k_poly_finish), as before.
+//    ids no processing changes) and writes its new monomer's slot.  An item
+//    whose previous monomer is not itself listed or shared with another item,
+//    and which is nobody's previous monomer, shares its footprint with no
+//    other: those run at once (k_poly_apply), the others in slot order by one
+//    thread (k_poly_finish).  An item holds one bond of its rule's group, so
+//    what another's processing can do to its previous monomer is to take it
+//    away; a list with an item that holds more runs in slot order as a whole.
 __device__ __forceinline__ bool poly_scheduled(const PFields &F, int n0, int i) {
     return i < n0 && (F.info[i].z & SC_ACTIVE) && F.spoly[i] >= 0;
 }
@@ -2830,17 +2842,19 @@ __device__ __forceinline__ int poly_drop_group(int *mb, int mnb, int group) {
     return mnb;
 }
 
-// One scheduled item: `pmi` its previous monomer (-2: find it now), its new
-// monomer at newIdx with id newId (used when newIdx < N).
+// One scheduled item: `pmi` its previous monomer (`planned`: found before the
+// items ahead of it ran, and good as long as its bond names that particle), its
+// new monomer at newIdx with id newId (used when newIdx < N).
 __device__ void poly_one(const ScParams &P, const uint32_t *cellStart, const PFields &F, int i, int step, int pmi,
-                         int newIdx, int newId) {
+                         bool planned, int newIdx, int newId) {
     int4 in = F.info[i];
     const sc_rule &poly = rule_at(P, F.spoly[i]);
     const int pid = in.x, ptype = in.y;
     int *pb = F.bonds + (size_t)i * 24;
     int pnb = min(max(F.nb[i], 0), SC_MAX_ACTIVE_INTERACTIONS);
     const int api = poly_api(poly, pb, pnb);
-    if (pmi == -2) pmi = api >= 0 ? poly_find(P, cellStart, F, i, pb[3 * api + 2]) : -1;
+    if (planned && !(api >= 0 && pmi >= 0 && F.info[pmi].x == pb[3 * api + 2]))
+        pmi = api >= 0 ? poly_find(P, cellStart, F, i, pb[3 * api + 2]) : -1;
     float4 p4 = F.pos[i];
     const sc_f3 ppos = sc_make_f3(p4.x, p4.y, p4.z);
     const bool first = poly.first_partner_type == ptype;
@@ -2969,8 +2983,10 @@ __global__ void __launch_bounds__(SC_POLY_SCAN_THREADS) k_poly_offsets(const int
 }
 
 // Lists the scheduled items in index order with their monomer ranks, finds
-// each one's previous monomer, and flags a conflict when a previous monomer
-// is itself scheduled or claimed by two items.
+// each one's previous monomer and counts the claims on it, SC_POLY_LISTED more
+// when it is itself scheduled; an item with two bonds of its rule's group sends
+// the whole list through the serial path.
+#define SC_POLY_LISTED 0x10000
 __global__ void __launch_bounds__(SC_THREADS) k_poly_plan(ScParams P, const uint32_t *__restrict__ cellStart, PFields F,
                                                           ScCounters *ctr, const int2 *__restrict__ off, int *list,
                                                           int *rank, int *pmiOut, int *claim) {
@@ -2995,40 +3011,61 @@ __global__ void __launch_bounds__(SC_THREADS) k_poly_plan(ScParams P, const uint
     const int api = poly_api(poly, pb, min(max(F.nb[i], 0), SC_MAX_ACTIVE_INTERACTIONS));
     const int pmi = api >= 0 ? poly_find(P, cellStart, F, i, pb[3 * api + 2]) : -1;
     pmiOut[slot] = pmi;
-    if (pmi >= 0 && (poly_scheduled(F, n0, pmi) || atomicAdd(&claim[pmi], 1) != 0)) ctr->polyConflict = 1;
+    if (pmi >= 0) atomicAdd(&claim[pmi], poly_scheduled(F, n0, pmi) ? 1 + SC_POLY_LISTED : 1);
+    int held = 0;
+    for (int k = 0; k < min(max(F.nb[i], 0), SC_MAX_ACTIVE_INTERACTIONS); k++) held += pb[3 * k + 1] == poly.group;
+    if (held > 1) ctr->polyConflict = 1;
 }
 
-// Without a conflict every listed item runs at once; either way the claims
-// are cleared for the next step.
+// Whether a listed item's footprint meets another's (the claims are complete).
+__device__ __forceinline__ bool poly_meets(const int *claim, int i, int pmi) {
+    return claim[i] != 0 || (pmi >= 0 && claim[pmi] != 1);
+}
+
+// The items that share nothing with another, all at once.
 __global__ void __launch_bounds__(SC_THREADS) k_poly_apply(ScParams P, const uint32_t *__restrict__ cellStart, PFields F,
                                                            const ScCounters *ctr, const int *__restrict__ list,
                                                            const int *__restrict__ rank, const int *__restrict__ pmiIn,
-                                                           int *claim) {
+                                                           const int *claim) {
     const int slot = blockIdx.x * blockDim.x + threadIdx.x;
     if (slot >= ctr->polyCount) return;
-    const int pmi = pmiIn[slot];
-    if (pmi >= 0) claim[pmi] = 0;
-    if (ctr->polyConflict) return;
+    const int i = list[slot], pmi = pmiIn[slot];
+    if (ctr->polyConflict || poly_meets(claim, i, pmi)) return;
     const int r = rank[slot];
-    poly_one(P, cellStart, F, list[slot], ctr->step, pmi, r >= 0 ? ctr->lastActive + 1 + r : P.N,
+    poly_one(P, cellStart, F, i, ctr->step, pmi, false, r >= 0 ? ctr->lastActive + 1 + r : P.N,
              r >= 0 ? ctr->nextId + r : -1);
 }
 
-// The serial path of a conflicting list, then the counters: lastActive
-// advances by every creating item (the reference increments it before its
+// The items left, in slot order by one thread, while the others look through
+// the list for them; then the claims are cleared and the counters advance:
+// lastActive by every creating item (the reference increments it before its
 // capacity test), nextId and nActive by those that fit.
-__global__ void k_poly_finish(ScParams P, const uint32_t *__restrict__ cellStart, PFields F, ScCounters *ctr,
-                              const int *__restrict__ list, const int *__restrict__ rank) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+__global__ void __launch_bounds__(SC_THREADS) k_poly_finish(ScParams P, const uint32_t *__restrict__ cellStart, PFields F,
+                                                            ScCounters *ctr, const int *__restrict__ list,
+                                                            const int *__restrict__ rank, const int *__restrict__ pmiIn,
+                                                            int *claim) {
+    __shared__ int s_left[SC_THREADS];
     const int count = ctr->polyCount;
     if (count == 0) return;
     const int last0 = ctr->lastActive, next0 = ctr->nextId;
-    if (ctr->polyConflict) {
-        for (int k = 0; k < count; k++) {
-            const int r = rank[k];
-            poly_one(P, cellStart, F, list[k], ctr->step, -2, r >= 0 ? last0 + 1 + r : P.N, r >= 0 ? next0 + r : -1);
+    const bool all = ctr->polyConflict != 0;
+    for (int k0 = 0; k0 < count; k0 += SC_THREADS) {
+        const int k = k0 + threadIdx.x;
+        s_left[threadIdx.x] = k < count && (all || poly_meets(claim, list[k], pmiIn[k]));
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int u = 0; u < min(SC_THREADS, count - k0); u++) {
+                if (!s_left[u]) continue;
+                const int r = rank[k0 + u];
+                poly_one(P, cellStart, F, list[k0 + u], ctr->step, pmiIn[k0 + u], true, r >= 0 ? last0 + 1 + r : P.N,
+                         r >= 0 ? next0 + r : -1);
+            }
         }
+        __syncthreads();
     }
+    for (int k = threadIdx.x; k < count; k += SC_THREADS)
+        if (pmiIn[k] >= 0) claim[pmiIn[k]] = 0;
+    if (threadIdx.x) return;
     const int R = ctr->polyCreates;
     const int made = max(0, min(R, P.N - 1 - last0));
     ctr->lastActive = last0 + R;
@@ -3809,7 +3846,8 @@ void sc_phase_polymerize(ScLaunchCtx &c) {
                                              B.polyPmi, B.polyClaim);
     k_poly_apply<<<nb, SC_THREADS, 0, c.st>>>(c.P, B.cellStartP, F, B.ctr, B.polyList, B.polyRank, B.polyPmi,
                                               B.polyClaim);
-    k_poly_finish<<<1, 32, 0, c.st>>>(c.P, B.cellStartP, F, B.ctr, B.polyList, B.polyRank);
+    k_poly_finish<<<1, SC_THREADS, 0, c.st>>>(c.P, B.cellStartP, F, B.ctr, B.polyList, B.polyRank, B.polyPmi,
+                                              B.polyClaim);
     (*c.launches) += 5;
 }
 
