@@ -181,17 +181,27 @@ void sc_launch_gather_particles(cudaStream_t st, const uint32_t *perm, int n, co
 void sc_launch_gather_metabolic(cudaStream_t st, const uint32_t *perm, int n, int sp4, ScBuffers &B,
                                 long long *launches);
 
-// sc_observe.cu: FP64 observables.  The observe launcher reduces one item set
-// into out[sc_observe_cols()] through a partials table of
-// sc_observe_rows() x sc_observe_cols() doubles (columns: MSD sum, MSD
-// items, |v|^2 sum, active items, bond slots, then one per species).
+// sc_observe.cu: FP64 observables.  The observe launcher reduces both item
+// sets, each into its sc_observe_cols() values of out (particles first),
+// through a partials table of sc_observe_rows() x sc_observe_cols() doubles
+// (columns: MSD sum, MSD items, |v|^2 sum, active items, bond slots, then one
+// per species).
+struct ScObserveSet {
+    const int *nActive;
+    const float4 *pos, *vel;
+    const int4 *info;
+    const int *nb;      // bond counts, or null
+    const float *met;   // amounts, S of sp a slot, or null
+    int sp, S;
+    const float4 *mark;   // positions by id, or null
+    int markCap;
+};
 int sc_observe_cols();
 int sc_observe_rows();
 void sc_launch_mark(cudaStream_t st, const int *nActive, const float4 *pos, const int4 *info, float4 *mark,
                     int markCap);
-void sc_launch_observe(cudaStream_t st, const int *nActive, const float4 *pos, const float4 *vel, const int4 *info,
-                       const int *nb, const float *met, int sp, int S, const float4 *mark, int markCap, double box,
-                       int periodic, double *partials, double *out);
+void sc_launch_observe(cudaStream_t st, const ScObserveSet &P, const ScObserveSet &M, double box, int periodic,
+                       double *partials, double *out);
 void sc_launch_pair_histogram(cudaStream_t st, const ScParams &P, const uint32_t *cellStart, const int *nActive,
                               const float4 *pos, const int4 *info, int typeA, int typeB, double rMax, int nBins,
                               unsigned long long *counts, int gridCap);

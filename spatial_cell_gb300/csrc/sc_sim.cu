@@ -1849,19 +1849,13 @@ int sc_observe(sc_sim *s, sc_observables *out) {
     }
     ScBuffers &B = s->B;
     double *res = s->obs + (size_t)rows * cols;
-    SC_CK(s, cudaMemsetAsync(res, 0, 2 * (size_t)cols * sizeof(double), s->st));
-    const double box = s->cfg.sim_size;
-    if (s->P.N > 0) {
-        PFields F = B.P();
-        sc_launch_observe(s->st, &B.ctr->nActive, F.pos, F.vel, F.info, F.nb, nullptr, 0, 0, s->markP, s->markCapP,
-                          box, s->P.periodic, s->obs, res);
-    }
-    if (s->P.Nm > 0) {
-        MFields M = B.M();
-        sc_launch_observe(s->st, &B.ctr->nActiveM, M.pos, M.vel, M.info, nullptr,
-                          reinterpret_cast<const float *>(M.met), s->P.SP, s->P.S, s->markM, s->markCapM, box,
-                          s->P.periodic, s->obs, res + cols);
-    }
+    PFields F = B.P();
+    MFields M = B.M();
+    sc_launch_observe(s->st,
+                      {&B.ctr->nActive, F.pos, F.vel, F.info, F.nb, nullptr, 0, 0, s->markP, s->markCapP},
+                      {&B.ctr->nActiveM, M.pos, M.vel, M.info, nullptr, reinterpret_cast<const float *>(M.met),
+                       s->P.SP, s->P.S, s->markM, s->markCapM},
+                      s->cfg.sim_size, s->P.periodic, s->obs, res);
     std::vector<double> h((size_t)2 * cols);
     SC_CK(s, cudaMemcpyAsync(h.data(), res, h.size() * sizeof(double), cudaMemcpyDeviceToHost, s->st));
     SC_CK(s, cudaStreamSynchronize(s->st));
