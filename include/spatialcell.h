@@ -421,7 +421,7 @@ int sc_export_replica(sc_sim *sim, int32_t replica, sc_particle *particles, sc_m
  *         [cell_start[c], cell_start[c + 1]); inactive items come last)
  *   stream: a cudaStream_t (NULL: the legacy default stream)
  * Limit: n <= 262144; larger n returns SC_E_INVALID and launches nothing.
- * The static array (about 4.3 MB) stays on every GPU that loads the library
+ * The static array (about 4.8 MB) stays on every GPU that loads the library
  * until the process exits.  All calls on a GPU share it, so calls whose work
  * overlaps on that GPU race; order them on one stream.  Every call looks up
  * the array's address on the current device (no allocation) and waits for

@@ -7,8 +7,8 @@
 //      bits) and the digit histograms of every pass, one read of pos + info;
 //   2. k_onesweep: one LSD pass per 8-bit digit over only the 3*bits+1 key bits
 //      (Adinets & Merrill, "Onesweep: A Faster Least Significant Digit Radix
-//      Sort for GPUs", 2022): each CTA ranks a 4096-key tile stably in shared
-//      memory, publishes its digit counts, resolves its global offsets by a
+//      Sort for GPUs", 2022): each CTA ranks its tile's keys stably, each warp its
+//      own in shared memory, publishes its digit counts, resolves its global offsets by a
 //      decoupled look-back over predecessor tiles, and scatters (key, slot);
 //      sorting the used bits only is the same total order as CUB's 32-bit
 //      stable sort, so the permutation is identical;
@@ -17,8 +17,13 @@
 //   4. k_gather_*: every SoA field moved by the permutation.
 #include "sc_launch.h"
 
+#include <algorithm>
+
+// Keys per thread of a sort pass at most (sort_ipt).
 #define SORT_IPT 16
-#define SORT_TILE (SC_THREADS * SORT_IPT)
+#define SORT_SMS 152
+#define SORT_KEYS 4
+#define SORT_LOOK 8   // tiles a look-back reads at a time
 #define LB_AGG 0x40000000u
 #define LB_INC 0x80000000u
 #define LB_FLAGS 0xC0000000u
@@ -36,26 +41,45 @@ __device__ __forceinline__ void st_relaxed(uint32_t *p, uint32_t v) {
 
 // In a batched sim the key is the item's replica's key base plus its cell
 // in that replica's grid: replicas sort into consecutive key ranges.
-template <bool BATCH>
+//
+// Past a block per SM a thread takes SORT_KEYS items, their loads together, so
+// that fewer blocks add to each of the histogram's words: 262,144 items 12.4 us
+// at one item, 6.1 us at four.  The kernel also clears what the passes behind it look at first (the look-back words and
+// tile counters) and farMove.
+template <bool BATCH, int KEYS>
 __global__ void __launch_bounds__(SC_THREADS) k_sort_keys(const float4 *__restrict__ pos, const int4 *__restrict__ info,
                                                           int n, ScParams P, uint32_t inactiveKey, int passes,
-                                                          uint32_t *__restrict__ keys, uint32_t *__restrict__ hist) {
+                                                          uint32_t *__restrict__ keys, uint32_t *__restrict__ hist,
+                                                          uint32_t *__restrict__ lookback, int lbWords, ScCounters *ctr) {
     __shared__ uint32_t sh[4 * 256];
     for (int t = threadIdx.x; t < passes * 256; t += blockDim.x) sh[t] = 0;
     __syncthreads();
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
+    const int first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    int4 in[KEYS];
+    sc_f3 p[KEYS];
+#pragma unroll
+    for (int r = 0; r < KEYS; r++) {
+        const int i = min(first + r * stride, n - 1);
+        in[r] = info[i];
+        p[r] = ld3(pos, i);
+    }
+#pragma unroll
+    for (int r = 0; r < KEYS; r++) {
+        const int i = first + r * stride;
+        if (i >= n) break;
         uint32_t k = inactiveKey;
-        const int4 in = info[i];
-        if (in.z & SC_ACTIVE) {
-            rep_apply<BATCH>(P, in.w);
-            sc_f3 p = ld3(pos, i);
+        if (in[r].z & SC_ACTIVE) {
+            rep_apply<BATCH>(P, in[r].w);
             int lim = cell_limit(P);
-            k = cell_key(P, sc_grid_idx(p.x, P.cell, lim), sc_grid_idx(p.y, P.cell, lim), sc_grid_idx(p.z, P.cell, lim));
+            k = cell_key(P, sc_grid_idx(p[r].x, P.cell, lim), sc_grid_idx(p[r].y, P.cell, lim),
+                         sc_grid_idx(p[r].z, P.cell, lim));
         }
         keys[i] = k;
         for (int d = 0; d < passes; d++) atomicAdd(&sh[d * 256 + ((k >> (8 * d)) & 0xffu)], 1u);
     }
+    for (int w = first; w < lbWords; w += stride) lookback[w] = 0;
+    if (first < 4) ctr->tileCounter[first] = 0;
+    if (first == 4) ctr->farMove = 0;
     __syncthreads();
     for (int t = threadIdx.x; t < passes * 256; t += blockDim.x)
         if (sh[t]) atomicAdd(&hist[t], sh[t]);
@@ -77,6 +101,11 @@ __device__ __forceinline__ uint32_t block_exclusive_scan256(uint32_t v, uint32_t
     return pre + x - v;
 }
 
+// One pass.  Bound by latency at these sizes (L2 holds the keys): with the
+// warps ranking their own keys without a barrier per round and eight tiles
+// looked back at a time, a pass over 262,144 keys takes 9.7 us, 14.4 with a
+// block-wide round per 256 keys and a tile at a time.
+template <int IPT>
 __global__ void __launch_bounds__(SC_THREADS) k_onesweep(const uint32_t *__restrict__ keysIn,
                                                          const uint32_t *__restrict__ valsIn,
                                                          uint32_t *__restrict__ keysOut, uint32_t *__restrict__ valsOut,
@@ -84,25 +113,22 @@ __global__ void __launch_bounds__(SC_THREADS) k_onesweep(const uint32_t *__restr
                                                          uint32_t *__restrict__ lookback, int *tileCounter,
                                                          ScCounters *ctr) {
     __shared__ uint32_t s_tile;
-    __shared__ uint32_t s_bin[256];
-    __shared__ uint32_t s_cnt[8][256];
-    __shared__ uint32_t s_off[8][256];
+    __shared__ uint32_t s_cnt[8][256];   // a warp's keys per digit so far; then its first key's rank
     __shared__ uint32_t s_base[256];
     __shared__ uint32_t s_wsum[8];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) s_tile = (uint32_t)atomicAdd(tileCounter, 1);
-    s_bin[tid] = 0;
 #pragma unroll
     for (int w = 0; w < 8; w++) s_cnt[w][tid] = 0;
     __syncthreads();
     const uint32_t tile = s_tile;
-    const long long base = (long long)tile * SORT_TILE;
+    const long long base = ((long long)tile * 8 + warp) * (32 * IPT) + lane;   // a warp's keys lie together
     const uint32_t ltmask = (1u << lane) - 1u;
 
-    uint32_t key[SORT_IPT], val[SORT_IPT], rank[SORT_IPT];
+    uint32_t key[IPT], val[IPT], rank[IPT];
 #pragma unroll
-    for (int r = 0; r < SORT_IPT; r++) {
-        long long idx = base + r * SC_THREADS + tid;
+    for (int r = 0; r < IPT; r++) {
+        long long idx = base + r * 32;
         if (idx < n) {
             key[r] = keysIn[idx];
             val[r] = valsIn ? valsIn[idx] : (uint32_t)idx;
@@ -111,55 +137,57 @@ __global__ void __launch_bounds__(SC_THREADS) k_onesweep(const uint32_t *__restr
             val[r] = 0;
         }
     }
-    // Stable ranking: tile order is (round, thread); within a round the warp
-    // match gives the rank among equal digits, and the per-digit running sum
-    // over warps and rounds gives the offset.
+    // Stable ranking: tile order is (warp, round, lane).  Within a round the
+    // warp match gives the rank among equal digits, behind the warp's count of
+    // the rounds before; the warps' counts then become their offsets.
 #pragma unroll
-    for (int r = 0; r < SORT_IPT; r++) {
-        bool valid = base + r * SC_THREADS + tid < n;
-        uint32_t d = valid ? ((key[r] >> shift) & 0xffu) : 256u;
-        uint32_t peers = __match_any_sync(0xffffffffu, d);
-        uint32_t wrank = __popc(peers & ltmask);
-        if (valid && wrank == 0) s_cnt[warp][d] = __popc(peers);
-        __syncthreads();
-        {
-            uint32_t run = s_bin[tid];
-#pragma unroll
-            for (int w = 0; w < 8; w++) {
-                uint32_t c = s_cnt[w][tid];
-                s_cnt[w][tid] = 0;
-                s_off[w][tid] = run;
-                run += c;
-            }
-            s_bin[tid] = run;
-        }
-        __syncthreads();
-        rank[r] = valid ? s_off[warp][d] + wrank : 0u;
+    for (int r = 0; r < IPT; r++) {
+        const bool valid = base + r * 32 < n;
+        const uint32_t d = valid ? ((key[r] >> shift) & 0xffu) : 256u;
+        const uint32_t peers = __match_any_sync(0xffffffffu, d);
+        const uint32_t before = valid ? s_cnt[warp][d] : 0u;
+        __syncwarp();
+        rank[r] = before + __popc(peers & ltmask);
+        if (valid && (peers & ltmask) == 0) s_cnt[warp][d] = before + __popc(peers);
+        __syncwarp();
     }
+    __syncthreads();
     // Decoupled look-back: thread tid owns digit tid.
-    const uint32_t cnt = s_bin[tid];
+    uint32_t cnt = 0;
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+        const uint32_t c = s_cnt[w][tid];
+        s_cnt[w][tid] = cnt;
+        cnt += c;
+    }
     uint32_t excl = 0;
     if (tile == 0) {
         st_relaxed(&lookback[tid], LB_INC | cnt);
     } else {
         st_relaxed(&lookback[(size_t)tile * 256 + tid], LB_AGG | cnt);
-        long long pred = (long long)tile - 1;
-        while (pred >= 0) {
-            uint32_t v = 0;
-            int spins = 0;
-            while (true) {
-                v = ld_relaxed(&lookback[(size_t)pred * 256 + tid]);
-                if (v & LB_FLAGS) break;
-                if (++spins > LB_SPIN_LIMIT) {
-                    set_error(ctr, SC_DERR_LOOKBACK_TIMEOUT);
-                    v = LB_INC;
-                    break;
+        // SORT_LOOK tiles' words on their way at once; a word that is not
+        // there yet is waited for when its turn comes
+        bool found = false;
+        for (long long pred = (long long)tile - 1; pred >= 0 && !found; pred -= SORT_LOOK) {
+            uint32_t v[SORT_LOOK];
+#pragma unroll
+            for (int u = 0; u < SORT_LOOK; u++)
+                v[u] = pred >= u ? ld_relaxed(&lookback[(size_t)(pred - u) * 256 + tid]) : LB_INC;
+#pragma unroll
+            for (int u = 0; u < SORT_LOOK; u++) {
+                if (found) continue;
+                for (int spins = 0; !(v[u] & LB_FLAGS);) {
+                    if (++spins > LB_SPIN_LIMIT) {
+                        set_error(ctr, SC_DERR_LOOKBACK_TIMEOUT);
+                        v[u] = LB_INC;
+                        break;
+                    }
+                    __nanosleep(32);
+                    v[u] = ld_relaxed(&lookback[(size_t)(pred - u) * 256 + tid]);
                 }
-                __nanosleep(32);
+                excl += v[u] & LB_VALUE;
+                found = v[u] & LB_INC;
             }
-            excl += v & LB_VALUE;
-            if (v & LB_INC) break;
-            pred--;
         }
         st_relaxed(&lookback[(size_t)tile * 256 + tid], LB_INC | (excl + cnt));
     }
@@ -167,11 +195,11 @@ __global__ void __launch_bounds__(SC_THREADS) k_onesweep(const uint32_t *__restr
     s_base[tid] = gofs + excl;
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < SORT_IPT; r++) {
-        long long idx = base + r * SC_THREADS + tid;
+    for (int r = 0; r < IPT; r++) {
+        long long idx = base + r * 32;
         if (idx < n) {
             uint32_t d = (key[r] >> shift) & 0xffu;
-            uint32_t dst = s_base[d] + rank[r];
+            uint32_t dst = s_base[d] + s_cnt[warp][d] + rank[r];
             keysOut[dst] = key[r];
             valsOut[dst] = val[r];
         }
@@ -255,7 +283,20 @@ __global__ void __launch_bounds__(SC_THREADS) k_gather_mfield(const uint32_t *__
 int sc_sort_passes(int bits) { return (3 * bits + 1 + 7) / 8; }
 int sc_sort_passes_for(const ScParams &P) { return ((P.keyBits > 0 ? P.keyBits : 3 * P.bits + 1) + 7) / 8; }
 
-size_t sc_sort_lookback_words(int cap) { return (size_t)((cap + SORT_TILE - 1) / SORT_TILE) * 256; }
+// Four or eight keys per thread while every tile has an SM of its own, sixteen
+// beyond: a pass of few tiles is the latency of one tile's rounds of ranking
+// (a whole sort of 32,768 items 61 us at sixteen, 52 at eight, 49 at four;
+// 131,072: 74, 63, 63; 200,000: 75, 66, 74); past an SM each there is nothing
+// left to gain (262,144: 75, 74, 75) and fewer tiles look back less.
+static size_t sort_tiles(long long n, int ipt) { return (size_t)((n + SC_THREADS * ipt - 1) / (SC_THREADS * ipt)); }
+static int sort_ipt(long long n) {
+    return sort_tiles(n, 4) <= SORT_SMS ? 4 : sort_tiles(n, 8) <= SORT_SMS ? 8 : SORT_IPT;
+}
+
+// Words of one pass's look-back table for up to cap items, whatever their number.
+size_t sc_sort_lookback_words(int cap) {
+    return std::max<size_t>(std::min<size_t>(sort_tiles(cap, 4), SORT_SMS), sort_tiles(cap, SORT_IPT)) * 256;
+}
 
 // Sorts the keys of one item set; returns the buffer index (0/1) holding the
 // sorted keys and the permutation.  hist: 4*256 words, lookback: per pass.
@@ -265,23 +306,28 @@ int sc_launch_sort(cudaStream_t st, const float4 *pos, const int4 *info, int n, 
     int passes = sc_sort_passes_for(P);
     int keyBits = P.keyBits > 0 ? P.keyBits : 3 * P.bits + 1;
     uint32_t inactiveKey = keyBits >= 32 ? 0xffffffffu : ((1u << keyBits) - 1u);
-    int tiles = (n + SORT_TILE - 1) / SORT_TILE;
-    size_t lbWords = (size_t)tiles * 256;
+    const int ipt = sort_ipt(n);
+    const int tiles = (int)sort_tiles(n, ipt);
+    auto *const pass = ipt == 4 ? k_onesweep<4> : ipt == 8 ? k_onesweep<8> : k_onesweep<SORT_IPT>;
+    const size_t lbWords = (size_t)tiles * 256;
     cudaMemsetAsync(hist, 0, 4 * 256 * sizeof(uint32_t), st);
-    cudaMemsetAsync(lookback, 0, (size_t)passes * lbWords * sizeof(uint32_t), st);
-    // the tile counters and farMove behind them
-    cudaMemsetAsync(ctr->tileCounter, 0, sizeof(ctr->tileCounter) + sizeof(ctr->farMove), st);
-    int blocks = (n + SC_THREADS - 1) / SC_THREADS;
     if (n > 0) {
-        (P.nRep > 1 ? k_sort_keys<true> : k_sort_keys<false>)<<<blocks, SC_THREADS, 0, st>>>(
-            pos, info, n, P, inactiveKey, passes, keys[0], hist);
+        const bool one = (n + SC_THREADS - 1) / SC_THREADS <= SORT_SMS;
+        const int per = SC_THREADS * (one ? 1 : SORT_KEYS), blocks = (int)(((long long)n + per - 1) / per);
+        auto *const make = P.nRep > 1 ? (one ? k_sort_keys<true, 1> : k_sort_keys<true, SORT_KEYS>)
+                                      : (one ? k_sort_keys<false, 1> : k_sort_keys<false, SORT_KEYS>);
+        make<<<blocks, SC_THREADS, 0, st>>>(pos, info, n, P, inactiveKey, passes, keys[0], hist, lookback,
+                                            (int)(passes * lbWords), ctr);
         (*launches)++;
+    } else {
+        // the tile counters and farMove behind them
+        cudaMemsetAsync(ctr->tileCounter, 0, sizeof(ctr->tileCounter) + sizeof(ctr->farMove), st);
     }
     int cur = 0;
     for (int d = 0; d < passes && n > 0; d++) {
-        k_onesweep<<<tiles, SC_THREADS, 0, st>>>(keys[cur], d == 0 ? nullptr : vals[cur], keys[1 - cur],
-                                                  vals[1 - cur], n, 8 * d, hist + 256 * d,
-                                                  lookback + (size_t)d * lbWords, &ctr->tileCounter[d], ctr);
+        pass<<<tiles, SC_THREADS, 0, st>>>(keys[cur], d == 0 ? nullptr : vals[cur], keys[1 - cur], vals[1 - cur], n,
+                                           8 * d, hist + 256 * d, lookback + (size_t)d * lbWords,
+                                           &ctr->tileCounter[d], ctr);
         (*launches)++;
         cur = 1 - cur;
     }

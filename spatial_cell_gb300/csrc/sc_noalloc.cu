@@ -11,7 +11,7 @@
 // Limits and sharing:
 //   * at most SC_STATIC_SORT_MAX_ITEMS items per call (larger calls are
 //     rejected with SC_E_INVALID before anything is launched);
-//   * the array occupies about 4.3 MB on every GPU that loads the library,
+//   * the array occupies about 4.8 MB on every GPU that loads the library,
 //     until the process exits;
 //   * every call on a device uses the same array, so calls whose work
 //     overlaps on the GPU (other streams, other host threads) race: order
@@ -29,8 +29,7 @@
 #include "sc_launch.h"
 
 #define SC_STATIC_SORT_MAX_ITEMS (1 << 18)
-#define SC_STATIC_SORT_TILE 4096
-#define SC_STATIC_SORT_TILES ((SC_STATIC_SORT_MAX_ITEMS + SC_STATIC_SORT_TILE - 1) / SC_STATIC_SORT_TILE)
+#define SC_STATIC_SORT_TILES 152   // most tiles of a pass (sc_sort_lookback_words, checked per call)
 
 namespace {
 
@@ -78,6 +77,7 @@ extern "C" int sc_sort_cells_static(const sc_config *cfg, const void *pos, const
     if (cfg->periodic && cfg->grid_cell_size > 0.0f)
         P.nUsed = sc_periodic_cells(cfg->sim_size, cfg->grid_cell_size, &P.cell);
     long long launches = 0;
+    if (sc_sort_lookback_words(SC_STATIC_SORT_MAX_ITEMS) > (size_t)SC_STATIC_SORT_TILES * 256) return SC_E_INVALID;
     if (cudaMemsetAsync(ctr, 0, sizeof(ScCounters), st) != cudaSuccess) return SC_E_CUDA;
     int cur = sc_launch_sort(st, (const float4 *)pos, (const int4 *)info, n, P, keys, vals, hist, lookback, ctr,
                              &launches);
