@@ -60,7 +60,8 @@ struct ScBuffers {
     int relaxMAge;                // relax_metab launches since the metabolic velocities were last out of step (0, 1)
     int diffuseAge;               // the same for the amounts
     int *permM, *permLM, *permD;  // count-ordered list position -> item
-    uint32_t *scratchLM;          // build scratch of the LM list (aliases listD when it fits)
+    uint32_t *scratchLM;          // build scratch of the LM list (in listD when it fits)
+    bool scratchInD, scratchApart;   // it lies in listD; clear of the metabolic list's scratch
     int *ovfPP, *ovfM;            // overflowed items
     // The metabolic items whose list overflowed keep their full pair list in
     // a second pool (16-byte entries as the main one, an item's entries
@@ -221,6 +222,7 @@ struct ScLaunchCtx {
     cudaEvent_t fork, join[2];
 };
 void sc_phase_move_brownian(ScLaunchCtx &c, bool metabolic);
+void sc_phase_build_all(ScLaunchCtx &c);  // the relaxation's lists at once, in sims that gain from it
 void sc_phase_coordinate_noise(ScLaunchCtx &c, float frac);
 void sc_phase_apply_noise(ScLaunchCtx &c);
 void sc_phase_relax(ScLaunchCtx &c);

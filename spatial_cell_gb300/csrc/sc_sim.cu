@@ -527,6 +527,10 @@ int step_direct(sc_sim *s) {
     const sc_config &c = s->cfg;
     run_phase(s, SC_PHASE_SORT_PARTICLES, 0);
     run_phase(s, SC_PHASE_SORT_METABOLIC, 0);
+    if (c.relaxation_steps > 0) {
+        ScLaunchCtx all = ctx(s);
+        sc_phase_build_all(all);
+    }
     run_phase(s, SC_PHASE_MOVE_BROWNIAN, 0);
     run_phase(s, SC_PHASE_MOVE_BROWNIAN_METAB, 0);
     for (int j = 0; j < c.noise_coordination_steps; j++) run_phase(s, SC_PHASE_COORDINATE_NOISE, j);
@@ -942,10 +946,15 @@ static int create_sim(const sc_config *cfg_in, const sc_replica *replicas, int32
         (rc = dalloc(s, &B.warpOffM, (size_t)Nm / 32 + 1)) || (rc = dalloc(s, &B.warpOffLM, (size_t)N / 32 + 1)) ||
         (rc = dalloc(s, &B.lipidP, N)) || (rc = dalloc(s, &B.comb, N + Nm + SC_CAND_PAD)))
         return bail(rc);
-    // The LM list is built in the diffusion list's buffer when it fits.
-    if (sc_list_words(SC_LIST_LM, (int)N) <= sc_list_words(SC_LIST_DBUF, (int)Nm)) {
-        B.scratchLM = B.listD;
-    } else if ((rc = dalloc(s, &B.scratchLM, sc_list_words(SC_LIST_LM, (int)N)))) {
+    // The LM list is built in the diffusion list's buffer when it fits, behind
+    // the metabolic list's scratch when both do.
+    const size_t wordsLM = sc_list_words(SC_LIST_LM, (int)N), wordsM = sc_list_words(SC_LIST_M, (int)Nm),
+                 wordsD = sc_list_words(SC_LIST_DBUF, (int)Nm);
+    B.scratchInD = wordsLM <= wordsD;
+    B.scratchApart = !B.scratchInD || wordsM + wordsLM <= wordsD;
+    if (B.scratchInD) {
+        B.scratchLM = B.listD + (B.scratchApart ? wordsM : 0);
+    } else if ((rc = dalloc(s, &B.scratchLM, wordsLM))) {
         return bail(rc);
     }
     B.invalidateLists();

@@ -248,17 +248,13 @@ __device__ __forceinline__ uint32_t pp_flags(const ScParams &P, const Imager &IM
 // Particle-particle list, built once after the sort; read by coordinateNoise
 // and relax.
 template <bool BATCH>
-__global__ void __launch_bounds__(SC_THREADS) k_build_pp(ScParams P, const uint32_t *__restrict__ cellStart,
-                                                         const int *__restrict__ nActivePtr,
-                                                         const float4 *__restrict__ pos, const int4 *__restrict__ info,
-                                                         const int *__restrict__ nb, const int *__restrict__ bonds,
-                                                         uint32_t *__restrict__ list, int *__restrict__ cnt, int cap,
-                                                         int *__restrict__ classIdx, int *__restrict__ classCount,
-                                                         int *__restrict__ ovf, int *__restrict__ ovfCount,
-                                                         uint32_t *__restrict__ match, int *__restrict__ matchN,
-                                                         float4 *__restrict__ geo) {
-    __shared__ ScanWords W;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void build_pp_block(
+    ScParams P, ScanWords &W, int block, const uint32_t *__restrict__ cellStart, const int *__restrict__ nActivePtr,
+    const float4 *__restrict__ pos, const int4 *__restrict__ info, const int *__restrict__ nb,
+    const int *__restrict__ bonds, uint32_t *__restrict__ list, int *__restrict__ cnt, int cap,
+    int *__restrict__ classIdx, int *__restrict__ classCount, int *__restrict__ ovf, int *__restrict__ ovfCount,
+    uint32_t *__restrict__ match, int *__restrict__ matchN, float4 *__restrict__ geo) {
+    int i = block * SC_THREADS + threadIdx.x;
     if (i >= *nActivePtr) return;
     int4 in = info[i];
     int cls = 2;
@@ -326,6 +322,17 @@ __global__ void __launch_bounds__(SC_THREADS) k_build_pp(ScParams P, const uint3
     if (lane == leader) base = atomicAdd(&classCount[cls], __popc(same));
     base = __shfl_sync(same, base, leader);
     classIdx[(size_t)cls * cap + base + __popc(same & ((1u << lane) - 1u))] = i | (int)inactive;
+}
+template <bool BATCH>
+__global__ void __launch_bounds__(SC_THREADS) k_build_pp(
+    ScParams P, const uint32_t *__restrict__ cellStart, const int *__restrict__ nActivePtr,
+    const float4 *__restrict__ pos, const int4 *__restrict__ info, const int *__restrict__ nb,
+    const int *__restrict__ bonds, uint32_t *__restrict__ list, int *__restrict__ cnt, int cap,
+    int *__restrict__ classIdx, int *__restrict__ classCount, int *__restrict__ ovf, int *__restrict__ ovfCount,
+    uint32_t *__restrict__ match, int *__restrict__ matchN, float4 *__restrict__ geo) {
+    __shared__ ScanWords W;
+    build_pp_block<BATCH>(P, W, blockIdx.x, cellStart, nActivePtr, pos, info, nb, bonds, list, cnt, cap, classIdx, classCount, ovf,
+                          ovfCount, match, matchN, geo);
 }
 
 // Visits the contributing pairs of particle i in the reference's order: from
@@ -1474,14 +1481,14 @@ struct PoolSlot {
     T *out;
 };
 template <int K, class T>
-__device__ __forceinline__ PoolSlot<T> pool_take(const ScParams &P, bool valid, int c, T *__restrict__ pool,
+__device__ __forceinline__ PoolSlot<T> pool_take(const ScParams &P, int block, bool valid, int c, T *__restrict__ pool,
                                               long long poolCap, unsigned long long *__restrict__ poolUsed, long long *__restrict__ warpOff,
                                               int *__restrict__ cnt, int *__restrict__ perm, int cap,
                                               int *__restrict__ ovf, int *__restrict__ ovfCount,
                                               const int *__restrict__ items = nullptr, int *__restrict__ ovfN = nullptr) {
     __shared__ int s_n[SC_THREADS / 32];
     __shared__ long long s_base;
-    const int b0 = blockIdx.x * SC_THREADS, t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int b0 = block * SC_THREADS, t = threadIdx.x, lane = t & 31, warp = t >> 5;
     int src, cs;
     count_rank<K>(valid, c, &src, &cs);
     const int limit = min(K, P.listLimit);
@@ -1537,14 +1544,14 @@ __device__ __forceinline__ PoolSlot<T> pool_take(const ScParams &P, bool valid, 
 // overflowed item, or every item of a block the pool has no room for, is
 // listed in `ovf` for the scan.
 template <bool BATCH>
-__device__ __forceinline__ void emit_m_pairs(const ScParams &P0, bool valid, int c, const uint32_t *scratch,
+__device__ __forceinline__ void emit_m_pairs(const ScParams &P0, int block, bool valid, int c, const uint32_t *scratch,
                                              const int4 *__restrict__ minfo,
                                              const float4 *__restrict__ mpos, const float4 *__restrict__ ppos_,
                                              uint4 *__restrict__ pool, long long poolCap, unsigned long long *__restrict__ poolUsed,
                                              long long *__restrict__ warpOff, int *__restrict__ cnt, int *__restrict__ perm,
                                              int cap, int *__restrict__ ovf, int *__restrict__ ovfCount,
                                              int *__restrict__ ovfN) {
-    const PoolSlot<uint4> S = pool_take<SC_LIST_M>(P0, valid, c, pool, poolCap, poolUsed, warpOff, cnt, perm, cap, ovf,
+    const PoolSlot<uint4> S = pool_take<SC_LIST_M>(P0, block, valid, c, pool, poolCap, poolUsed, warpOff, cnt, perm, cap, ovf,
                                                    ovfCount, nullptr, ovfN);
     if (S.n == 0) return;
     const int i = S.i;
@@ -1582,30 +1589,25 @@ __device__ __forceinline__ void emit_m_pairs(const ScParams &P0, bool valid, int
 // sub-iteration (a 16-byte gather that nearby items share in L1 / L2, and a
 // square root and a division per pair) instead of streaming 12 more bytes
 // per pair from HBM.
-__device__ __forceinline__ void emit_m_pairs_lean(const ScParams &P, bool valid, int c, const uint32_t *scratch,
+__device__ __forceinline__ void emit_m_pairs_lean(const ScParams &P, int block, bool valid, int c, const uint32_t *scratch,
                                                   uint32_t *__restrict__ pool, long long poolCap,
                                                   unsigned long long *__restrict__ poolUsed, long long *__restrict__ warpOff,
                                                   int *__restrict__ cnt, int *__restrict__ perm, int cap,
                                                   int *__restrict__ ovf, int *__restrict__ ovfCount,
                                                   int *__restrict__ ovfN) {
-    const PoolSlot<uint32_t> S = pool_take<SC_LIST_M>(P, valid, c, pool, poolCap, poolUsed, warpOff, cnt, perm, cap,
+    const PoolSlot<uint32_t> S = pool_take<SC_LIST_M>(P, block, valid, c, pool, poolCap, poolUsed, warpOff, cnt, perm, cap,
                                                       ovf, ovfCount, nullptr, ovfN);
     for (int k = 0; k < S.n; k++) S.out[(size_t)k * 32] = scratch[sc_list_at(SC_LIST_M, S.i, k)];
 }
 
 template <bool LEAN, bool BATCH>
-__global__ void __launch_bounds__(SC_THREADS, 4) k_build_m(ScParams P0, CombStart cs, const float4 *__restrict__ comb,
-                                                        const int *__restrict__ nActivePtr,
-                                                        const float4 *__restrict__ mpos, const int4 *__restrict__ minfo,
-                                                        const float4 *__restrict__ ppos_,
-                                                        uint32_t *__restrict__ pool, long long poolCap,
-                                                        unsigned long long *__restrict__ poolUsed,
-                                                        long long *__restrict__ warpOff, uint32_t *scratch,
-                                                        int *__restrict__ cnt, int *__restrict__ perm, int cap,
-                                                        int *__restrict__ ovf, int *__restrict__ ovfCount,
-                                                        int *__restrict__ ovfN) {
-    __shared__ ScanWords W;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void build_m_block(
+    const ScParams &P0, ScanWords &W, int block, CombStart cs, const float4 *__restrict__ comb, const int *__restrict__ nActivePtr, const float4 *__restrict__ mpos,
+    const int4 *__restrict__ minfo, const float4 *__restrict__ ppos_, uint32_t *__restrict__ pool, long long poolCap,
+    unsigned long long *__restrict__ poolUsed, long long *__restrict__ warpOff, uint32_t *scratch,
+    int *__restrict__ cnt, int *__restrict__ perm, int cap, int *__restrict__ ovf, int *__restrict__ ovfCount,
+    int *__restrict__ ovfN) {
+    const int i = block * SC_THREADS + threadIdx.x;
     const bool valid = i < *nActivePtr;
     int c = 0;
     if (valid) {
@@ -1615,10 +1617,22 @@ __global__ void __launch_bounds__(SC_THREADS, 4) k_build_m(ScParams P0, CombStar
         if (mi.z & SC_ACTIVE) build_m_item(P, W, cs, comb, i, mpos, ppos_, scratch, c);
     }
     if (LEAN)
-        emit_m_pairs_lean(P0, valid, c, scratch, pool, poolCap, poolUsed, warpOff, cnt, perm, cap, ovf, ovfCount, ovfN);
+        emit_m_pairs_lean(P0, block, valid, c, scratch, pool, poolCap, poolUsed, warpOff, cnt, perm, cap, ovf, ovfCount,
+                          ovfN);
     else
-        emit_m_pairs<BATCH>(P0, valid, c, scratch, minfo, mpos, ppos_, reinterpret_cast<uint4 *>(pool), poolCap,
+        emit_m_pairs<BATCH>(P0, block, valid, c, scratch, minfo, mpos, ppos_, reinterpret_cast<uint4 *>(pool), poolCap,
                             poolUsed, warpOff, cnt, perm, cap, ovf, ovfCount, ovfN);
+}
+template <bool LEAN, bool BATCH>
+__global__ void __launch_bounds__(SC_THREADS, 4) k_build_m(
+    ScParams P0, CombStart cs, const float4 *__restrict__ comb, const int *__restrict__ nActivePtr, const float4 *__restrict__ mpos,
+    const int4 *__restrict__ minfo, const float4 *__restrict__ ppos_, uint32_t *__restrict__ pool, long long poolCap,
+    unsigned long long *__restrict__ poolUsed, long long *__restrict__ warpOff, uint32_t *scratch,
+    int *__restrict__ cnt, int *__restrict__ perm, int cap, int *__restrict__ ovf, int *__restrict__ ovfCount,
+    int *__restrict__ ovfN) {
+    __shared__ ScanWords W;
+    build_m_block<LEAN, BATCH>(P0, W, blockIdx.x, cs, comb, nActivePtr, mpos, minfo, ppos_, pool, poolCap, poolUsed,
+                               warpOff, scratch, cnt, perm, cap, ovf, ovfCount, ovfN);
 }
 
 
@@ -2243,19 +2257,13 @@ __global__ void __launch_bounds__(SC_THREADS) k_lipid_select(const int *__restri
 }
 
 template <bool BATCH>
-__global__ void __launch_bounds__(SC_THREADS, 4) k_build_lm(ScParams P0, const uint32_t *__restrict__ cellStartM,
-                                                         const int *__restrict__ lipids,
-                                                         const int *__restrict__ lipidCount,
-                                                         const int4 *__restrict__ pinfo,
-                                                         const float4 *__restrict__ ppos_,
-                                                         const float4 *__restrict__ mpos, const int4 *__restrict__ minfo,
-                                                         uint4 *__restrict__ pool, long long poolCap,
-                                                         unsigned long long *__restrict__ poolUsed,
-                                                         long long *__restrict__ warpOff,
-                                                         uint32_t *scratch, int *__restrict__ cnt,
-                                                         int *__restrict__ perm, int cap) {
-    __shared__ ScanWords W;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void build_lm_block(
+    const ScParams &P0, ScanWords &W, int block, const uint32_t *__restrict__ cellStartM, const int *__restrict__ lipids,
+    const int *__restrict__ lipidCount, const int4 *__restrict__ pinfo, const float4 *__restrict__ ppos_,
+    const float4 *__restrict__ mpos, const int4 *__restrict__ minfo, uint4 *__restrict__ pool, long long poolCap,
+    unsigned long long *__restrict__ poolUsed, long long *__restrict__ warpOff, uint32_t *scratch,
+    int *__restrict__ cnt, int *__restrict__ perm, int cap) {
+    const int t = block * SC_THREADS + threadIdx.x;
     const bool valid = t < *lipidCount;
     int c = 0;
     if (valid) {
@@ -2263,7 +2271,7 @@ __global__ void __launch_bounds__(SC_THREADS, 4) k_build_lm(ScParams P0, const u
         rep_apply<BATCH>(P, pinfo[lipids[t]].w);
         build_lm_item(P, W, cellStartM, lipids[t], ppos_, mpos, minfo, scratch, c);
     }
-    const PoolSlot<uint4> S = pool_take<SC_LIST_LM>(P0, valid, c, pool, poolCap, poolUsed, warpOff, cnt, perm, cap,
+    const PoolSlot<uint4> S = pool_take<SC_LIST_LM>(P0, block, valid, c, pool, poolCap, poolUsed, warpOff, cnt, perm, cap,
                                                     nullptr, nullptr, lipids);
     if (S.n == 0) return;
     ScParams P = P0;
@@ -2289,6 +2297,49 @@ __global__ void __launch_bounds__(SC_THREADS, 4) k_build_lm(ScParams P0, const u
             S.out[(size_t)(k0 + q) * 32] = make_uint4(j[q], __float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(a.z));
         }
     }
+}
+
+template <bool BATCH>
+__global__ void __launch_bounds__(SC_THREADS, 4) k_build_lm(
+    ScParams P0, const uint32_t *__restrict__ cellStartM, const int *__restrict__ lipids,
+    const int *__restrict__ lipidCount, const int4 *__restrict__ pinfo, const float4 *__restrict__ ppos_,
+    const float4 *__restrict__ mpos, const int4 *__restrict__ minfo, uint4 *__restrict__ pool, long long poolCap,
+    unsigned long long *__restrict__ poolUsed, long long *__restrict__ warpOff, uint32_t *scratch,
+    int *__restrict__ cnt, int *__restrict__ perm, int cap) {
+    __shared__ ScanWords W;
+    build_lm_block<BATCH>(P0, W, blockIdx.x, cellStartM, lipids, lipidCount, pinfo, ppos_, mpos, minfo, pool, poolCap,
+                          poolUsed, warpOff, scratch, cnt, perm, cap);
+}
+
+// The three lists of the relaxation in one launch, blocks of the metabolic
+// items first, then the lipids', then the particles': the lists read the same
+// positions and none of the others.  A sim that does not fill the device has
+// each build wait for its own few blocks' longest item (sc_phase_build_all).
+template <bool BATCH>
+__global__ void __launch_bounds__(SC_THREADS, 3) k_build_all(
+    ScParams P, int nbM, int nbLM, CombStart cs, const float4 *__restrict__ comb, const int *__restrict__ nActiveM,
+    const int *__restrict__ nActive, const float4 *__restrict__ mpos, const int4 *__restrict__ minfo,
+    const float4 *__restrict__ ppos_, const int4 *__restrict__ pinfo,
+    uint32_t *__restrict__ poolM, long long poolCapM, unsigned long long *__restrict__ poolUsedM,
+    long long *__restrict__ warpOffM, uint32_t *scratchM, int *__restrict__ cntM, int *__restrict__ permM,
+    int *__restrict__ ovfM, int *__restrict__ ovfCountM, int *__restrict__ ovfNM,
+    const int *__restrict__ lipids, const int *__restrict__ lipidCount, uint4 *__restrict__ poolLM, long long poolCapLM,
+    unsigned long long *__restrict__ poolUsedLM, long long *__restrict__ warpOffLM, uint32_t *scratchLM,
+    int *__restrict__ cntLM, int *__restrict__ permLM,
+    const int *__restrict__ nb, const int *__restrict__ bonds, uint32_t *__restrict__ list, int *__restrict__ cnt,
+    int *__restrict__ classIdx, int *__restrict__ classCount, int *__restrict__ ovf, int *__restrict__ ovfCount,
+    uint32_t *__restrict__ match, int *__restrict__ matchN, float4 *__restrict__ geo) {
+    __shared__ ScanWords W;
+    const int b = blockIdx.x;
+    if (b < nbM)
+        build_m_block<false, BATCH>(P, W, b, cs, comb, nActiveM, mpos, minfo, ppos_, poolM, poolCapM, poolUsedM,
+                                    warpOffM, scratchM, cntM, permM, P.Nm, ovfM, ovfCountM, ovfNM);
+    else if (b < nbM + nbLM)
+        build_lm_block<BATCH>(P, W, b - nbM, cs.m, lipids, lipidCount, pinfo, ppos_, mpos, minfo, poolLM, poolCapLM,
+                              poolUsedLM, warpOffLM, scratchLM, cntLM, permLM, P.N);
+    else
+        build_pp_block<BATCH>(P, W, b - nbM - nbLM, cs.p, nActive, ppos_, pinfo, nb, bonds, list, cnt, P.N, classIdx,
+                              classCount, ovf, ovfCount, match, matchN, geo);
 }
 
 // metabolites.cuh:267-340 for one lipid: each listed metabolic neighbour
@@ -3582,6 +3633,45 @@ static void ensure_pp(ScLaunchCtx &c) {
     B.relaxAge = B.noiseAge = 0;
 }
 
+// Every list of the relaxation in one launch (k_build_all), where none is built
+// and the blocks fit the device at four per SM.  A launch each and so, ten
+// steps: 4,096 + 8,192 items 7.7 / 6.9 ms, 38,000 + 76,000 10.4 / 9.5; with four
+// sims in flight 2.35 / 2.10 and 5.88 / 5.74, but 65,536 + 131,072 6.82 / 6.91.
+// Streams of their own beside the noise phases gain as much for one sim and
+// lose for several (4,096, four in flight: 2.9 ms).
+void sc_phase_build_all(ScLaunchCtx &c) {
+    ScBuffers &B = *c.B;
+    const int nbP = nblocks(c.P.N), nbM = nblocks(c.P.Nm);
+    if (c.P.N <= 0 || c.P.Nm <= 0 || nbM + 2 * nbP > c.gridCap / 2 || c.P.tileCapM > 0 || c.P.metabLean ||
+        !B.scratchApart || B.validPP || B.validM || B.validLM)
+        return;
+    MFields M = B.M();
+    PFields F = B.P();
+    // every counter of the lists: the diffusion's too, which the builds' scratch invalidates
+    cudaMemsetAsync(B.ctr->ppClassCount, 0, sizeof(ScCounters) - offsetof(ScCounters, ppClassCount), c.st);
+    const CombStart cs{B.cellStartM, B.cellStartP};
+    k_combine<<<(int)std::min<long long>(((long long)c.P.N + c.P.Nm + SC_THREADS - 1) / SC_THREADS, 8 * c.gridCap),
+                SC_THREADS, 0, c.st>>>(c.P, B.keysM[B.sortCurM], B.keysP[B.sortCurP], cs, M.pos, M.info, F.pos, F.info,
+                                       B.comb);
+    k_lipid_select<<<nbP, SC_THREADS, 0, c.st>>>(&B.ctr->nActive, F.info, B.workP, &B.ctr->workCount);
+    SC_BATCHED(k_build_all)<<<nbM + 2 * nbP, SC_THREADS, 0, c.st>>>(
+        c.P, nbM, nbP, cs, B.comb, &B.ctr->nActiveM, &B.ctr->nActive, M.pos, M.info, F.pos, F.info,
+        B.listM, (long long)B.poolCapM, &B.ctr->poolM, B.warpOffM, B.listD, B.cntM, B.permM, B.ovfM, &B.ctr->ovfM, B.ovfNM,
+        B.workP, &B.ctr->workCount, reinterpret_cast<uint4 *>(B.listLM),
+        (long long)(sc_list_words(SC_LIST_LM, c.P.N) / 4), &B.ctr->poolLM, B.warpOffLM, B.scratchLM, B.cntLM, B.permLM,
+        F.nb, F.bonds, B.listPP, B.cntPP, B.classPP, B.ctr->ppClassCount, B.ovfPP, &B.ctr->ovfPP, B.matchPP, B.matchN,
+        B.geoPP);
+    k_bond_plan<<<std::min(nbP, c.gridCap), SC_THREADS, 0, c.st>>>(
+        c.P, pp_list(c), B.classPP, B.ctr->ppClassCount, F.bonds, B.matchPP, B.matchN, B.bondRec);
+    SC_BATCHED(k_build_m_ovf)<<<std::min(nbM, c.gridCap / 4), SC_THREADS, 0, c.st>>>(
+        c.P, B.cellStartM, B.cellStartP, M.pos, M.info, F.pos, F.info, B.ovfM, &B.ctr->ovfM, B.ovfNM, B.ovfOffM,
+        B.ovfPoolM, (long long)B.ovfPoolCapM, &B.ctr->poolOvfM);
+    (*c.launches) += 5;
+    B.validPP = B.validM = B.validLM = true;
+    B.validD = false;
+    B.relaxAge = B.noiseAge = 0;
+}
+
 void sc_phase_coordinate_noise(ScLaunchCtx &c, float frac) {
     ScBuffers &B = *c.B;
     if (c.P.N <= 0) return;
@@ -3752,7 +3842,7 @@ void sc_phase_build_lm(ScLaunchCtx &c) {
     MFields M = B.M();
     PFields F = B.P();
     if (!B.validLM) {
-        if (B.scratchLM == B.listD) B.validD = false;
+        if (B.scratchInD) B.validD = false;
         cudaMemsetAsync(&B.ctr->poolLM, 0, sizeof(B.ctr->poolLM) + sizeof(B.ctr->workCount), c.st);
         k_lipid_select<<<nblocks(c.P.N), SC_THREADS, 0, c.st>>>(&B.ctr->nActive, F.info, B.workP, &B.ctr->workCount);
         SC_BATCHED(k_build_lm)<<<nblocks(c.P.N), SC_THREADS, 0, c.st>>>(
