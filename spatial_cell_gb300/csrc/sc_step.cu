@@ -1831,16 +1831,13 @@ __device__ __noinline__ void relax_metab_overflow(const ScParams &P, const Relax
 // G = 4 keeps four blocks per SM for sims that fill the device, where the
 // pool's stream from HBM bounds the launch; G = 8 halves the rounds of sims
 // that do not, where the rounds' latency does.
+//
+// At G = 4 a block's warps take its 32-item groups as they come free: the lists
+// of every 256 items are ranked by length, so of a warp to a group the later
+// ones would wait, their registers held, for the first.  sc_phase_relax_metab
+// chooses how many groups a block has.
 template <int G, bool BATCH>
-__global__ void __launch_bounds__(SC_THREADS, G == 4 ? 4 : 2) k_relax_metab(ScParams P, RelaxMArgs A, int extra) {
-    if constexpr (G == 8) {
-        __shared__ float sTerm[SC_THREADS / 32][32][SC_TERM_ROW];
-        if ((int)blockIdx.x < extra) {
-            if (*A.ovfCount > 0) relax_metab_overflow<BATCH>(P, A, blockIdx.x, extra, sTerm);
-            return;
-        }
-    }
-    const int g = ((int)blockIdx.x - extra) * SC_THREADS + threadIdx.x;   // list position (count-ordered)
+__device__ __forceinline__ void relax_metab_item(const ScParams &P, const RelaxMArgs &A, int g) {
     if (g >= *A.nActivePtr) return;
     const int i = A.L.perm[g], c = A.L.cnt[g];
     const uint4 *pairs = A.pool + A.warpOff[g >> 5] + (g & 31);
@@ -1878,6 +1875,29 @@ __global__ void __launch_bounds__(SC_THREADS, G == 4 ? 4 : 2) k_relax_metab(ScPa
         }
     }
     st3(A.mvelOut, i, pv + dV / fmaxf(w, 1.0f), v4.w);
+}
+template <int G, bool BATCH>
+__global__ void __launch_bounds__(SC_THREADS, G == 4 ? 4 : 2) k_relax_metab(ScParams P, RelaxMArgs A, int extra,
+                                                                            int groups) {
+    if constexpr (G == 8) {
+        __shared__ float sTerm[SC_THREADS / 32][32][SC_TERM_ROW];
+        if ((int)blockIdx.x < extra) {
+            if (*A.ovfCount > 0) relax_metab_overflow<BATCH>(P, A, blockIdx.x, extra, sTerm);
+            return;
+        }
+        relax_metab_item<G, BATCH>(P, A, ((int)blockIdx.x - extra) * SC_THREADS + threadIdx.x);   // groups = 8
+    } else {
+        __shared__ int s_next;
+        if (threadIdx.x == 0) s_next = SC_THREADS / 32;
+        __syncthreads();
+        const int lane = threadIdx.x & 31;
+        for (int q = threadIdx.x >> 5; q < groups;) {
+            relax_metab_item<G, BATCH>(P, A, ((int)blockIdx.x * groups + q) * 32 + lane);
+            int n = 0;
+            if (lane == 0) n = atomicAdd(&s_next, 1);
+            q = __shfl_sync(0xffffffffu, n, 0);
+        }
+    }
 }
 
 // The lean pool's sweep: per pair the neighbour's position and velocity are
@@ -3817,14 +3837,22 @@ void sc_phase_relax_metab(ScLaunchCtx &c) {
         SC_BATCHED(k_relax_metab_overflow)<<<std::min(nb, c.gridCap / 4), SC_THREADS, 0, c.st>>>(c.P, A);
         (*c.launches) += 3;
     } else {
+        // 256 items times this a block of the sweep: up to eight where that
+        // leaves four waves of blocks (8,388,608 items 414 us a launch at one,
+        // 386 at four, 383 at eight), one below, where fewer blocks than the
+        // device holds cost more (500,009 items, five steps: 11.9 ms at one,
+        // 12.4 at four)
+        const int sweep = std::max(1, std::min(8, nb / (2 * c.gridCap)));
         const bool batch = c.P.nRep > 1, small = nb <= c.gridCap / 4;   // at most two blocks per SM: all resident at G = 8
         const int extra = small || c.P.metabLean ? std::min(nb, c.gridCap / 2) : 0;
         if (c.P.metabLean)
             SC_BATCHED(k_relax_metab_lean)<<<extra + nb, SC_THREADS, 0, c.st>>>(c.P, A, extra);
         else if (small)
-            (batch ? k_relax_metab<8, true> : k_relax_metab<8, false>)<<<extra + nb, SC_THREADS, 0, c.st>>>(c.P, A, extra);
+            (batch ? k_relax_metab<8, true> : k_relax_metab<8, false>)<<<extra + nb, SC_THREADS, 0, c.st>>>(c.P, A, extra,
+                                                                                                          8);
         else
-            (batch ? k_relax_metab<4, true> : k_relax_metab<4, false>)<<<nb, SC_THREADS, 0, c.st>>>(c.P, A, 0);
+            (batch ? k_relax_metab<4, true> : k_relax_metab<4, false>)<<<(nb + sweep - 1) / sweep, SC_THREADS, 0,
+                                                                         c.st>>>(c.P, A, 0, 8 * sweep);
         (*c.launches)++;
         if (!extra) {
             SC_BATCHED(k_relax_metab_overflow)<<<std::min(nb, c.gridCap), SC_THREADS, 0, c.st>>>(c.P, A);
