@@ -86,7 +86,7 @@ struct ScCounters {
     int polyConflict; // 1: an item holds two bonds of its rule's group (k_poly_plan)
     int step;         // the step loop counter (main.cu:347)
     // what one builder resets lies together, so one memset resets it
-    int tileCounter[4];   // k_onesweep, per pass
+    int tileCounter[8];   // k_onesweep, per item set and pass
     int farMove;          // a metabolic item moved more than a cell along an axis since its sort
     int ppClassCount[4];  // items per relax work class (k_build_pp); [3]: RelaxArgs::unsettled
     int ovfPP;            // items whose particle list overflowed (k_build_pp)

@@ -39,6 +39,13 @@ __device__ __forceinline__ void st_relaxed(uint32_t *p, uint32_t v) {
     asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// The sets one launch sorts, grid y being the set: both of a small sim, whose
+// passes are as long as one tile's latency, or one.
+struct SortPair {
+    ScSortSet s[2];
+};
+__host__ __device__ static inline size_t sort_tiles(long long n, int ipt) { return (size_t)((n + SC_THREADS * ipt - 1) / (SC_THREADS * ipt)); }
+
 // In a batched sim the key is the item's replica's key base plus its cell
 // in that replica's grid: replicas sort into consecutive key ranges.
 //
@@ -47,20 +54,24 @@ __device__ __forceinline__ void st_relaxed(uint32_t *p, uint32_t v) {
 // at one item, 6.1 us at four.  The kernel also clears what the passes behind it look at first (the look-back words and
 // tile counters) and farMove.
 template <bool BATCH, int KEYS>
-__global__ void __launch_bounds__(SC_THREADS) k_sort_keys(const float4 *__restrict__ pos, const int4 *__restrict__ info,
-                                                          int n, ScParams P, uint32_t inactiveKey, int passes,
-                                                          uint32_t *__restrict__ keys, uint32_t *__restrict__ hist,
-                                                          uint32_t *__restrict__ lookback, int lbWords, ScCounters *ctr) {
+__global__ void __launch_bounds__(SC_THREADS) k_sort_keys(SortPair sets, ScParams P, uint32_t inactiveKey, int passes,
+                                                          int ipt, ScCounters *ctr) {
     __shared__ uint32_t sh[4 * 256];
+    const ScSortSet &S = sets.s[blockIdx.y];
+    const int n = S.n, blocks = (int)sort_tiles(n, KEYS), lbWords = passes * (int)sort_tiles(n, ipt) * 256;
+    if ((int)blockIdx.x >= blocks) return;
+    const float4 *__restrict__ pos = S.pos;
+    const int4 *__restrict__ info = S.info;
+    uint32_t *__restrict__ keys = S.keys[0], *__restrict__ hist = S.hist;
     for (int t = threadIdx.x; t < passes * 256; t += blockDim.x) sh[t] = 0;
     __syncthreads();
-    const int first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    const int first = blockIdx.x * blockDim.x + threadIdx.x, stride = blocks * SC_THREADS;
     int4 in[KEYS];
     sc_f3 p[KEYS];
 #pragma unroll
     for (int r = 0; r < KEYS; r++) {
         const int i = min(first + r * stride, n - 1);
-        in[r] = info[i];
+        in[r] = __ldg(info + i);
         p[r] = ld3(pos, i);
     }
 #pragma unroll
@@ -77,8 +88,8 @@ __global__ void __launch_bounds__(SC_THREADS) k_sort_keys(const float4 *__restri
         keys[i] = k;
         for (int d = 0; d < passes; d++) atomicAdd(&sh[d * 256 + ((k >> (8 * d)) & 0xffu)], 1u);
     }
-    for (int w = first; w < lbWords; w += stride) lookback[w] = 0;
-    if (first < 4) ctr->tileCounter[first] = 0;
+    for (int w = first; w < lbWords; w += stride) S.lookback[w] = 0;
+    if (first < 4) S.tileCounter[first] = 0;
     if (first == 4) ctr->farMove = 0;
     __syncthreads();
     for (int t = threadIdx.x; t < passes * 256; t += blockDim.x)
@@ -106,18 +117,20 @@ __device__ __forceinline__ uint32_t block_exclusive_scan256(uint32_t v, uint32_t
 // looked back at a time, a pass over 262,144 keys takes 9.7 us, 14.4 with a
 // block-wide round per 256 keys and a tile at a time.
 template <int IPT>
-__global__ void __launch_bounds__(SC_THREADS) k_onesweep(const uint32_t *__restrict__ keysIn,
-                                                         const uint32_t *__restrict__ valsIn,
-                                                         uint32_t *__restrict__ keysOut, uint32_t *__restrict__ valsOut,
-                                                         int n, int shift, const uint32_t *__restrict__ hist,
-                                                         uint32_t *__restrict__ lookback, int *tileCounter,
-                                                         ScCounters *ctr) {
+__global__ void __launch_bounds__(SC_THREADS) k_onesweep(SortPair sets, int pass, ScCounters *ctr) {
+    const ScSortSet &S = sets.s[blockIdx.y];
+    const int n = S.n, tiles = (int)sort_tiles(n, IPT), shift = 8 * pass;
+    if ((int)blockIdx.x >= tiles) return;
+    const uint32_t *__restrict__ keysIn = S.keys[pass & 1], *__restrict__ valsIn = pass ? S.vals[pass & 1] : nullptr;
+    uint32_t *__restrict__ keysOut = S.keys[~pass & 1], *__restrict__ valsOut = S.vals[~pass & 1];
+    const uint32_t *__restrict__ hist = S.hist + 256 * pass;
+    uint32_t *lookback = S.lookback + (size_t)pass * tiles * 256;
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_cnt[8][256];   // a warp's keys per digit so far; then its first key's rank
     __shared__ uint32_t s_base[256];
     __shared__ uint32_t s_wsum[8];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0) s_tile = (uint32_t)atomicAdd(tileCounter, 1);
+    if (tid == 0) s_tile = (uint32_t)atomicAdd(&S.tileCounter[pass], 1);
 #pragma unroll
     for (int w = 0; w < 8; w++) s_cnt[w][tid] = 0;
     __syncthreads();
@@ -130,8 +143,8 @@ __global__ void __launch_bounds__(SC_THREADS) k_onesweep(const uint32_t *__restr
     for (int r = 0; r < IPT; r++) {
         long long idx = base + r * 32;
         if (idx < n) {
-            key[r] = keysIn[idx];
-            val[r] = valsIn ? valsIn[idx] : (uint32_t)idx;
+            key[r] = __ldg(keysIn + idx);
+            val[r] = valsIn ? __ldg(valsIn + idx) : (uint32_t)idx;
         } else {
             key[r] = 0;
             val[r] = 0;
@@ -208,17 +221,20 @@ __global__ void __launch_bounds__(SC_THREADS) k_onesweep(const uint32_t *__restr
 
 // cellStart[c] = first sorted slot whose key >= c, for c in [0, cells];
 // inactive keys (>= cells) count as cells.  One binary search per cell.
-__global__ void k_cell_start(const uint32_t *__restrict__ keys, int n, uint32_t cells, uint32_t *__restrict__ cellStart) {
+__global__ void k_cell_start(SortPair sets, int cur, uint32_t cells) {
+    const ScSortSet &S = sets.s[blockIdx.y];
+    const uint32_t *__restrict__ keys = S.keys[cur];
+    const int n = S.n;
     long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c > (long long)cells) return;
     int lo = 0, hi = n;
     while (lo < hi) {
         int mid = (int)(((unsigned)lo + (unsigned)hi) >> 1);
-        uint32_t k = keys[mid];
+        uint32_t k = __ldg(keys + mid);
         if ((long long)k < c) lo = mid + 1;
         else hi = mid;
     }
-    cellStart[c] = (uint32_t)lo;
+    S.cellStart[c] = (uint32_t)lo;
 }
 
 // The gathers load every field of the source slot before storing any: the
@@ -288,58 +304,51 @@ int sc_sort_passes_for(const ScParams &P) { return ((P.keyBits > 0 ? P.keyBits :
 // (a whole sort of 32,768 items 61 us at sixteen, 52 at eight, 49 at four;
 // 131,072: 74, 63, 63; 200,000: 75, 66, 74); past an SM each there is nothing
 // left to gain (262,144: 75, 74, 75) and fewer tiles look back less.
-static size_t sort_tiles(long long n, int ipt) { return (size_t)((n + SC_THREADS * ipt - 1) / (SC_THREADS * ipt)); }
 static int sort_ipt(long long n) {
     return sort_tiles(n, 4) <= SORT_SMS ? 4 : sort_tiles(n, 8) <= SORT_SMS ? 8 : SORT_IPT;
 }
+
 
 // Words of one pass's look-back table for up to cap items, whatever their number.
 size_t sc_sort_lookback_words(int cap) {
     return std::max<size_t>(std::min<size_t>(sort_tiles(cap, 4), SORT_SMS), sort_tiles(cap, SORT_IPT)) * 256;
 }
 
-// Sorts the keys of one item set; returns the buffer index (0/1) holding the
-// sorted keys and the permutation.  hist: 4*256 words, lookback: per pass.
-int sc_launch_sort(cudaStream_t st, const float4 *pos, const int4 *info, int n, const ScParams &P,
-                   uint32_t *keys[2], uint32_t *vals[2], uint32_t *hist, uint32_t *lookback, ScCounters *ctr,
+// Both sets of a sim are sorted by the same launches while either's tiles fit the
+// device at four keys a thread: 4,096 + 8,192 items, ten steps 6.94 / 6.76 ms,
+// four sims in flight 2.10 / 2.06; 65,536 + 131,072 12.4 / 12.3.
+bool sc_sort_together(int n, int m) { return n > 0 && m > 0 && sort_ipt(std::max(n, m)) == 4; }
+
+// Sorts the keys of one item set or two (sc_sort_together) and finds their
+// cells' starts; returns the buffer index (0/1) holding the sorted keys and the
+// permutations.
+int sc_launch_sort(cudaStream_t st, const ScSortSet *sets, int count, const ScParams &P, ScCounters *ctr,
                    long long *launches) {
     int passes = sc_sort_passes_for(P);
     int keyBits = P.keyBits > 0 ? P.keyBits : 3 * P.bits + 1;
     uint32_t inactiveKey = keyBits >= 32 ? 0xffffffffu : ((1u << keyBits) - 1u);
-    const int ipt = sort_ipt(n);
-    const int tiles = (int)sort_tiles(n, ipt);
+    const SortPair pair{{sets[0], sets[count - 1]}};
+    const int n = std::max(pair.s[0].n, pair.s[1].n), ipt = sort_ipt(n);
     auto *const pass = ipt == 4 ? k_onesweep<4> : ipt == 8 ? k_onesweep<8> : k_onesweep<SORT_IPT>;
-    const size_t lbWords = (size_t)tiles * 256;
-    cudaMemsetAsync(hist, 0, 4 * 256 * sizeof(uint32_t), st);
+    for (int k = 0; k < count; k++) cudaMemsetAsync(sets[k].hist, 0, 4 * 256 * sizeof(uint32_t), st);
     if (n > 0) {
-        const bool one = (n + SC_THREADS - 1) / SC_THREADS <= SORT_SMS;
-        const int per = SC_THREADS * (one ? 1 : SORT_KEYS), blocks = (int)(((long long)n + per - 1) / per);
+        const bool one = sort_tiles(n, 1) <= SORT_SMS;
         auto *const make = P.nRep > 1 ? (one ? k_sort_keys<true, 1> : k_sort_keys<true, SORT_KEYS>)
                                       : (one ? k_sort_keys<false, 1> : k_sort_keys<false, SORT_KEYS>);
-        make<<<blocks, SC_THREADS, 0, st>>>(pos, info, n, P, inactiveKey, passes, keys[0], hist, lookback,
-                                            (int)(passes * lbWords), ctr);
-        (*launches)++;
+        make<<<dim3((unsigned)sort_tiles(n, one ? 1 : SORT_KEYS), count), SC_THREADS, 0, st>>>(pair, P, inactiveKey,
+                                                                                              passes, ipt, ctr);
+        for (int d = 0; d < passes; d++)
+            pass<<<dim3((unsigned)sort_tiles(n, ipt), count), SC_THREADS, 0, st>>>(pair, d, ctr);
+        (*launches) += 1 + passes;
     } else {
         // the tile counters and farMove behind them
         cudaMemsetAsync(ctr->tileCounter, 0, sizeof(ctr->tileCounter) + sizeof(ctr->farMove), st);
     }
-    int cur = 0;
-    for (int d = 0; d < passes && n > 0; d++) {
-        pass<<<tiles, SC_THREADS, 0, st>>>(keys[cur], d == 0 ? nullptr : vals[cur], keys[1 - cur], vals[1 - cur], n,
-                                           8 * d, hist + 256 * d, lookback + (size_t)d * lbWords,
-                                           &ctr->tileCounter[d], ctr);
-        (*launches)++;
-        cur = 1 - cur;
-    }
-    return cur;
-}
-
-void sc_launch_cell_start(cudaStream_t st, const uint32_t *keys, int n, uint32_t cells, uint32_t *cellStart,
-                          long long *launches) {
-    long long total = (long long)cells + 1;
-    int blocks = (int)((total + SC_THREADS - 1) / SC_THREADS);
-    k_cell_start<<<blocks, SC_THREADS, 0, st>>>(keys, n, cells, cellStart);
+    const int cur = n > 0 ? passes & 1 : 0;
+    const unsigned blocks = (unsigned)(((long long)P.cells + 1 + SC_THREADS - 1) / SC_THREADS);
+    k_cell_start<<<dim3(blocks, count), SC_THREADS, 0, st>>>(pair, cur, P.cells);
     (*launches)++;
+    return cur;
 }
 
 void sc_launch_gather_particles(cudaStream_t st, const uint32_t *perm, int n, const PFields &src, const PFields &dst,

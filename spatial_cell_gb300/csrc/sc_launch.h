@@ -41,7 +41,7 @@ struct ScBuffers {
     int *mcFlag;   // device word of k_mc_scan
     // binning: keys / slot values ping-pong per item set, the buffer of the
     // last pass holding the sorted keys and the permutation
-    uint32_t *keysP[2], *valsP[2], *keysM[2], *valsM[2], *hist, *lookback;
+    uint32_t *keysP[2], *valsP[2], *keysM[2], *valsM[2], *hist, *lookback, *lookbackM;
     int sortCurP, sortCurM;
     uint32_t *cellStartP, *cellStartM;
     // pair lists (sc_dev.cuh) and whether each matches the current state
@@ -173,10 +173,19 @@ struct ScBuffers {
 int sc_sort_passes(int bits);
 int sc_sort_passes_for(const ScParams &P);  // passes over P's key bits
 size_t sc_sort_lookback_words(int cap);
-int sc_launch_sort(cudaStream_t st, const float4 *pos, const int4 *info, int n, const ScParams &P, uint32_t *keys[2],
-                   uint32_t *vals[2], uint32_t *hist, uint32_t *lookback, ScCounters *ctr, long long *launches);
-void sc_launch_cell_start(cudaStream_t st, const uint32_t *keys, int n, uint32_t cells, uint32_t *cellStart,
-                          long long *launches);
+// One item set to sort: keys and vals ping-pong, hist 4*256 words, lookback
+// sc_sort_lookback_words(n) per pass, four tile counters, cells + 1 starts.
+struct ScSortSet {
+    const float4 *pos;
+    const int4 *info;
+    int n;
+    uint32_t *keys[2], *vals[2], *hist, *lookback;
+    int *tileCounter;
+    uint32_t *cellStart;
+};
+bool sc_sort_together(int n, int m);
+int sc_launch_sort(cudaStream_t st, const ScSortSet *sets, int count, const ScParams &P, ScCounters *ctr,
+                   long long *launches);
 void sc_launch_gather_particles(cudaStream_t st, const uint32_t *perm, int n, const PFields &src, const PFields &dst,
                                 long long *launches);
 void sc_launch_gather_metabolic(cudaStream_t st, const uint32_t *perm, int n, int sp4, ScBuffers &B,

@@ -79,9 +79,9 @@ extern "C" int sc_sort_cells_static(const sc_config *cfg, const void *pos, const
     long long launches = 0;
     if (sc_sort_lookback_words(SC_STATIC_SORT_MAX_ITEMS) > (size_t)SC_STATIC_SORT_TILES * 256) return SC_E_INVALID;
     if (cudaMemsetAsync(ctr, 0, sizeof(ScCounters), st) != cudaSuccess) return SC_E_CUDA;
-    int cur = sc_launch_sort(st, (const float4 *)pos, (const int4 *)info, n, P, keys, vals, hist, lookback, ctr,
-                             &launches);
-    sc_launch_cell_start(st, keys[cur], n, P.cells, cell_start, &launches);
+    const ScSortSet set{(const float4 *)pos, (const int4 *)info, n, {keys[0], keys[1]}, {vals[0], vals[1]},
+                        hist, lookback, ctr->tileCounter, cell_start};
+    const int cur = sc_launch_sort(st, &set, 1, P, ctr, &launches);
     if (n > 0 && cudaMemcpyAsync(perm, vals[cur], (size_t)n * 4, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
         return SC_E_CUDA;
     cudaError_t e = cudaGetLastError();

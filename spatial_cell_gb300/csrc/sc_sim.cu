@@ -397,27 +397,42 @@ int check_launch(sc_sim *s) {
     return SC_OK;
 }
 
-void sort_particles(sc_sim *s) {
+ScSortSet sort_set(sc_sim *s, bool metabolic) {
+    ScBuffers &B = s->B;
+    if (!metabolic) {
+        const PFields F = B.P();
+        return {F.pos, F.info, s->P.N, {B.keysP[0], B.keysP[1]}, {B.valsP[0], B.valsP[1]},
+                B.hist, B.lookback, B.ctr->tileCounter, B.cellStartP};
+    }
+    const MFields F = B.M();
+    return {F.pos, F.info, s->P.Nm, {B.keysM[0], B.keysM[1]}, {B.valsM[0], B.valsM[1]},
+            B.hist + 4 * 256, B.lookbackM, B.ctr->tileCounter + 4, B.cellStartM};
+}
+
+void gather_particles(sc_sim *s, int cur) {
     ScBuffers &B = s->B;
     const int N = s->P.N;
-    PFields F = B.P();
-    int cur = sc_launch_sort(s->st, F.pos, F.info, N, s->P, B.keysP, B.valsP, B.hist, B.lookback, B.ctr, &s->launches);
     B.sortCurP = cur;
-    sc_launch_cell_start(s->st, B.keysP[cur], N, s->P.cells, B.cellStartP, &s->launches);
     sc_launch_gather_particles(s->st, B.valsP[cur], N, B.P(), B.Pnext(), &s->launches);
     B.flipAllP();
     k_mark_lipids<<<std::max(nb_of(N), 1), SC_THREADS, 0, s->st>>>(B.ctr, N, B.P().info, B.lipidP);
     s->launches++;
 }
 
-void sort_metabolic(sc_sim *s) {
+void gather_metabolic(sc_sim *s, int cur) {
     ScBuffers &B = s->B;
-    const int Nm = s->P.Nm;
-    MFields F = B.M();
-    int cur = sc_launch_sort(s->st, F.pos, F.info, Nm, s->P, B.keysM, B.valsM, B.hist, B.lookback, B.ctr, &s->launches);
     B.sortCurM = cur;
-    sc_launch_cell_start(s->st, B.keysM[cur], Nm, s->P.cells, B.cellStartM, &s->launches);
-    sc_launch_gather_metabolic(s->st, B.valsM[cur], Nm, s->P.SP / 4, B, &s->launches);
+    sc_launch_gather_metabolic(s->st, B.valsM[cur], s->P.Nm, s->P.SP / 4, B, &s->launches);
+}
+
+void sort_particles(sc_sim *s) {
+    const ScSortSet set = sort_set(s, false);
+    gather_particles(s, sc_launch_sort(s->st, &set, 1, s->P, s->B.ctr, &s->launches));
+}
+
+void sort_metabolic(sc_sim *s) {
+    const ScSortSet set = sort_set(s, true);
+    gather_metabolic(s, sc_launch_sort(s->st, &set, 1, s->P, s->B.ctr, &s->launches));
 }
 
 // Which pair lists a phase invalidates (it changes positions, flags, types,
@@ -522,11 +537,27 @@ int run_phase(sc_sim *s, int phase, int arg) {
     return check_launch(s);
 }
 
+// Both sort phases, in the same launches where that pays.
+void sort_sets(sc_sim *s) {
+    if (!sc_sort_together(s->P.N, s->P.Nm)) {
+        run_phase(s, SC_PHASE_SORT_PARTICLES, 0);
+        run_phase(s, SC_PHASE_SORT_METABOLIC, 0);
+        return;
+    }
+    for (int phase : {SC_PHASE_SORT_PARTICLES, SC_PHASE_SORT_METABOLIC}) {
+        invalidate_after(s->B, phase);
+        binned_after(s->P, phase);
+    }
+    const ScSortSet sets[2] = {sort_set(s, false), sort_set(s, true)};
+    const int cur = sc_launch_sort(s->st, sets, 2, s->P, s->B.ctr, &s->launches);
+    gather_particles(s, cur);
+    gather_metabolic(s, cur);
+}
+
 // One iteration of the step loop (main.cu:347-661), launched phase by phase.
 int step_direct(sc_sim *s) {
     const sc_config &c = s->cfg;
-    run_phase(s, SC_PHASE_SORT_PARTICLES, 0);
-    run_phase(s, SC_PHASE_SORT_METABOLIC, 0);
+    sort_sets(s);
     if (c.relaxation_steps > 0) {
         ScLaunchCtx all = ctx(s);
         sc_phase_build_all(all);
@@ -926,8 +957,9 @@ static int create_sim(const sc_config *cfg_in, const sc_replica *replicas, int32
     const int poolEntryWords = P.metabLean ? 1 : 4;
     size_t poolWords = sc_list_words(SC_LIST_M, (int)Nm);
     if (P.tileCapM == 0) poolWords = std::min(poolWords, sc_list_words(kPoolStart * poolEntryWords, (int)Nm));
-    if ((rc = dalloc(s, &B.mcFlag, 4)) || (rc = dalloc(s, &B.hist, 4 * 256)) ||
-        (rc = dalloc(s, &B.lookback, (size_t)passes * sc_sort_lookback_words((int)std::max(N, Nm)))) ||
+    if ((rc = dalloc(s, &B.mcFlag, 4)) || (rc = dalloc(s, &B.hist, 2 * 4 * 256)) ||
+        (rc = dalloc(s, &B.lookback, (size_t)passes * sc_sort_lookback_words((int)N))) ||
+        (rc = dalloc(s, &B.lookbackM, (size_t)passes * sc_sort_lookback_words((int)Nm))) ||
         (rc = dalloc(s, &B.cellStartP, (size_t)P.cells + 1)) || (rc = dalloc(s, &B.cellStartM, (size_t)P.cells + 1)) ||
         (rc = dalloc(s, &B.polyList, N)) || (rc = dalloc(s, &B.polyRank, N)) || (rc = dalloc(s, &B.polyPmi, N)) ||
         (rc = dalloc(s, &B.polyClaim, N)) || (rc = dalloc(s, &B.polyBlk, 2 * ((size_t)N / SC_THREADS + 1))) || (rc = dalloc(s, &B.ctr, 1)) || (rc = dalloc(s, &B.listPP, sc_list_words(SC_LIST_PP, (int)N))) ||

@@ -52,3 +52,21 @@ def test_sim_sort(product, n):
     key = _keys(before["pos"], before["flags"] & 1 != 0, box, 6.0, abi.grid_dims(cfg)[0])
     assert np.array_equal(perm, np.argsort(key, kind="stable"))
     sim.close()
+
+
+@pytest.mark.parametrize("n,nm", [(5, 155648), (155648, 300), (70000, 140000), (300, 155649)])
+def test_both_sets_of_a_step(product, n, nm):
+    """A step's sorts, in the same launches up to 155,648 items a set."""
+    box = float((max(n, nm) / 0.02) ** (1 / 3))
+    cfg = abi.make_config(num_particles=n, num_metabolic_particles=nm, sim_size=box, grid_cell_size=6.0,
+                          max_interaction_distance=5.5, max_diffusion_distance=6.0, num_metabolites=1, seed=1,
+                          noise_coordination_steps=0, relaxation_steps=0, metabolite_diffusion_steps=0)
+    sim = product.Simulation(cfg, scenes.baseline_types(), scenes.baseline_rules())
+    sim.generate_uniform(n, nm, (0, 1, 2, 3), (0.25,) * 4, 7)
+    before = sim.export_state()
+    sim.step(1)
+    for which, state in enumerate(before):
+        _, perm = sim.export_grid(which)
+        key = _keys(state["pos"], state["flags"] & 1 != 0, box, 6.0, abi.grid_dims(cfg)[0])
+        assert np.array_equal(perm, np.argsort(key, kind="stable"))
+    sim.close()
