@@ -761,7 +761,6 @@ static int create_sim(const sc_config *cfg_in, const sc_replica *replicas, int32
         for (int k = 0; k < 2 && e == cudaSuccess; k++) {
             e = cudaEventCreateWithFlags(&s->reduced[k], cudaEventDisableTiming);
             if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->copied[k], cudaEventDisableTiming);
-            if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->side[k], cudaStreamNonBlocking);
             if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->join[k], cudaEventDisableTiming);
         }
         if (e != cudaSuccess) {
@@ -794,6 +793,16 @@ static int create_sim(const sc_config *cfg_in, const sc_replica *replicas, int32
     // cross-stream joins (class_streams 1 / 3 overrides).
     s->forkClasses = cfg->class_streams == 0 ? (int64_t)P.N >= (int64_t)s->gridCap * SC_THREADS
                                              : cfg->class_streams > 1;
+    // Only then are the side streams created: streams beyond the device's eight
+    // connections make concurrent sims wait for one another (vesicle at 1/16,
+    // passes of several sims in flight 36.5 / 35.7 ms, with and without).
+    for (int k = 0; k < 2 && s->forkClasses; k++) {
+        const cudaError_t e = cudaStreamCreateWithFlags(&s->side[k], cudaStreamNonBlocking);
+        if (e != cudaSuccess) {
+            sc_destroy(s);
+            return set_err(nullptr, SC_E_CUDA, cudaGetErrorString(e));
+        }
+    }
     P.coordSteps = cfg->noise_coordination_steps;
     P.seed = cfg->seed;
     // pair_list_limit >= 0 caps the pair lists (tests use it to run the
