@@ -1906,13 +1906,20 @@ __global__ void __launch_bounds__(SC_THREADS, G == 4 ? 4 : 2) k_relax_metab(ScPa
 // periodic box is decided once per item (Imager), the collision distance per
 // neighbour kind (the lipids' and the metabolic items' radii are each one
 // value in practice, CollisionDistCache recomputes it when they are not).
+//
+// With OVF the first `extra` blocks take the overflowed items, in sims that do
+// not fill the device; in those that do, the walk's stack and shared memory
+// cost the sweep more than a launch (196,613 + 983,041 items, five steps 29.1 /
+// 27.3 ms with and without).
 #define SC_METAB_GROUP 4
-template <bool BATCH>
+template <bool BATCH, bool OVF>
 __global__ void __launch_bounds__(SC_THREADS, 4) k_relax_metab_lean(ScParams P, RelaxMArgs A, int extra) {
-    __shared__ float sTerm[SC_THREADS / 32][32][SC_TERM_ROW];
-    if ((int)blockIdx.x < extra) {
-        if (*A.ovfCount > 0) relax_metab_overflow<BATCH>(P, A, blockIdx.x, extra, sTerm);
-        return;
+    if constexpr (OVF) {
+        __shared__ float sTerm[SC_THREADS / 32][32][SC_TERM_ROW];
+        if ((int)blockIdx.x < extra) {
+            if (*A.ovfCount > 0) relax_metab_overflow<BATCH>(P, A, blockIdx.x, extra, sTerm);
+            return;
+        }
     }
     const int g = ((int)blockIdx.x - extra) * SC_THREADS + threadIdx.x;   // list position (count-ordered)
     if (g >= *A.nActivePtr) return;
@@ -3844,9 +3851,11 @@ void sc_phase_relax_metab(ScLaunchCtx &c) {
         // 12.4 at four)
         const int sweep = std::max(1, std::min(8, nb / (2 * c.gridCap)));
         const bool batch = c.P.nRep > 1, small = nb <= c.gridCap / 4;   // at most two blocks per SM: all resident at G = 8
-        const int extra = small || c.P.metabLean ? std::min(nb, c.gridCap / 2) : 0;
+        const int extra = small ? std::min(nb, c.gridCap / 2) : 0;
+        auto *const lean = batch ? (small ? k_relax_metab_lean<true, true> : k_relax_metab_lean<true, false>)
+                                 : (small ? k_relax_metab_lean<false, true> : k_relax_metab_lean<false, false>);
         if (c.P.metabLean)
-            SC_BATCHED(k_relax_metab_lean)<<<extra + nb, SC_THREADS, 0, c.st>>>(c.P, A, extra);
+            lean<<<extra + nb, SC_THREADS, 0, c.st>>>(c.P, A, extra);
         else if (small)
             (batch ? k_relax_metab<8, true> : k_relax_metab<8, false>)<<<extra + nb, SC_THREADS, 0, c.st>>>(c.P, A, extra,
                                                                                                           8);
