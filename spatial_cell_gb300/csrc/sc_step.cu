@@ -1910,10 +1910,12 @@ __global__ void __launch_bounds__(SC_THREADS, G == 4 ? 4 : 2) k_relax_metab(ScPa
 // With OVF the first `extra` blocks take the overflowed items, in sims that do
 // not fill the device; in those that do, the walk's stack and shared memory
 // cost the sweep more than a launch (196,613 + 983,041 items, five steps 29.1 /
-// 27.3 ms with and without).
-#define SC_METAB_GROUP 4
+// 27.3 ms with and without).  Waits for gathers bound the sweep, and its spills
+// did: two pairs at a time at three blocks per SM have none, 24.4 ms, against
+// 26.9 for four at four, 25.1 for four at three and 24.6 for two at four.
+#define SC_METAB_GROUP 2
 template <bool BATCH, bool OVF>
-__global__ void __launch_bounds__(SC_THREADS, 4) k_relax_metab_lean(ScParams P, RelaxMArgs A, int extra) {
+__global__ void __launch_bounds__(SC_THREADS, 3) k_relax_metab_lean(ScParams P, RelaxMArgs A, int extra) {
     if constexpr (OVF) {
         __shared__ float sTerm[SC_THREADS / 32][32][SC_TERM_ROW];
         if ((int)blockIdx.x < extra) {
