@@ -3456,9 +3456,13 @@ __global__ void __launch_bounds__(SC_THREADS) k_diffuse_pool(ScParams P, const i
 // kernel takes L1 from the gathers that bound it (large workload: 330 -> 361 us
 // a launch), while a sim that does not fill the device saves a launch.
 // Inactive items' amounts are copied until both buffers hold them (age:
-// launches since the amounts were last out of step).
+// launches since the amounts were last out of step).  Twelve amounts keep to
+// three blocks per SM without spills (983,041 items, 118 us a launch with four
+// rows in flight, 106 us with two at four blocks, 97 us so).  Eight and four
+// amounts fit as they are, in a loop of their own: written as one with the
+// twelve's, the eight's spills (8,388,608 items 334 -> 407 us).
 template <int SP, bool BATCH, bool POOL>
-__global__ void __launch_bounds__(SC_THREADS) k_diffuse(ScParams P, const uint32_t *__restrict__ cellStart,
+__global__ void __launch_bounds__(SC_THREADS, SP == 12 ? 3 : 0) k_diffuse(ScParams P, const uint32_t *__restrict__ cellStart,
                                                         const int *__restrict__ nActivePtr,
                                                         const float4 *__restrict__ pos, const int4 *__restrict__ info,
                                                         PairList<SC_LIST_D> L, const float4 *__restrict__ metIn,
@@ -3500,11 +3504,28 @@ __global__ void __launch_bounds__(SC_THREADS) k_diffuse(ScParams P, const uint32
     if (c <= min(SC_LIST_D, P.listLimit)) {
         const uint4 *__restrict__ chunks = sc_list4_chunks(L.list, SC_LIST_D, g);
         uint4 E = c > 0 ? chunks[0] : make_uint4(0, 0, 0, 0);
-        // four entries per list load; their amounts are gathered together and
-        // the next chunk of the list is loaded while this one is applied
+        // four entries per list load; their amounts are gathered together (two
+        // and two of twelve amounts, which would spill) and the next chunk of
+        // the list is loaded while this one is applied
         for (int k0 = 0; k0 < c; k0 += 4) {
             const uint4 En = k0 + 4 < c ? chunks[(size_t)(k0 / 4 + 1) * 32] : make_uint4(0, 0, 0, 0);
             const int e[4] = {(int)E.x, (int)E.y, (int)E.z, (int)E.w};
+            if constexpr (SP == 12) {
+#pragma unroll
+                for (int h = 0; h < 4; h += 2) {
+                    float4 v[2][Q];
+#pragma unroll
+                    for (int kk = 0; kk < 2; kk++)
+                        if (k0 + h + kk < c) met_row<Q>(metIn, e[h + kk], v[kk]);
+#pragma unroll
+                    for (int kk = 0; kk < 2; kk++) {
+                        if (k0 + h + kk >= c) break;
+                        diffuse_term<SP>(v[kk], pm, dm, S);
+                    }
+                }
+                E = En;
+                continue;
+            }
             float4 v[4][Q];
 #pragma unroll
             for (int kk = 0; kk < 4; kk++)
