@@ -365,6 +365,10 @@ int dalloc(sc_sim *s, T **p, size_t count) {
 
 inline int nb_of(long long n) { return (int)((n + SC_THREADS - 1) / SC_THREADS); }
 
+// Whether a step may meet a scheduled polymerisation: by the rules, or because
+// the loaded state holds one.
+bool may_polymerize(const sc_sim *s) { return s->rulesPolymerize || s->loadScheduled; }
+
 ScLaunchCtx ctx(sc_sim *s) {
     ScLaunchCtx c;
     c.st = s->st;
@@ -372,7 +376,7 @@ ScLaunchCtx ctx(sc_sim *s) {
     c.B = &s->B;
     c.launches = &s->launches;
     c.gridCap = s->gridCap;
-    c.mayPolymerize = s->rulesPolymerize || s->loadScheduled;
+    c.mayPolymerize = may_polymerize(s);
     c.side[0] = s->forkClasses ? s->side[0] : nullptr;
     c.side[1] = s->forkClasses ? s->side[1] : nullptr;
     c.fork = s->fork;
@@ -473,14 +477,16 @@ void binned_after(ScParams &P, int phase) {
     if (phase == SC_PHASE_SORT_PARTICLES) P.lipidValid = 1;  // marked by sort_particles
 }
 
-// The host-side state a step reads and changes.
+// The host-side state a step reads and changes, and last what it only reads:
+// whether it polymerises (the launches it makes, so a captured step is looked
+// up by it too).
 std::vector<int> host_state(const sc_sim *s) {
     const ScBuffers &B = s->B;
     std::vector<int> v(B.cp, B.cp + FP_COUNT);
     v.insert(v.end(), B.cm, B.cm + FM_COUNT);
     v.insert(v.end(), {B.sortCurP, B.sortCurM, (int)B.validPP, (int)B.validM, (int)B.validLM, (int)B.validD,
                        s->P.binned, s->P.mAllActive, s->P.lipidValid, B.mParity, B.relaxAge, s->P.movedOnce, B.relaxMAge,
-                       B.diffuseAge, B.noiseAge});
+                       B.diffuseAge, B.noiseAge, (int)may_polymerize(s)});
     return v;
 }
 void set_host_state(sc_sim *s, const std::vector<int> &v) {
@@ -503,6 +509,20 @@ void set_host_state(sc_sim *s, const std::vector<int> &v) {
     B.relaxMAge = v[k++];
     B.diffuseAge = v[k++];
     B.noiseAge = v[k++];
+}
+
+// The host-side state before a load or a generated scene: the first buffers
+// current, no set in its cells, no list, nothing scheduled.
+void forget_state(sc_sim *s) {
+    ScBuffers &B = s->B;
+    B.invalidateLists();
+    s->P.binned = 0;
+    s->P.movedOnce = 0;
+    s->P.mAllActive = 0;
+    s->P.lipidValid = 0;
+    s->loadScheduled = false;
+    for (int k = 0; k < FP_COUNT; k++) B.cp[k] = 0;
+    for (int k = 0; k < FM_COUNT; k++) B.cm[k] = 0;
 }
 
 int run_phase(sc_sim *s, int phase, int arg) {
@@ -1105,14 +1125,8 @@ int sc_load_state(sc_sim *s, const sc_particle *particles, int32_t n, const sc_m
     int rc = ensure_staging(s, kStageBytes);
     if (rc) return rc;
     ScBuffers &B = s->B;
-    B.invalidateLists();
+    forget_state(s);
     s->loaded = false;
-    s->P.binned = 0;
-    s->P.movedOnce = 0;
-    s->P.mAllActive = 0;
-    s->P.lipidValid = 0;
-    for (int k = 0; k < FP_COUNT; k++) B.cp[k] = 0;
-    for (int k = 0; k < FM_COUNT; k++) B.cm[k] = 0;
     // mcFlag: [0] a metabolic record differs from the first, [1] the lowest
     // particle index with an interaction count outside 0..8, [2] a particle is
     // scheduled to polymerise
@@ -1627,13 +1641,7 @@ static int generate_into(sc_sim *s, int n, int nm, uint64_t seed, const std::fun
     int rc = ensure_staging(s, std::max<size_t>(bytes, 16));
     if (rc) return rc;
     ScBuffers &B = s->B;
-    B.invalidateLists();
-    s->P.binned = 0;
-    s->P.movedOnce = 0;
-    s->P.mAllActive = 0;
-    s->P.lipidValid = 0;
-    for (int k = 0; k < FP_COUNT; k++) B.cp[k] = 0;
-    for (int k = 0; k < FM_COUNT; k++) B.cm[k] = 0;
+    forget_state(s);
     const float box = s->cfg.sim_size;
     if (N > 0) {
         if (n) particles(box);
@@ -1704,13 +1712,7 @@ int sc_generate_batch(sc_sim *s, const int32_t *n, const int32_t *nm, const int3
     int rc = ensure_staging(s, std::max<size_t>(bytes, 16));
     if (rc) return rc;
     ScBuffers &B = s->B;
-    B.invalidateLists();
-    s->P.binned = 0;
-    s->P.movedOnce = 0;
-    s->P.mAllActive = 0;
-    s->P.lipidValid = 0;
-    for (int k = 0; k < FP_COUNT; k++) B.cp[k] = 0;
-    for (int k = 0; k < FM_COUNT; k++) B.cm[k] = 0;
+    forget_state(s);
     // each replica's records as sc_generate_uniform writes them for a sim of
     // its own (ids from 0, its box, its mix and seed), one replica after another
     if (N > 0) {
@@ -1790,13 +1792,7 @@ int sc_generate_scene_batch(sc_sim *s, const sc_scene_group *groups, int32_t n_g
                                                          (size_t)nm * sizeof(sc_metabolic_particle)), 16));
     if (rc) return rc;
     ScBuffers &B = s->B;
-    B.invalidateLists();
-    s->P.binned = 0;
-    s->P.movedOnce = 0;
-    s->P.mAllActive = 0;
-    s->P.lipidValid = 0;
-    for (int k = 0; k < FP_COUNT; k++) B.cp[k] = 0;
-    for (int k = 0; k < FM_COUNT; k++) B.cm[k] = 0;
+    forget_state(s);
     const size_t Q = (size_t)s->P.SP / 4;
     const sc_type_info *mt = nm > 0 ? &s->types[SC_PARTICLE_TYPE_METABOLIC] : nullptr;
     bool uniform = true;
