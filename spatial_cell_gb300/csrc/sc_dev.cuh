@@ -162,7 +162,14 @@ struct ScParams {
     const int *farMove;
     int lipidValid;
     const uint8_t *lipidP;
+    // per set: nonzero if the last sort found an active item outside its
+    // periodic box (loaded so, or moved by more than a box in one step)
+    const uint32_t *outsideP, *outsideM;
 };
+// Whether a position lies in the box [0, L]^3 (no NaN does).
+__device__ __forceinline__ bool in_box(sc_f3 p, float L) {
+    return p.x >= 0.0f && p.x <= L && p.y >= 0.0f && p.y <= L && p.z >= 0.0f && p.z <= L;
+}
 
 // Whether sorted particle j is an active lipid.
 __device__ __forceinline__ bool active_lipid(const ScParams &P, const int4 *__restrict__ pinfo, int j) {
@@ -384,10 +391,16 @@ __device__ __forceinline__ void cells27(const ScParams &P, sc_f3 pos, F &&f) {
     cells27(P, pos, Reach(), f);
 }
 
-// Whether candidates of sets `need` may lie on either side of a periodic face
-// whatever cell they are listed in (scan_words).
-__device__ __forceinline__ bool scan_mixed(const ScParams &P, int need) {
-    return P.periodic && ((P.binned & need) != need || !(P.simSize >= 5.0f * P.cell));
+// Whether an item's candidates of sets `need` may lie on either side of a
+// periodic face whatever cell they are listed in (scan_words): the sets have
+// moved since their sort, the box is under five cells, or a position lies
+// outside the box, in the cell on the face that its index is clamped to and up
+// to a box length from it.  An item that takes no images (Imager::wrap) has
+// none to look for.
+__device__ __forceinline__ bool scan_mixed(const ScParams &P, const Imager &IM, int need) {
+    if (!IM.wrap) return false;
+    if ((P.binned & need) != need || !(P.simSize >= 5.0f * P.cell) || !in_box(IM.p, P.simSize)) return true;
+    return ((need & SC_BINNED_P) && *P.outsideP) || ((need & SC_BINNED_M) && *P.outsideM);
 }
 // The same neighbourhood for the list builds, in two passes a thread takes
 // word by word.  A builder's thread spends its time on candidates that leave
@@ -408,9 +421,8 @@ __device__ __forceinline__ bool scan_mixed(const ScParams &P, int need) {
 // periodic face is tested against the item shifted by the box, with a margin:
 // a coordinate difference and its image differ from the box length by the
 // rounding of coordinates no larger than |pp| + 2 L + lim.  With `mixed`
-// (candidates that may lie on either side of a face: sets that have moved
-// since their sort, boxes under five cells) every candidate within that
-// margin directly or across a face is kept.  f(k, cand[k]) makes the exact
+// (scan_mixed) every candidate within that margin directly or across a face is
+// kept.  f(k, cand[k]) makes the exact
 // tests; without an image (Imager::wrap) the cube holds already.
 //
 // What bounds it is the latency of the candidates' loads at 32 warps per SM,

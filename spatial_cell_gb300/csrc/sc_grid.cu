@@ -52,7 +52,7 @@ __host__ __device__ static inline size_t sort_tiles(long long n, int ipt) { retu
 // Past a block per SM a thread takes SORT_KEYS items, their loads together, so
 // that fewer blocks add to each of the histogram's words: 262,144 items 12.4 us
 // at one item, 6.1 us at four.  The kernel also clears what the passes behind it look at first (the look-back words and
-// tile counters) and farMove.
+// tile counters) and farMove, and notes positions outside a periodic box.
 template <bool BATCH, int KEYS>
 __global__ void __launch_bounds__(SC_THREADS) k_sort_keys(SortPair sets, ScParams P, uint32_t inactiveKey, int passes,
                                                           int ipt, ScCounters *ctr) {
@@ -84,6 +84,7 @@ __global__ void __launch_bounds__(SC_THREADS) k_sort_keys(SortPair sets, ScParam
             int lim = cell_limit(P);
             k = cell_key(P, sc_grid_idx(p[r].x, P.cell, lim), sc_grid_idx(p[r].y, P.cell, lim),
                          sc_grid_idx(p[r].z, P.cell, lim));
+            if (P.periodic && !in_box(p[r], P.simSize)) hist[SC_SORT_OUTSIDE] = 1;
         }
         keys[i] = k;
         for (int d = 0; d < passes; d++) atomicAdd(&sh[d * 256 + ((k >> (8 * d)) & 0xffu)], 1u);
@@ -330,7 +331,7 @@ int sc_launch_sort(cudaStream_t st, const ScSortSet *sets, int count, const ScPa
     const SortPair pair{{sets[0], sets[count - 1]}};
     const int n = std::max(pair.s[0].n, pair.s[1].n), ipt = sort_ipt(n);
     auto *const pass = ipt == 4 ? k_onesweep<4> : ipt == 8 ? k_onesweep<8> : k_onesweep<SORT_IPT>;
-    for (int k = 0; k < count; k++) cudaMemsetAsync(sets[k].hist, 0, 4 * 256 * sizeof(uint32_t), st);
+    for (int k = 0; k < count; k++) cudaMemsetAsync(sets[k].hist, 0, SC_SORT_HIST * sizeof(uint32_t), st);
     if (n > 0) {
         const bool one = sort_tiles(n, 1) <= SORT_SMS;
         auto *const make = P.nRep > 1 ? (one ? k_sort_keys<true, 1> : k_sort_keys<true, SORT_KEYS>)

@@ -296,7 +296,7 @@ __device__ __forceinline__ void build_pp_block(
             }
         };
         scan_words(P, W, pos, [&](uint32_t key) { return cellStart[key]; }, ppos, reach(P, ppos, P.maxInt, SC_BINNED_P),
-                   P.maxInt, scan_mixed(P, SC_BINNED_P), [&](int j, float4 t4) {
+                   P.maxInt, scan_mixed(P, IM, SC_BINNED_P), [&](int j, float4 t4) {
                        if (j == i) return;
                        const sc_f3 delta = IM(sc_make_f3(t4.x, t4.y, t4.z)) - ppos;
                        if (IM.wrap && outside_cube(delta, P.maxInt)) return;
@@ -1394,7 +1394,8 @@ __device__ __forceinline__ void build_m_item(const ScParams &P, ScanWords &W, Co
     const float lim = P.maxInt;
     const bool wrap = IM.wrap;
     uint32_t *out = list + sc_list_at(SC_LIST_M, i, 0);
-    scan_words(P, W, comb, cs, pp, reach(P, pp, lim, SC_BINNED_M | SC_BINNED_P), lim, scan_mixed(P, SC_BINNED_M | SC_BINNED_P), [&](int, float4 t) {
+    scan_words(P, W, comb, cs, pp, reach(P, pp, lim, SC_BINNED_M | SC_BINNED_P), lim,
+               scan_mixed(P, IM, SC_BINNED_M | SC_BINNED_P), [&](int, float4 t) {
         const uint32_t e = __float_as_uint(t.w);
         if ((e & ~SC_M_ODD) == (uint32_t)i) return;
         sc_f3 delta;
@@ -2249,7 +2250,7 @@ __device__ __forceinline__ void build_lm_item(const ScParams &P, ScanWords &W, c
     const float prad = p4.w, lim = P.maxInt;
     CollisionDistCache cc;
     scan_words(P, W, mpos, [&](uint32_t key) { return cellStartM[key]; }, pp, reach(P, pp, lim, SC_BINNED_M), lim,
-               scan_mixed(P, SC_BINNED_M), [&](int j, float4 t4) {
+               scan_mixed(P, IM, SC_BINNED_M), [&](int j, float4 t4) {
                    sc_f3 delta = IM(sc_make_f3(t4.x, t4.y, t4.z)) - pp;
                    if ((IM.wrap && outside_cube(delta, lim)) || !active_m(P, minfo, j)) return;
                    if (cc.collides(prad, t4.w, delta)) {
