@@ -84,7 +84,7 @@ struct ScBuffers {
     size_t poolCapM;              // entries the metabolic pair pool (listM) holds
     int poolEntryWords;           // 4-byte words per metabolic pool entry: 1 (lean) or 4 (with geometry)
     long long *warpOffLM;         // lipid-metabolic pair pool: the same
-    float4 *comb;                 // candidates of the metabolic list build, cell by cell (k_combine)
+    float4 *comb;                 // candidates of the metabolic list build, cell by cell (k_combine; in listD when they fit)
     uint8_t *lipidP;              // per sorted particle slot: active lipid (after each particle sort)
     bool validPP, validM, validLM, validD;
     void invalidateLists() { validPP = validM = validLM = validD = false; relaxAge = noiseAge = relaxMAge = diffuseAge = 0; }

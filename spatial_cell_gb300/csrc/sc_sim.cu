@@ -1005,7 +1005,7 @@ static int create_sim(const sc_config *cfg_in, const sc_replica *replicas, int32
         (rc = dalloc(s, &B.ovfD, Nm)) || (rc = dalloc(s, &B.ovfOffD, Nm)) || (rc = dalloc(s, &B.ovfPoolD, 1)) ||
         (rc = dalloc(s, &B.claimP, P.pairClaim ? N : 1)) ||
         (rc = dalloc(s, &B.warpOffM, (size_t)Nm / 32 + 1)) || (rc = dalloc(s, &B.warpOffLM, (size_t)N / 32 + 1)) ||
-        (rc = dalloc(s, &B.lipidP, N)) || (rc = dalloc(s, &B.comb, N + Nm + SC_CAND_PAD)))
+        (rc = dalloc(s, &B.lipidP, N)))
         return bail(rc);
     // The LM list is built in the diffusion list's buffer when it fits, behind
     // the metabolic list's scratch when both do.
@@ -1017,6 +1017,14 @@ static int create_sim(const sc_config *cfg_in, const sc_replica *replicas, int32
         B.scratchLM = B.listD + (B.scratchApart ? wordsM : 0);
     } else if ((rc = dalloc(s, &B.scratchLM, wordsLM))) {
         return bail(rc);
+    }
+    // The metabolic list's candidates live from k_combine to that build (none in
+    // the tiled sweep): behind both scratches where the rest of the buffer holds
+    // them (about 1.9 metabolic items a particle and more), else on their own.
+    const size_t combAt = wordsM + (B.scratchInD && B.scratchApart ? wordsLM : 0), comb = N + Nm + SC_CAND_PAD;
+    if (P.tileCapM == 0) {
+        if (combAt + 4 * comb <= wordsD) B.comb = reinterpret_cast<float4 *>(B.listD + combAt);
+        else if ((rc = dalloc(s, &B.comb, comb))) return bail(rc);
     }
     B.invalidateLists();
     B.poolEntryWords = poolEntryWords;
