@@ -21,9 +21,12 @@ from . import abi, native, scenes
 
 # Device bytes per item of a request's simulation (state, two buffers of
 # every field, and pair lists as sc_create and sc_prepare size them at this
-# density), used to decide admission; once admitted, a request counts against
-# the budget with what its sim holds (sc_device_bytes).
-BYTES_PER_PARTICLE = 1400
+# density, the metabolic items' share covering frame slots too), used to decide
+# admission: from 1,000 particles on more than the sim comes to hold, by 2 to 6 %
+# for mixes with hardly any lipids (few metabolic items displaced, the largest
+# pool) and 11 to 15 % at 0.4 lipids.  Once admitted, a request counts against the
+# budget with what its sim holds (sc_device_bytes).
+BYTES_PER_PARTICLE = 1550
 BYTES_PER_METABOLIC = 1700
 
 
