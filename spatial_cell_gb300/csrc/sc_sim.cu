@@ -1038,6 +1038,9 @@ static int create_sim(const sc_config *cfg_in, const sc_replica *replicas, int32
     P.outsideM = B.hist + SC_SORT_HIST + SC_SORT_OUTSIDE;
     cudaMemsetAsync(B.ctr, 0, sizeof(ScCounters), s->st);
     cudaMemsetAsync(B.polyClaim, 0, std::max<size_t>(N, 1) * sizeof(int), s->st);
+    // until its first sort a set lies in no cell: every cell empty, every key past them
+    cudaMemsetAsync(B.keysP[0], 0xff, N * sizeof(uint32_t), s->st);
+    cudaMemsetAsync(B.keysM[0], 0xff, Nm * sizeof(uint32_t), s->st);
     cudaMemsetAsync(B.cellStartP, 0, ((size_t)P.cells + 1) * 4, s->st);
     cudaMemsetAsync(B.cellStartM, 0, ((size_t)P.cells + 1) * 4, s->st);
     cudaError_t e = cudaStreamSynchronize(s->st);
