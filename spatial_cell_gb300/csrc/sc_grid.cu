@@ -44,7 +44,9 @@ __device__ __forceinline__ void st_relaxed(uint32_t *p, uint32_t v) {
 struct SortPair {
     ScSortSet s[2];
 };
-__host__ __device__ static inline size_t sort_tiles(long long n, int ipt) { return (size_t)((n + SC_THREADS * ipt - 1) / (SC_THREADS * ipt)); }
+__host__ __device__ static inline size_t sort_tiles(long long n, int ipt) {
+    return (size_t)((n + SC_THREADS * ipt - 1) / (SC_THREADS * ipt));
+}
 
 // In a batched sim the key is the item's replica's key base plus its cell
 // in that replica's grid: replicas sort into consecutive key ranges.
@@ -297,7 +299,6 @@ __global__ void __launch_bounds__(SC_THREADS) k_gather_mfield(const uint32_t *__
 
 // ---- host-side launchers -----------------------------------------------------
 
-int sc_sort_passes(int bits) { return (3 * bits + 1 + 7) / 8; }
 int sc_sort_passes_for(const ScParams &P) { return ((P.keyBits > 0 ? P.keyBits : 3 * P.bits + 1) + 7) / 8; }
 
 // Four or eight keys per thread while every tile has an SM of its own, sixteen

@@ -38,7 +38,7 @@ struct ScBuffers {
     // the four arrays above are then unallocated until a load needs them).
     bool mcUniform;
     int mcLscs0, mcSpoly0;
-    int *mcFlag;   // device word of k_mc_scan
+    int *mcFlag;   // device words of a load's scans (k_mc_scan, k_unpack_particles)
     // binning: keys / slot values ping-pong per item set, the buffer of the
     // last pass holding the sorted keys and the permutation
     uint32_t *keysP[2], *valsP[2], *keysM[2], *valsM[2], *hist, *lookback, *lookbackM;
@@ -170,7 +170,6 @@ struct ScBuffers {
 };
 
 // sc_grid.cu
-int sc_sort_passes(int bits);
 int sc_sort_passes_for(const ScParams &P);  // passes over P's key bits
 size_t sc_sort_lookback_words(int cap);
 // One item set to sort: keys and vals ping-pong, SC_SORT_HIST words of hist (the

@@ -454,7 +454,6 @@ __global__ void __launch_bounds__(SC_THREADS) k_coordinate_noise(
 // ---- dynamics.cuh:405-822 relax ------------------------------------------------
 struct RelaxArgs {
     const uint32_t *__restrict__ cellStart;
-    const int *__restrict__ nActivePtr;
     const float4 *__restrict__ pos;
     const int4 *__restrict__ info;
     const int *__restrict__ nb;
@@ -1258,8 +1257,8 @@ __global__ void __launch_bounds__(relax_threads(CLS), CLS == 0 ? 10 : CLS == 1 ?
     const int n0 = B0 ? A.classCount[0] : 0, n1 = B1 ? A.classCount[1] : 0, n2 = B2 ? A.classCount[2] : 0,
               nv = B0 ? *A.ovfCount : 0;
     constexpr int PL = CLS == SC_RELAX_ALL_LANES ? SC_POLAR_LANES : 1;   // threads per polar item
-    const int b0 = T == 64 ? (n0 + SC_THREADS - 1) / SC_THREADS * 8 : (n0 + T / 2 - 1) / (T / 2), b1 = b0 + (n1 * PL + T - 1) / T, b2 = b1 + (n2 + T - 1) / T,
-              b3 = b2 + (nv + T - 1) / T;
+    const int b0 = T == 64 ? (n0 + SC_THREADS - 1) / SC_THREADS * 8 : (n0 + T / 2 - 1) / (T / 2),
+              b1 = b0 + (n1 * PL + T - 1) / T, b2 = b1 + (n2 + T - 1) / T, b3 = b2 + (nv + T - 1) / T;
     for (int b = blockIdx.x; b < b3; b += gridDim.x) {
         if (B0 && b < b0) {
             relax_bonded_block<BATCH, CLS == SC_RELAX_ALL_LANES, T>(P, A, b, n0, s_av);
@@ -1603,8 +1602,8 @@ __device__ __forceinline__ void emit_m_pairs_lean(const ScParams &P, int block, 
 
 template <bool LEAN, bool BATCH>
 __device__ __forceinline__ void build_m_block(
-    const ScParams &P0, ScanWords &W, int block, CombStart cs, const float4 *__restrict__ comb, const int *__restrict__ nActivePtr, const float4 *__restrict__ mpos,
-    const int4 *__restrict__ minfo, const float4 *__restrict__ ppos_, uint32_t *__restrict__ pool, long long poolCap,
+    const ScParams &P0, ScanWords &W, int block, CombStart cs, const float4 *__restrict__ comb,
+    const int *__restrict__ nActivePtr, const float4 *__restrict__ mpos, const int4 *__restrict__ minfo, const float4 *__restrict__ ppos_, uint32_t *__restrict__ pool, long long poolCap,
     unsigned long long *__restrict__ poolUsed, long long *__restrict__ warpOff, uint32_t *scratch,
     int *__restrict__ cnt, int *__restrict__ perm, int cap, int *__restrict__ ovf, int *__restrict__ ovfCount,
     int *__restrict__ ovfN) {
@@ -1626,8 +1625,8 @@ __device__ __forceinline__ void build_m_block(
 }
 template <bool LEAN, bool BATCH>
 __global__ void __launch_bounds__(SC_THREADS, 4) k_build_m(
-    ScParams P0, CombStart cs, const float4 *__restrict__ comb, const int *__restrict__ nActivePtr, const float4 *__restrict__ mpos,
-    const int4 *__restrict__ minfo, const float4 *__restrict__ ppos_, uint32_t *__restrict__ pool, long long poolCap,
+    ScParams P0, CombStart cs, const float4 *__restrict__ comb, const int *__restrict__ nActivePtr,
+    const float4 *__restrict__ mpos, const int4 *__restrict__ minfo, const float4 *__restrict__ ppos_, uint32_t *__restrict__ pool, long long poolCap,
     unsigned long long *__restrict__ poolUsed, long long *__restrict__ warpOff, uint32_t *scratch,
     int *__restrict__ cnt, int *__restrict__ perm, int cap, int *__restrict__ ovf, int *__restrict__ ovfCount,
     int *__restrict__ ovfN) {
@@ -3759,7 +3758,7 @@ void sc_phase_relax(ScLaunchCtx &c) {
     if (c.P.N <= 0) return;
     ensure_pp(c);
     PFields F = B.P(), X = B.Pnext();
-    RelaxArgs A{B.cellStartP, &B.ctr->nActive, F.pos, F.info, F.nb, F.bonds, pp_list(c),
+    RelaxArgs A{B.cellStartP, F.pos, F.info, F.nb, F.bonds, pp_list(c),
                 F.vel, F.rot, F.angvel, X.vel, X.rot, X.angvel, F.dbg, B.classPP, B.ctr->ppClassCount,
                 B.matchPP, B.matchN, B.geoPP, B.bondRec, B.ovfPP, &B.ctr->ovfPP, &B.ctr->ppClassCount[3], B.relaxAge};
     const int nb = nblocks(c.P.N);
@@ -3831,8 +3830,8 @@ void sc_phase_build_m(ScLaunchCtx &c) {
             (c.P.nRep > 1 ? (c.P.metabLean ? k_build_m<true, true> : k_build_m<false, true>)
                           : (c.P.metabLean ? k_build_m<true, false> : k_build_m<false, false>))<<<
                 nblocks(c.P.Nm), SC_THREADS, 0, c.st>>>(
-                c.P, cs, B.comb, &B.ctr->nActiveM, M.pos, M.info, F.pos, B.listM, (long long)B.poolCapM, &B.ctr->poolM, B.warpOffM, B.listD, B.cntM, B.permM, c.P.Nm, B.ovfM, &B.ctr->ovfM,
-                B.ovfNM);
+                c.P, cs, B.comb, &B.ctr->nActiveM, M.pos, M.info, F.pos, B.listM, (long long)B.poolCapM, &B.ctr->poolM,
+                B.warpOffM, B.listD, B.cntM, B.permM, c.P.Nm, B.ovfM, &B.ctr->ovfM, B.ovfNM);
             // the overflowed items' full lists
             SC_BATCHED(k_build_m_ovf)<<<std::min(nblocks(c.P.Nm), c.gridCap / 4), SC_THREADS, 0, c.st>>>(
                 c.P, B.cellStartM, B.cellStartP, M.pos, M.info, F.pos, F.info, B.ovfM, &B.ctr->ovfM, B.ovfNM,
@@ -3964,8 +3963,9 @@ void sc_phase_complexify(ScLaunchCtx &c, bool prep) {
         (*c.launches) += 2;
     } else {
         cudaMemsetAsync(B.claimP, 0xff, (size_t)c.P.N * sizeof(unsigned long long), c.st);
-        SC_BATCHED(k_claim_offer)<<<std::min(nblocks(c.P.N) * 11, 4 * c.gridCap), SC_THREADS, 0, c.st>>>(c.P, B.cellStartP, B.workP, &B.ctr->workCount, F.pos, F.rot,
-                                                       F.info, F.state, F.nb, F.bonds, &B.ctr->step, prep, B.claimP);
+        SC_BATCHED(k_claim_offer)<<<std::min(nblocks(c.P.N) * 11, 4 * c.gridCap), SC_THREADS, 0, c.st>>>(
+            c.P, B.cellStartP, B.workP, &B.ctr->workCount, F.pos, F.rot, F.info, F.state, F.nb, F.bonds, &B.ctr->step,
+            prep, B.claimP);
         SC_BATCHED(k_claim_bind)<<<blocks, SC_THREADS, 0, c.st>>>(c.P, B.workP, &B.ctr->workCount, F.pos, F.rot, F.info, F.state,
                                                       F.nb, X.nb, F.bonds, &B.ctr->step, prep, B.claimP);
         (*c.launches) += 3;
