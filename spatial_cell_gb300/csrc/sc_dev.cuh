@@ -162,10 +162,12 @@ struct ScParams {
     const int *farMove;
     int lipidValid;
     const uint8_t *lipidP;
-    // per set: nonzero if the last sort found an active item outside its
-    // periodic box (loaded so, or moved by more than a box in one step)
-    const uint32_t *outsideP, *outsideM;
+    // per set, the last sort's digit counts: SC_SORT_OUTSIDE in the first if it
+    // found an active item outside its periodic box (loaded so, or moved by
+    // more than a box in one step)
+    const uint32_t *histP, *histM;
 };
+#define SC_SORT_OUTSIDE 0x80000000u
 // Whether a position lies in the box [0, L]^3 (no NaN does).
 __device__ __forceinline__ bool in_box(sc_f3 p, float L) {
     return p.x >= 0.0f && p.x <= L && p.y >= 0.0f && p.y <= L && p.z >= 0.0f && p.z <= L;
@@ -400,7 +402,7 @@ __device__ __forceinline__ void cells27(const ScParams &P, sc_f3 pos, F &&f) {
 __device__ __forceinline__ bool scan_mixed(const ScParams &P, const Imager &IM, int need) {
     if (!IM.wrap) return false;
     if ((P.binned & need) != need || !(P.simSize >= 5.0f * P.cell) || !in_box(IM.p, P.simSize)) return true;
-    return ((need & SC_BINNED_P) && *P.outsideP) || ((need & SC_BINNED_M) && *P.outsideM);
+    return (((need & SC_BINNED_P) ? *P.histP : 0u) | ((need & SC_BINNED_M) ? *P.histM : 0u)) & SC_SORT_OUTSIDE;
 }
 // The same neighbourhood for the list builds, in two passes a thread takes
 // word by word.  A builder's thread spends its time on candidates that leave

@@ -54,7 +54,9 @@ __host__ __device__ static inline size_t sort_tiles(long long n, int ipt) {
 // Past a block per SM a thread takes SORT_KEYS items, their loads together, so
 // that fewer blocks add to each of the histogram's words: 262,144 items 12.4 us
 // at one item, 6.1 us at four.  The kernel also clears what the passes behind it look at first (the look-back words and
-// tile counters) and farMove, and notes positions outside a periodic box.
+// tile counters) and farMove, and marks a set with a position outside a periodic
+// box (a bit of the first digit count: words of their own behind the counts make
+// the clearing memset 2 us longer, of 80 for a sort of 262,144 items).
 template <bool BATCH, int KEYS>
 __global__ void __launch_bounds__(SC_THREADS) k_sort_keys(SortPair sets, ScParams P, uint32_t inactiveKey, int passes,
                                                           int ipt, ScCounters *ctr) {
@@ -70,6 +72,7 @@ __global__ void __launch_bounds__(SC_THREADS) k_sort_keys(SortPair sets, ScParam
     const int first = blockIdx.x * blockDim.x + threadIdx.x, stride = blocks * SC_THREADS;
     int4 in[KEYS];
     sc_f3 p[KEYS];
+    bool outside = false;
 #pragma unroll
     for (int r = 0; r < KEYS; r++) {
         const int i = min(first + r * stride, n - 1);
@@ -86,7 +89,7 @@ __global__ void __launch_bounds__(SC_THREADS) k_sort_keys(SortPair sets, ScParam
             int lim = cell_limit(P);
             k = cell_key(P, sc_grid_idx(p[r].x, P.cell, lim), sc_grid_idx(p[r].y, P.cell, lim),
                          sc_grid_idx(p[r].z, P.cell, lim));
-            if (P.periodic && !in_box(p[r], P.simSize)) hist[SC_SORT_OUTSIDE] = 1;
+            outside |= P.periodic && !in_box(p[r], P.simSize);
         }
         keys[i] = k;
         for (int d = 0; d < passes; d++) atomicAdd(&sh[d * 256 + ((k >> (8 * d)) & 0xffu)], 1u);
@@ -94,7 +97,7 @@ __global__ void __launch_bounds__(SC_THREADS) k_sort_keys(SortPair sets, ScParam
     for (int w = first; w < lbWords; w += stride) S.lookback[w] = 0;
     if (first < 4) S.tileCounter[first] = 0;
     if (first == 4) ctr->farMove = 0;
-    __syncthreads();
+    if (__syncthreads_or(outside) && threadIdx.x == 0) atomicOr(hist, SC_SORT_OUTSIDE);
     for (int t = threadIdx.x; t < passes * 256; t += blockDim.x)
         if (sh[t]) atomicAdd(&hist[t], sh[t]);
 }
@@ -207,7 +210,7 @@ __global__ void __launch_bounds__(SC_THREADS) k_onesweep(SortPair sets, int pass
         }
         st_relaxed(&lookback[(size_t)tile * 256 + tid], LB_INC | (excl + cnt));
     }
-    uint32_t gofs = block_exclusive_scan256(hist[tid], s_wsum);
+    uint32_t gofs = block_exclusive_scan256(hist[tid] & ~SC_SORT_OUTSIDE, s_wsum);
     s_base[tid] = gofs + excl;
     __syncthreads();
 #pragma unroll
@@ -332,7 +335,7 @@ int sc_launch_sort(cudaStream_t st, const ScSortSet *sets, int count, const ScPa
     const SortPair pair{{sets[0], sets[count - 1]}};
     const int n = std::max(pair.s[0].n, pair.s[1].n), ipt = sort_ipt(n);
     auto *const pass = ipt == 4 ? k_onesweep<4> : ipt == 8 ? k_onesweep<8> : k_onesweep<SORT_IPT>;
-    for (int k = 0; k < count; k++) cudaMemsetAsync(sets[k].hist, 0, SC_SORT_HIST * sizeof(uint32_t), st);
+    for (int k = 0; k < count; k++) cudaMemsetAsync(sets[k].hist, 0, 4 * 256 * sizeof(uint32_t), st);
     if (n > 0) {
         const bool one = sort_tiles(n, 1) <= SORT_SMS;
         auto *const make = P.nRep > 1 ? (one ? k_sort_keys<true, 1> : k_sort_keys<true, SORT_KEYS>)

@@ -172,11 +172,8 @@ struct ScBuffers {
 // sc_grid.cu
 int sc_sort_passes_for(const ScParams &P);  // passes over P's key bits
 size_t sc_sort_lookback_words(int cap);
-// One item set to sort: keys and vals ping-pong, SC_SORT_HIST words of hist (the
-// passes' digit counts, then ScParams::outsideP / outsideM), lookback
+// One item set to sort: keys and vals ping-pong, hist 4*256 words, lookback
 // sc_sort_lookback_words(n) per pass, four tile counters, cells + 1 starts.
-#define SC_SORT_OUTSIDE (4 * 256)
-#define SC_SORT_HIST (SC_SORT_OUTSIDE + 4)
 struct ScSortSet {
     const float4 *pos;
     const int4 *info;

@@ -37,8 +37,8 @@ namespace {
 constexpr size_t kWords = SC_STATIC_SORT_MAX_ITEMS;
 constexpr size_t kKeysOff = 0;                                    // uint32 keys[2][MAX]
 constexpr size_t kValsOff = kKeysOff + 2 * kWords * 4;            // uint32 vals[2][MAX]
-constexpr size_t kHistOff = kValsOff + 2 * kWords * 4;            // uint32 hist[SC_SORT_HIST]
-constexpr size_t kLookOff = kHistOff + (SC_SORT_HIST * 4 + 255) / 256 * 256;  // uint32 lookback[4][tiles][256]
+constexpr size_t kHistOff = kValsOff + 2 * kWords * 4;            // uint32 hist[4][256]
+constexpr size_t kLookOff = kHistOff + 4 * 256 * 4;               // uint32 lookback[4][tiles][256]
 constexpr size_t kCtrOff = kLookOff + (size_t)4 * SC_STATIC_SORT_TILES * 256 * 4;  // ScCounters
 constexpr size_t kBytes = ((kCtrOff + sizeof(ScCounters) + 255) / 256) * 256;
 

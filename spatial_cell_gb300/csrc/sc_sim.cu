@@ -410,7 +410,7 @@ ScSortSet sort_set(sc_sim *s, bool metabolic) {
     }
     const MFields F = B.M();
     return {F.pos, F.info, s->P.Nm, {B.keysM[0], B.keysM[1]}, {B.valsM[0], B.valsM[1]},
-            B.hist + SC_SORT_HIST, B.lookbackM, B.ctr->tileCounter + 4, B.cellStartM};
+            B.hist + 4 * 256, B.lookbackM, B.ctr->tileCounter + 4, B.cellStartM};
 }
 
 void gather_particles(sc_sim *s, int cur) {
@@ -986,7 +986,7 @@ static int create_sim(const sc_config *cfg_in, const sc_replica *replicas, int32
     const int poolEntryWords = P.metabLean ? 1 : 4;
     size_t poolWords = sc_list_words(SC_LIST_M, (int)Nm);
     if (P.tileCapM == 0) poolWords = std::min(poolWords, sc_list_words(kPoolStart * poolEntryWords, (int)Nm));
-    if ((rc = dalloc(s, &B.mcFlag, 4)) || (rc = dalloc(s, &B.hist, 2 * SC_SORT_HIST)) ||
+    if ((rc = dalloc(s, &B.mcFlag, 4)) || (rc = dalloc(s, &B.hist, 2 * 4 * 256)) ||
         (rc = dalloc(s, &B.lookback, (size_t)passes * sc_sort_lookback_words((int)N))) ||
         (rc = dalloc(s, &B.lookbackM, (size_t)passes * sc_sort_lookback_words((int)Nm))) ||
         (rc = dalloc(s, &B.cellStartP, (size_t)P.cells + 1)) || (rc = dalloc(s, &B.cellStartM, (size_t)P.cells + 1)) ||
@@ -1036,8 +1036,8 @@ static int create_sim(const sc_config *cfg_in, const sc_replica *replicas, int32
         B.poolCapM = std::min(B.poolCapM, (size_t)cfg->pool_per_item * (size_t)std::max<int64_t>(Nm, 1));
     P.lipidP = B.lipidP;
     P.farMove = &B.ctr->farMove;
-    P.outsideP = B.hist + SC_SORT_OUTSIDE;
-    P.outsideM = B.hist + SC_SORT_HIST + SC_SORT_OUTSIDE;
+    P.histP = B.hist;
+    P.histM = B.hist + 4 * 256;
     cudaMemsetAsync(B.ctr, 0, sizeof(ScCounters), s->st);
     cudaMemsetAsync(B.polyClaim, 0, std::max<size_t>(N, 1) * sizeof(int), s->st);
     // until its first sort a set lies in no cell: every cell empty, every key past them
