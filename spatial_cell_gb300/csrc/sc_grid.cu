@@ -53,10 +53,11 @@ __host__ __device__ static inline size_t sort_tiles(long long n, int ipt) {
 //
 // Past a block per SM a thread takes SORT_KEYS items, their loads together, so
 // that fewer blocks add to each of the histogram's words: 262,144 items 12.4 us
-// at one item, 6.1 us at four.  The kernel also clears what the passes behind it look at first (the look-back words and
-// tile counters) and farMove, and marks a set with a position outside a periodic
-// box (a bit of the first digit count: words of their own behind the counts make
-// the clearing memset 2 us longer, of 80 for a sort of 262,144 items).
+// at one item, 6.1 us at four.  The kernel also clears what the passes behind
+// it look at first (the look-back words and tile counters) and farMove, and
+// marks a set with a position outside a periodic box (a bit of the first digit
+// count: words of their own behind the counts make the clearing memset 2 us
+// longer, of 80 for a sort of 262,144 items).
 template <bool BATCH, int KEYS>
 __global__ void __launch_bounds__(SC_THREADS) k_sort_keys(SortPair sets, ScParams P, uint32_t inactiveKey, int passes,
                                                           int ipt, ScCounters *ctr) {
